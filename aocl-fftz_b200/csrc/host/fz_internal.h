@@ -151,6 +151,12 @@ int64_t fz_tc64_tables(fz_blob *b);
 /* packed-real twiddles W_{2M}^k, k = 0..M (W^M = -1) */
 int64_t fz_real_twiddles(fz_blob *b, int dtype, int64_t M);
 
+/* ---- mixed-radix lines (mixed.c) ---- */
+int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost);
+int fz_mr_fits(int dtype, int64_t n);
+int fz_mr_shape(fftz_pass_t *k, int want_tpc);
+int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k);
+
 /* ---- shared by api.c and ragged.c ---- */
 void fz_plan_free(fz_plan *pl);
 void fz_ragged_free(fz_ragged *rg);

@@ -1,0 +1,278 @@
+/* Launch shape of mixed-radix lines (kernels/fft_mr.cuh): radix list, digit
+ * strides with their bank padding, transforms and threads per CTA (C99). */
+#include <string.h>
+
+#include "fz_internal.h"
+
+/* Issue slots of one radix-R butterfly: the codelet's arithmetic, about ten a
+ * value for its shared-memory accesses, twiddle and addresses, and the index
+ * maps. 0: no butterfly of that radix. */
+static int mr_cost(int R)
+{
+    static const int flops[17] = {0, 0, 4, 16, 16, 44, 44, 100, 56, 112, 108, 240, 112, 330, 228, 212, 168};
+    return R >= 2 && R <= 16 ? flops[R] + 10 * R + 12 : 0;
+}
+
+typedef struct
+{
+    int64_t n; /* the whole line */
+    int min_stages;
+    int cur[FFTZ_MR_STAGES], best[FFTZ_MR_STAGES];
+    int nbest;
+    double score;
+} mr_search;
+
+static void mr_try(mr_search *q, int64_t rest, int depth, int top, double cost)
+{
+    if (rest == 1)
+    {
+        if (depth >= q->min_stages && (q->nbest == 0 || cost < q->score))
+        {
+            q->score = cost;
+            q->nbest = depth;
+            memcpy(q->best, q->cur, sizeof(int) * (size_t)depth);
+        }
+        return;
+    }
+    if (depth == FFTZ_MR_STAGES || (q->nbest && cost >= q->score)) return;
+    for (int R = top; R >= 2; R--)
+        if (rest % R == 0)
+        {
+            q->cur[depth] = R;
+            /* three slots a value stand for the stage's barrier */
+            mr_try(q, rest / R, depth + 1, R, cost + (double)mr_cost(R) / R + 3.0);
+        }
+}
+
+/* Radices (largest first) of the cheapest split of n into at least min_stages
+ * stages; returns their number, 0 when n has a prime factor above 13. cost
+ * (may be NULL): issue slots a point. */
+int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost)
+{
+    mr_search q;
+    memset(&q, 0, sizeof(q));
+    q.n = n;
+    q.min_stages = min_stages;
+    int64_t m = n;
+    static const int pr[] = {2, 3, 5, 7, 11, 13};
+    for (int i = 0; i < 6; i++)
+        while (m % pr[i] == 0) m /= pr[i];
+    if (n < 2 || m != 1) return 0;
+    mr_try(&q, n, 0, 16, 0.0);
+    for (int s = 0; s < q.nbest; s++) radix[s] = q.best[s];
+    if (cost) *cost = q.score;
+    return q.nbest;
+}
+
+static uint32_t magic(int64_t d) { return d <= 1 ? 0u : (uint32_t)((0xFFFFFFFFull + (uint64_t)d) / (uint64_t)d); }
+
+/* slots of one line with `pad` extra per digit-0 block */
+static int64_t mr_span(const fftz_pass_t *k, int pad) { return k->n + (int64_t)pad * (k->nstages > 1 ? k->radix[0] : 0); }
+
+/* Most lines of this length a CTA can hold (0: none). */
+static int64_t mr_lines(const fftz_pass_t *k)
+{
+    const int64_t esz = k->dtype == 0 ? 8 : 16;
+    const int64_t per = (k->sstride + ((k->flags & FFTZ_F_TW4) ? 16 : 0)) * esz + 24;
+    return fftz_smem_limit() / per;
+}
+
+/* 1 if a line of n points fits one CTA as a mixed-radix tile. */
+int fz_mr_fits(int dtype, int64_t n)
+{
+    int32_t r[FFTZ_MR_STAGES];
+    const int64_t esz = dtype == 0 ? 8 : 16;
+    if (n < 2 || (n + 1 + 16) * esz + 24 > fftz_smem_limit()) return 0;
+    return fz_mr_radices(n, 1, r, NULL) > 0;
+}
+
+/* Slot of item i (of one line, or of tpc lines when col) of stage s; first /
+ * last are the maps of the HBM-side stages. */
+static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)
+{
+    const int S = k->nstages;
+    const int64_t R = k->radix[s], M = k->mr.m[s], nb = k->n / R;
+    int64_t p, x;
+    if (col)
+    {
+        x = i / k->tpc;
+        p = i % k->tpc;
+    }
+    else
+    {
+        p = i / nb;
+        x = i % nb;
+    }
+    const int64_t base = p * k->sstride;
+    if (s == 0) return base + x;
+    if (s == S - 1)
+    {
+        int64_t o = 0;
+        for (int j = 0; j < S - 1; j++)
+        {
+            o += (x % k->radix[j]) * (k->mr.m[j] + (j == 0 ? k->mr.pad : 0));
+            x /= k->radix[j];
+        }
+        return base + o;
+    }
+    const int64_t b = x / M;
+    int64_t B = 1;
+    for (int j = 1; j < s; j++) B *= k->radix[j];
+    return base + x + b * M * (R - 1) + (b / B) * k->mr.pad;
+}
+
+/* Shared-memory wavefronts per lane group (16 float or 8 double slots span all
+ * banks) over the first groups of every stage, for the pad and stride in k. */
+static int mr_conflicts(const fftz_pass_t *k)
+{
+    const int W = k->dtype == 0 ? 16 : 8;
+    int tot = 0;
+    for (int s = 0; s < k->nstages; s++)
+    {
+        const int col = (s == 0 && k->in_mode == 1) || (s == k->nstages - 1 && k->out_mode == 1);
+        const int64_t items = (int64_t)k->tpc * (k->n / k->radix[s]);
+        for (int g = 0; g < 8 && (int64_t)g * W < items; g++)
+        {
+            int cnt[16] = {0}, worst = 0;
+            for (int l = 0; l < W && (int64_t)g * W + l < items; l++)
+            {
+                int c = ++cnt[mr_addr(k, s, (int64_t)g * W + l, col) % W];
+                if (c > worst) worst = c;
+            }
+            tot += worst * k->radix[s] * (s > 0 && s < k->nstages - 1 ? 2 : 1);
+        }
+    }
+    return tot;
+}
+
+static void mr_stride(fftz_pass_t *k, int colmap, int pad)
+{
+    const int W = k->dtype == 0 ? 16 : 8;
+    int64_t s = mr_span(k, pad);
+    /* neighbouring lines: an odd distance, or W / tpc apart where lanes run
+     * across a power of two of lines */
+    const int spread = colmap && k->tpc > 1 && k->tpc <= W && (k->tpc & (k->tpc - 1)) == 0;
+    if (k->tpc > 1)
+        while (spread ? (s % W) != W / k->tpc : (s & 1) == 0) s++;
+    k->mr.pad = pad;
+    k->sstride = (int32_t)s;
+}
+
+/* Fills k's mixed-radix launch shape (its lengths, strides, batch and flags are
+ * set); want_tpc > 0 fixes the lines per CTA where they fit. Returns 0, or -1
+ * when the line does not fit a CTA. */
+int fz_mr_shape(fftz_pass_t *k, int want_tpc)
+{
+    const int two = (k->flags & FFTZ_F_MID_TAB) != 0;
+    const int colmap = k->in_mode == 1 || k->out_mode == 1;
+    k->nstages = fz_mr_radices(k->n, two ? 2 : 1, k->radix, NULL);
+    if (k->nstages <= 0) return -1;
+    k->variant = FFTZ_VAR_MR;
+    k->mr.big = 0;
+    int64_t M = k->n, B = 1;
+    for (int s = 0; s < k->nstages; s++)
+    {
+        const int R = k->radix[s];
+        if (R == 11 || R == 13) k->mr.big = 1;
+        M /= R;
+        k->mr.m[s] = (int32_t)M;
+        k->mr.mg_nb[s] = magic(k->n / R);
+        k->mr.mg_m[s] = magic(M);
+        k->mr.mg_r[s] = magic(R);
+        k->mr.mg_b[s] = magic(B);
+        if (s > 0) B *= R;
+    }
+    k->tpc = 1;
+    mr_stride(k, colmap, 0);
+    const int tmax = fftz_mr_max_threads(k->dtype, k->mr.big);
+    int64_t most = mr_lines(k);
+    if (most < 1) return -1;
+    if (most > k->ntf) most = k->ntf;
+    if (most > 256) most = 256;
+    /* lines per CTA: about 4096 float / 2048 double points of row lines; whole
+     * 64-byte segments (8 float / 4 double neighbours) of column lines */
+    const int64_t pts = k->dtype == 0 ? 4096 : 2048;
+    int64_t lo = 1, hi = most;
+    if (want_tpc > 0)
+        lo = hi = want_tpc < most ? want_tpc : most;
+    else if (colmap)
+    {
+        const int64_t seg = k->dtype == 0 ? 8 : 4;
+        lo = hi = seg < most ? seg : most;
+        while (hi * 2 <= most && hi * 2 * k->n <= pts && hi < 32) lo = hi = hi * 2;
+    }
+    else
+    {
+        /* fewer lines where whole CTAs would not give every SM two */
+        while (hi > 1 && (hi * k->n > pts + pts / 2 || k->ntf / hi < 2 * 148)) hi--;
+        lo = hi > 1 ? (hi + 1) / 2 : 1;
+    }
+    double best = -1;
+    int btpc = 1, bthr = 32;
+    for (int64_t c = lo; c <= hi; c++)
+    {
+        k->tpc = (int32_t)c;
+        mr_stride(k, colmap, 0);
+        const int64_t smem = fftz_pass_smem_bytes(k) + 1024;
+        if (smem - 1024 > fftz_smem_limit()) continue;
+        int64_t by_smem = (228 * 1024) / smem;
+        if (by_smem > 24) by_smem = 24;
+        for (int t = 64; t <= tmax; t += 32)
+        {
+            int64_t ctas = tmax / t;
+            if (ctas > by_smem) ctas = by_smem;
+            double used = 0, spent = 0;
+            for (int s = 0; s < k->nstages; s++)
+            {
+                const int64_t items = c * (k->n / k->radix[s]);
+                used += (double)items * mr_cost(k->radix[s]);
+                spent += (double)((items + t - 1) / t * t) * mr_cost(k->radix[s]);
+            }
+            /* lanes at work, times warps in flight (half weight), times the
+             * overlap of independent CTAs' phases */
+            double occ = (double)(ctas * t) / tmax;
+            double sc = used / spent * (0.4 + 0.6 * occ) * (ctas >= 4 ? 1.0 : ctas == 3 ? 0.98 : ctas == 2 ? 0.94 : 0.8);
+            if (sc > best + 1e-9)
+            {
+                best = sc;
+                btpc = (int)c;
+                bthr = t;
+            }
+        }
+    }
+    k->tpc = btpc;
+    k->threads = bthr;
+    k->tpt = bthr / btpc > 0 ? bthr / btpc : 1;
+    /* the digit-0 pad with the fewest bank conflicts that still fits */
+    int bp = -1, bc = 0;
+    for (int pad = 0; pad < (k->nstages > 1 ? 16 : 1); pad++)
+    {
+        mr_stride(k, colmap, pad);
+        if (pad > 0 && fftz_pass_smem_bytes(k) > fftz_smem_limit()) break;
+        const int c = mr_conflicts(k);
+        if (bp < 0 || c < bc)
+        {
+            bp = pad;
+            bc = c;
+        }
+    }
+    mr_stride(k, colmap, bp);
+    k->mr.mg_tpc = magic(k->tpc);
+    k->fuse_load = k->fuse_store = 1;
+    k->use_tma = 0;
+    k->smem_tw = 0;
+    return fftz_pass_smem_bytes(k) <= fftz_smem_limit() ? 0 : -1;
+}
+
+/* Stage twiddles of a mixed-radix line: stage s multiplies by
+ * W_{R_s M_s}^{k r} at [(k - 1) M_s + r], which is the Stockham table of the
+ * reversed radix list. Returns the blob offset, -1 on allocation failure. */
+int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k)
+{
+    int32_t rev[FFTZ_MR_STAGES], off[FFTZ_MR_STAGES];
+    const int S = k->nstages;
+    for (int s = 0; s < S; s++) rev[s] = k->radix[S - 1 - s];
+    const int64_t o = fz_stage_twiddles(b, k->dtype, k->n, S, rev, off);
+    for (int s = 0; s < S; s++) k->tw_off[s] = off[S - 1 - s];
+    return o;
+}

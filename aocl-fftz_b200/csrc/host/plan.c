@@ -110,6 +110,11 @@ static int64_t fast_max_n(const fz_plan *pl)
 }
 static int fast_max_threads(const fz_plan *pl) { return ragged_mode(pl) ? 256 : (pl->dtype == 0 ? 1024 : 512); }
 
+/* Runtime-radix lines run as mixed-radix tiles (one buffer, kernels/fft_mr.cuh);
+ * kernel_family 12 keeps the older in-place kernel, the ragged executor its
+ * ping-pong tiles. */
+static int mixed_lines(const fz_plan *pl) { return pl->hints.kernel_family != 12 && !ragged_mode(pl); }
+
 /* Batch dims: optionally sorted by stride (smallest first, so that bdim[0]
  * is the one lanes may run along), then adjacent dims merged when they form
  * one arithmetic progression on both sides (the reference's fuse_vecs,
@@ -312,6 +317,20 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
     else
     {
     generic:
+        if (n > 1 && mixed_lines(pl))
+        {
+            k->smem_tw = k->use_tma = 0;
+            const int colm = k->in_mode == 1 || k->out_mode == 1;
+            if (fz_mr_shape(k, colm ? pl->hints.tpc_col : pl->hints.tpc_row))
+            {
+                fz_set_error("length %lld does not fit a mixed-radix tile", (long long)n);
+                return NULL;
+            }
+            p->off_tw = fz_mr_twiddles(&pl->blob, k);
+            if (p->off_tw < 0) return NULL;
+            snprintf(p->what, sizeof(p->what), "generic-mr n=%lld x%lld", (long long)n, (long long)k->ntf);
+            return p;
+        }
         k->variant = FFTZ_VAR_GENERIC;
         k->nstages = n > 1 ? generic_radices(n, k->radix) : 0;
         if (k->nstages < 0)
@@ -321,9 +340,9 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
         }
         k->tpt = k->nstages ? fftz_threads_per_transform(pl->dtype, (int)n, k->nstages, k->radix) : 1;
         maxthr = fftz_generic_max_threads();
-        /* lines longer than the in-place tile's thread budget run as ping-pong
-         * tiles (chosen below) */
-        if (k->tpt > maxthr && pl->hints.kernel_family != 12 && pp_one_line_bytes(pl->dtype, n) <= fftz_smem_limit())
+        /* the executor's lines longer than the in-place tile's thread budget run
+         * as ping-pong tiles (chosen below) */
+        if (k->tpt > maxthr && ragged_mode(pl) && pp_one_line_bytes(pl->dtype, n) <= fftz_smem_limit())
             k->tpt = maxthr;
         if (k->tpt > maxthr)
         {
@@ -349,10 +368,10 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
         finish_launch_shape(pl, k, nslots, maxthr);
     }
     if (k->smem_tw && fftz_pass_smem_bytes(k) > fftz_smem_limit()) k->smem_tw = 0;
-    /* runtime-radix lines: the ping-pong kernel (two shared-memory buffers,
-     * one butterfly per thread at a time, 256 threads) when both buffers fit;
-     * kernel_family 12 keeps the in-place kernel */
-    if (k->variant == FFTZ_VAR_GENERIC && pl->hints.kernel_family != 12)
+    /* the ragged executor's runtime-radix lines: ping-pong tiles (two
+     * shared-memory buffers, one butterfly per thread at a time, 256 threads)
+     * when both buffers fit */
+    if (k->variant == FFTZ_VAR_GENERIC && ragged_mode(pl))
     {
         const int esz = pl->dtype == 0 ? 8 : 16;
         const int32_t sst = fftz_smem_stride(pl->dtype, nslots);
@@ -423,7 +442,7 @@ static int single_pass_ok(const fz_plan *pl, int64_t n)
     if (s < 0 || n > (1 << 20)) return 0;
     /* the executor's tiles (ragged batches) are ping-pong tiles within its cap */
     if (ragged_mode(pl)) return pp_one_line_bytes(pl->dtype, n) <= fz_ragged_smem_cap(pl->dtype);
-    if (pl->hints.kernel_family != 12 && pp_one_line_bytes(pl->dtype, n) <= fftz_smem_limit()) return 1;
+    if (mixed_lines(pl)) return fz_mr_fits(pl->dtype, n);
     int tpt = fftz_threads_per_transform(pl->dtype, (int)n, s, r);
     if (tpt < 1 || tpt > fftz_generic_max_threads()) return 0;
     int64_t esz = pl->dtype == 0 ? 8 : 16;

@@ -36,6 +36,7 @@ int fftz_max_smem_n(int dtype) { return dtype == 0 ? 16384 : 8192; }
 int fftz_fast_max_n(int dtype) { return dtype == 0 ? 16384 : 8192; }
 int fftz_fast_tpt(int n) { return fftz::ct_tpt(n); }
 int fftz_generic_max_threads(void) { return 256; }
+int fftz_mr_max_threads(int dtype, int big) { return dtype == 0 ? (big ? 768 : 1024) : (big ? 384 : 512); }
 int fftz_pipe_max_threads(int n) { return fftz::ct_pipe_lb(n); }
 
 int fftz_fast_radices(int n, int32_t *radix) {
@@ -107,6 +108,9 @@ int64_t fftz_pass_smem_bytes(const fftz_pass_t *p) {
   const int64_t esz = p->dtype == 0 ? 8 : 16;
   if (p->variant == FFTZ_VAR_GENERIC_PP)
     return 2 * (int64_t)p->tpc * p->sstride * esz + 3 * 8 * (int64_t)p->tpc + 8 * FFTZ_MAX_STAGES;
+  if (p->variant == FFTZ_VAR_MR)
+    return (int64_t)p->tpc * p->sstride * esz + ((p->flags & FFTZ_F_TW4) ? 16 * esz * p->tpc : 0) +
+           3 * 8 * (int64_t)p->tpc;
   if (is_pipe(p)) return 2 * (int64_t)p->tpc * p->sstride * esz + 9 * 8 * (int64_t)p->tpc;
   int64_t b = (int64_t)p->tpc * p->sstride * esz + 3 * 8 * (int64_t)p->tpc;
   if (p->smem_tw) b += 16 + (int64_t)fftz_fast_tw_entries(p->n) * esz;  // shared copy of the stage twiddles
@@ -134,6 +138,11 @@ int fftz_launch_pass(const fftz_pass_t *p, void *stream) {
                        : (const void *)&fftz::fft_smem_kernel<double>;
   } else if (p->variant == FFTZ_VAR_GENERIC_PP) {
     fn = p->dtype == 0 ? (const void *)&fftz::fft_pp_kernel<float> : (const void *)&fftz::fft_pp_kernel<double>;
+  } else if (p->variant == FFTZ_VAR_MR) {
+    int feat = (p->flags & FFTZ_F_TW4) ? 1 : 0;
+    if ((p->flags & (FFTZ_F_PRE_TAB | FFTZ_F_POST_TAB | FFTZ_F_SCALE)) || p->pre_n || p->post_n) feat = 2;
+    if (p->flags & FFTZ_F_MID_TAB) feat = 2 | 4;
+    fn = p->dtype == 0 ? fftz_mr_kernel_f32(feat, p->mr.big) : fftz_mr_kernel_f64(feat, p->mr.big);
   } else {
     fn = fast_kernel(p->dtype, fftz::ct_log2(p->n), p->variant);
   }
@@ -146,7 +155,9 @@ int fftz_launch_pass(const fftz_pass_t *p, void *stream) {
     if (e != cudaSuccess) return (int)e;
     if (nopted[dev] < 96) opted[dev][nopted[dev]++] = fn;
   }
-  const dim3 block(p->variant == FFTZ_VAR_GENERIC_PP ? 256u : (unsigned)(p->tpc * p->tpt));
+  const dim3 block(p->variant == FFTZ_VAR_GENERIC_PP ? 256u
+                   : p->variant == FFTZ_VAR_MR       ? (unsigned)p->threads
+                                                     : (unsigned)(p->tpc * p->tpt));
   const size_t smem = (size_t)fftz_pass_smem_bytes(p);
   dim3 grid((unsigned)nblk);
   if (is_pipe(p)) {

@@ -1,0 +1,46 @@
+// Instances of the mixed-radix line kernel for one dtype (FZ_MR_T): plain
+// lines and four-step column passes for every radix, chirp passes (tables,
+// two sweeps) for radices without 11 and 13, which no convolution length has.
+#include "fft_mr.cuh"
+
+namespace fftz {
+
+// float: at most 1024 threads = 64 registers; double: 512 threads = 128
+// registers (a radix-16 butterfly holds 32 / 64 registers of data); the
+// radix-11 / 13 instances get 768 / 384 threads for their longer live ranges.
+template <typename T, bool BIG> __host__ __device__ constexpr int mr_lb() {
+  return sizeof(T) == 4 ? (BIG ? 768 : 1024) : (BIG ? 384 : 512);
+}
+
+// Measured on B200 against the ping-pong tiles this replaced (two buffers, one
+// prime radix a stage, 153 thread instructions a point at n = 1000; now 94):
+// n = 1000 x 32768 float 242 -> 135 us (2.16 -> 3.89 TB/s read + written),
+// 1920 x 4320 64 -> 49 us, 1080-point columns of four 1920 x 1080 images 117 ->
+// 56 us, 120000 = 375 x 320 in double x 64 (two passes) 307 -> 189 us. ncu at
+// n = 1000: issue 56%, shared-memory wavefronts 58%, DRAM 36% of peak -- issue and
+// the shared-memory pipe together, not HBM, bound it. Lines per CTA at n = 1000: 2
+// 166, 3 136, 4 146, 5 135 (fz_mr_shape's choice), 6 142 us.
+template <typename T, int FEAT, bool BIG>
+__global__ void __launch_bounds__(mr_lb<T, BIG>()) fft_mr_kernel(const __grid_constant__ fftz_pass_t P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  mr_tile<T, FEAT, BIG>(P, (int64_t)blockIdx.x, smem_raw);
+}
+
+}  // namespace fftz
+
+/* The mixed-radix kernel for a feature set (FEAT_MR_*), or NULL. */
+extern "C" const void *FZ_MR_GET(int feat, int big) {
+  using namespace fftz;
+  if (big) switch (feat) {
+      case 0: return (const void *)&fft_mr_kernel<FZ_MR_T, 0, true>;
+      case FEAT_MR_TW4: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TW4, true>;
+      default: return 0;
+    }
+  switch (feat) {
+    case 0: return (const void *)&fft_mr_kernel<FZ_MR_T, 0, false>;
+    case FEAT_MR_TW4: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TW4, false>;
+    case FEAT_MR_TABS: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TABS, false>;
+    case FEAT_MR_TABS | FEAT_MR_BLUE: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TABS | FEAT_MR_BLUE, false>;
+    default: return 0;
+  }
+}

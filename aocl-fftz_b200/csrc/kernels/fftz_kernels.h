@@ -54,6 +54,8 @@ enum fftz_out_kind {
 #define FFTZ_VAR_TC 8        /* 4096-point rows as two radix-64 tensor-core GEMM stages */
 #define FFTZ_VAR_FAST_REAL 9 /* packed real line: generic load/store phases, compile-time stages */
 #define FFTZ_VAR_GENERIC_PP 10 /* runtime radix list over two shared-memory buffers, 256 threads */
+#define FFTZ_VAR_MR 11       /* runtime radix list (2..16) in place in one shared-memory buffer */
+#define FFTZ_MR_STAGES 8     /* most stages of a mixed-radix line */
 
 /* pass flags */
 #define FFTZ_F_CONJ_IN    0x01 /* conjugate each loaded value (after kind decode) */
@@ -67,6 +69,21 @@ enum fftz_out_kind {
  * element k of column c at (k / 4) * 4 * ncols + 4 * c + k % 4 past the line */
 #define FFTZ_F_BLK4_OUT   0x80  /* the pass writes its output blocked */
 #define FFTZ_F_BLK4_IN    0x100 /* the pass reads its input blocked (rows = k) */
+
+/* Mixed-radix line (FFTZ_VAR_MR): digit strides M_s, the slots added per step
+ * of digit 0, and ceil(2^32 / d) (0 for d = 1) of the divisors that the
+ * stages' index maps need */
+typedef struct fftz_mr
+{
+    int32_t pad;                     /* slots between digit-0 blocks beyond M_0 */
+    int32_t m[FFTZ_MR_STAGES];       /* M_s = R_{s+1} ... R_{S-1} */
+    uint32_t mg_nb[FFTZ_MR_STAGES];  /* d = n / R_s: butterflies of a line */
+    uint32_t mg_m[FFTZ_MR_STAGES];   /* d = M_s */
+    uint32_t mg_b[FFTZ_MR_STAGES];   /* d = R_1 ... R_{s-1}: blocks per digit-0 step */
+    uint32_t mg_r[FFTZ_MR_STAGES];   /* d = R_s */
+    uint32_t mg_tpc;                 /* d = tpc */
+    int32_t big;                     /* a radix of 11 or 13 among them */
+} fftz_mr_t;
 
 typedef struct fftz_pass
 {
@@ -119,6 +136,8 @@ typedef struct fftz_pass
     int32_t test_tx_short;              /* fault injection (tests): TMA tiles expect this many bytes more
                                            than their copies deliver, so the bounded tile wait runs out */
     const int64_t *ind_in, *ind_out;
+    int32_t threads;                    /* FFTZ_VAR_MR: block size */
+    fftz_mr_t mr;
 } fftz_pass_t;
 
 /* Persistent DAG executor (fft_ragged.cu): one launch runs the CTA tiles of
@@ -231,6 +250,13 @@ int32_t fftz_smem_stride_cols(int dtype, int32_t nslots, int32_t tpc);
 
 /* Maximum dynamic SMEM bytes per CTA the kernels may use. */
 int64_t fftz_smem_limit(void);
+
+/* Mixed-radix kernel of one dtype for a feature set (1 four-step twiddles,
+ * 2 tables, 4 two sweeps; 2 and 4 without radices 11 and 13), or NULL. */
+const void *fftz_mr_kernel_f32(int feat, int big);
+const void *fftz_mr_kernel_f64(int feat, int big);
+/* Largest block of those kernels. */
+int fftz_mr_max_threads(int dtype, int big);
 
 /* Launches one pass on the given stream; returns a cudaError_t value. */
 int fftz_launch_pass(const fftz_pass_t *p, void *stream);

@@ -1,0 +1,180 @@
+"""CPU check of the mixed-radix tile (csrc/kernels/fft_mr.cuh): the planner's
+launch shape (fz_mr_shape, called in the built library) drives a restatement of
+the kernel's index maps, slot by slot. Every stage has to touch each slot of its
+lines exactly once and stay inside its shared memory, the reciprocals have to
+divide exactly, and the tile's result has to be numpy's FFT."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import aoclfftz_b200
+
+I32, I64, U32, VP = C.c_int32, C.c_int64, C.c_uint32, C.c_void_p
+MAXS, MAXB, MRS = 12, 8, 8
+VAR_MR, F_TW4, F_MID = 11, 0x04, 0x40
+
+
+class Mr(C.Structure):
+    _fields_ = [("pad", I32), ("m", I32 * MRS), ("mg_nb", U32 * MRS), ("mg_m", U32 * MRS), ("mg_b", U32 * MRS),
+                ("mg_r", U32 * MRS), ("mg_tpc", U32), ("big", I32)]
+
+
+class Pass(C.Structure):
+    """fftz_pass_t (csrc/kernels/fftz_kernels.h)."""
+    _fields_ = [("n", I32), ("nstages", I32), ("radix", I32 * MAXS), ("tw_off", I32 * MAXS), ("tpt", I32), ("tpc", I32),
+                ("sstride", I32), ("nload", I32), ("nstore", I32), ("in_kind", I32), ("out_kind", I32), ("in_mode", I32),
+                ("out_mode", I32), ("flags", I32), ("fuse_load", I32), ("fuse_store", I32), ("variant", I32),
+                ("dtype", I32), ("nbdims", I32), ("ies", I64), ("oes", I64), ("ntf", I64), ("bdim", I64 * MAXB),
+                ("ibs", I64 * MAXB), ("obs", I64 * MAXB), ("tw4_n", I64), ("tw4_l", I64), ("pre_n", I64),
+                ("pre_es", I64), ("pre_cs", I64), ("post_n", I64), ("post_es", I64), ("post_cs", I64), ("mid_cs", I64),
+                ("scale", C.c_double), ("in_", VP), ("out", VP), ("tw", VP), ("tw4_hi", VP), ("tw4_lo", VP),
+                ("pre_tab", VP), ("post_tab", VP), ("mid_tab", VP), ("rtw", VP), ("src_buf", I32), ("dst_buf", I32),
+                ("ind_dim", I32), ("use_tma", I32), ("smem_tw", I32), ("test_tx_short", I32), ("ind_in", VP),
+                ("ind_out", VP), ("threads", I32), ("mr", Mr)]
+
+
+def shape(n, dtype=0, col=False, two=False, tw4=False, ntf=100000, tpc=0):
+    lib = aoclfftz_b200.load()
+    lib.fftz_pass_smem_bytes.restype = I64
+    lib.fftz_smem_limit.restype = I64
+    p = Pass(n=n, dtype=dtype, ntf=ntf, in_mode=int(col), out_mode=int(col), nbdims=1,
+             flags=(F_MID if two else 0) | (F_TW4 if tw4 else 0))
+    assert lib.fz_mr_shape(C.byref(p), tpc) == 0
+    assert p.variant == VAR_MR and 1 <= p.tpc <= ntf and 1 <= p.threads <= lib.fftz_mr_max_threads(dtype, p.mr.big)
+    assert lib.fftz_pass_smem_bytes(C.byref(p)) <= lib.fftz_smem_limit()
+    assert int(np.prod(p.radix[: p.nstages])) == n
+    return p
+
+
+def div(x, m):
+    return (x.astype(np.uint64) * np.uint64(m) >> np.uint64(32)).astype(np.int64) if m else x
+
+
+def exact_div(x, m, d):
+    q = div(x, m)
+    assert np.array_equal(q, x // d)
+    return q
+
+
+def items(p, s, col):
+    """(line, position) of every item of a boundary stage."""
+    nb = p.n // p.radix[s]
+    i = np.arange(p.tpc * nb)
+    if col:
+        x = exact_div(i, p.mr.mg_tpc, p.tpc)
+        return i - x * p.tpc, x
+    q = exact_div(i, p.mr.mg_nb[s], nb)
+    return q, i - q * nb
+
+
+def mid_slots(p, s):
+    R, M = p.radix[s], p.mr.m[s]
+    nb = p.n // R
+    i = np.arange(p.tpc * nb)
+    q = exact_div(i, p.mr.mg_nb[s], nb)
+    j = i - q * nb
+    b = exact_div(j, p.mr.mg_m[s], M)
+    B = int(np.prod(p.radix[1:s]))
+    return q * p.sstride + j + b * M * (R - 1) + exact_div(b, p.mr.mg_b[s], B) * p.mr.pad, j - b * M
+
+
+def last_slots(p, line, K):
+    o, q = np.zeros_like(K), K
+    for s in range(p.nstages - 1):
+        R, M = p.radix[s], p.mr.m[s]
+        nxt = exact_div(q, p.mr.mg_r[s], R)
+        o, q = o + (q - nxt * R) * (M + p.mr.pad if s == 0 else M), nxt
+    return line * p.sstride + o
+
+
+def twiddle(R, M, rest):
+    return np.exp(-2j * np.pi * np.outer(np.arange(R), rest) / (R * M))
+
+
+def dft(v):
+    return np.fft.fft(v, axis=0)
+
+
+def check_slots(p, slots):
+    assert slots.min() >= 0 and slots.max() < p.tpc * p.sstride
+    assert np.unique(slots).size == slots.size == p.tpc * p.n
+
+
+def simulate(p, x, mid=None):
+    S, n = p.nstages, p.n
+    sd = np.full(p.tpc * p.sstride, np.nan + 0j)
+    y = np.full((p.tpc, n), np.nan + 0j)
+    R, M = p.radix[0], n // p.radix[0]
+    r = np.arange(R)[:, None]
+    if S == 1:
+        return np.fft.fft(x, axis=1)
+    line, rest = items(p, 0, p.in_mode)
+    v = dft(x[line, rest + r * M]) * twiddle(R, M, rest)
+    first = line * p.sstride + rest + r * (M + p.mr.pad)
+    check_slots(p, first)
+    sd[first] = v
+    for s in range(1, S - 1):
+        Rs, Ms = p.radix[s], p.mr.m[s]
+        base, rs = mid_slots(p, s)
+        a = base + np.arange(Rs)[:, None] * Ms
+        check_slots(p, a)
+        sd[a] = dft(sd[a]) * twiddle(Rs, Ms, rs)
+    Rl = p.radix[S - 1]
+    nb = n // Rl
+    line, K = items(p, S - 1, p.out_mode if mid is None else 0)
+    a = last_slots(p, line, K) + np.arange(Rl)[:, None]
+    check_slots(p, a)
+    v = dft(sd[a])
+    if mid is None:
+        y[line, K + np.arange(Rl)[:, None] * nb] = v
+        return y
+    sd[a] = dft(np.conj(v) * mid[K + np.arange(Rl)[:, None] * nb])
+    for s in range(S - 2, 0, -1):
+        Rs, Ms = p.radix[s], p.mr.m[s]
+        base, rs = mid_slots(p, s)
+        a = base + np.arange(Rs)[:, None] * Ms
+        sd[a] = dft(sd[a] * twiddle(Rs, Ms, rs))
+    line, rest = items(p, 0, p.out_mode)
+    v = dft(sd[line * p.sstride + rest + r * (M + p.mr.pad)] * twiddle(R, M, rest))
+    y[line, rest + r * M] = v
+    return y
+
+
+# one-stage lines, two to five stages, every radix, odd and even, the longest of each dtype
+SIZES = [3, 11, 13, 14, 15, 16, 18, 35, 77, 100, 169, 360, 375, 1000, 1080, 1920, 2187, 2401, 4096, 11011, 14400, 15625,
+         28000, 28800]
+
+
+@pytest.mark.parametrize("col", [False, True])
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("n", SIZES)
+def test_tile_is_the_transform(n, dtype, col):
+    lib = aoclfftz_b200.load()
+    if not lib.fz_mr_fits(dtype, I64(n)):
+        assert n * (8 if dtype == 0 else 16) > 220 * 1024
+        return
+    p = shape(n, dtype, col)
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((p.tpc, n)) + 1j * rng.standard_normal((p.tpc, n))
+    y = simulate(p, x)
+    ref = np.fft.fft(x, axis=1)
+    assert np.linalg.norm(y - ref) <= 1e-13 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [4, 6, 16, 40, 225, 2100, 20160])
+def test_two_sweeps_are_the_convolution(n):
+    p = shape(n, two=True)
+    assert p.nstages >= 2
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((p.tpc, n)) + 1j * rng.standard_normal((p.tpc, n))
+    mid = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    ref = np.fft.fft(np.conj(np.fft.fft(x, axis=1)) * mid, axis=1)
+    assert np.linalg.norm(simulate(p, x, mid) - ref) <= 1e-13 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("ntf,tpc", [(1, 0), (3, 0), (5, 2), (700, 0), (100000, 3)])
+def test_lines_per_cta_follow_the_batch_and_the_hint(ntf, tpc):
+    p = shape(360, ntf=ntf, tpc=tpc, tw4=True)
+    assert p.tpc <= ntf and (tpc == 0 or p.tpc == tpc)
+    assert p.tpc == 1 or ntf // p.tpc >= 296 or tpc
