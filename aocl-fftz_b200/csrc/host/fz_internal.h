@@ -139,7 +139,7 @@ int64_t fz_blob_reserve(fz_blob *b, size_t bytes);
 int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off);
 /* four-step factor tables W_N^(hi*L), W_N^lo in the working dtype */
 int fz_tw4_tables(fz_blob *b, int dtype, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo);
-/* Bluestein tables for length n, pow2 convolution length m, direction */
+/* Bluestein tables for length n, 7-smooth convolution length m, direction */
 int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int direction, int64_t *off_pre,
                         int64_t *off_post, int64_t *off_mid);
 /* appends the row-major copy T'[k1 * n2 + k2] = T[k1 + n1 * k2] of the table
@@ -154,6 +154,8 @@ int64_t fz_real_twiddles(fz_blob *b, int dtype, int64_t M);
 /* ---- mixed-radix lines (mixed.c) ---- */
 int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost);
 int fz_mr_fits(int dtype, int64_t n);
+int64_t fz_mr_blue_len(int dtype, int64_t n);
+int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t *n1, int64_t *n2);
 int fz_mr_shape(fftz_pass_t *k, int want_tpc);
 int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k);
 

@@ -86,6 +86,67 @@ int fz_mr_fits(int dtype, int64_t n)
     return fz_mr_radices(n, 1, r, NULL) > 0;
 }
 
+/* the smallest product of 2, 3, 5 and 7 that is at least n */
+static int64_t next_smooth7(int64_t n)
+{
+    for (;; n++)
+    {
+        int64_t m = n;
+        while (m % 2 == 0) m /= 2;
+        while (m % 3 == 0) m /= 3;
+        while (m % 5 == 0) m /= 5;
+        while (m % 7 == 0) m /= 7;
+        if (m == 1) return n;
+    }
+}
+
+/* Convolution length of a chirp-z transform of n points in one tile: the
+ * 7-smooth m >= 2n - 1 with the fewest issue slots over both sweeps (a longer m
+ * with fewer stages beats the nearest one); 0 when none fits a CTA. */
+int64_t fz_mr_blue_len(int dtype, int64_t n)
+{
+    int32_t r[FFTZ_MR_STAGES];
+    int64_t best = 0;
+    double score = 0, c;
+    const int64_t need = 2 * n - 1;
+    if (need * (dtype == 0 ? 8 : 16) > fftz_smem_limit()) return 0;
+    for (int64_t m = next_smooth7(need < 4 ? 4 : need); m <= need + need / 4 + 4; m = next_smooth7(m + 1))
+        if (fz_mr_fits(dtype, m) && fz_mr_radices(m, 2, r, &c) > 1 && (!best || (double)m * c < score))
+        {
+            best = m;
+            score = (double)m * c;
+        }
+    return best;
+}
+
+/* Convolution length m = n1 * n2 of a chirp-z transform in three passes: the
+ * cheapest of the first 7-smooth lengths from 2n - 1 on, both factors one tile
+ * and n2 of at least two stages, within a factor of four of each other. */
+int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t *n1, int64_t *n2)
+{
+    int32_t r[FFTZ_MR_STAGES];
+    int64_t best = 0, m = 2 * n - 2;
+    double score = 0, ca, cb;
+    for (int tries = 0; tries < 64 && (tries < 12 || !best); tries++)
+    {
+        m = next_smooth7(m + 1);
+        for (int64_t a = 2; a * a <= 4 * m; a++)
+        {
+            const int64_t b = m / a;
+            if (m % a || a > 4 * b || b > 4 * a || !fz_mr_fits(dtype, a) || !fz_mr_fits(dtype, b)) continue;
+            if (fz_mr_radices(a, 1, r, &ca) < 1 || fz_mr_radices(b, 2, r, &cb) < 2) continue;
+            if (!best || (double)m * (ca + cb) < score)
+            {
+                best = m;
+                score = (double)m * (ca + cb);
+                *n1 = a;
+                *n2 = b;
+            }
+        }
+    }
+    return best;
+}
+
 /* Slot of item i (of one line, or of tpc lines when col) of stage s; first /
  * last are the maps of the HBM-side stages. */
 static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)

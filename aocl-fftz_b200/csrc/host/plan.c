@@ -14,7 +14,7 @@
  *          (column FFTs with the W_n^{j2 k1} twiddle fused into their store,
  *           then row FFTs whose store performs the transpose)
  *   any prime factor > 13
- *       -> Bluestein over a power-of-two convolution length m >= 2n - 1, in one
+ *       -> Bluestein over a 7-smooth convolution length m >= 2n - 1, in one
  *          kernel when m fits shared memory, in three passes otherwise
  *   N-D -> one line pass per dimension (dims[0] first, the rest in place)
  *   real, dims[0] even -> packed: n0/2-point complex FFT with the Hermitian
@@ -247,7 +247,7 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
     p->dst = dst;
     if (set_batch(k, b, nb, keep_first)) return NULL;
     set_modes(k);
-    const int fast = !generic_only(pl) && is_pow2(n) && n >= 2 && n <= fast_max_n(pl);
+    const int fast = !generic_only(pl) && is_pow2(n) && n >= 2 && n <= fast_max_n(pl) && !(variant_bits & 8);
     int maxthr;
     if (fast)
     {
@@ -616,22 +616,44 @@ static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_d
     return fourstep_lines(pl, n, n1, n2, ies, oes, b, nb, src, dst, flags, 0, 0, hi, lo, L, S);
 }
 
-/* Bluestein (chirp-z) over a power-of-two m >= 2n - 1 (the reference pads to
- * a 13-smooth m, core/common/bluestein_utils.c:39-67; a power of two keeps
- * every sub-transform on the compile-time kernels). */
+/* Bluestein (chirp-z) over a 7-smooth m >= 2n - 1 on mixed-radix tiles (the
+ * reference pads to a 13-smooth m, core/common/bluestein_utils.c:39-67). The
+ * ragged executor and kernel_family 12 keep a power of two, whose
+ * sub-transforms run on the compile-time kernels. A convolution that fits a
+ * CTA (m up to 28672 float, 14400 double) is one kernel, which reads and writes
+ * HBM once: measured on B200, n = 10007 float x 512, m = 32768 in three passes 452
+ * us, m = 20736 in three passes 317 us, in one kernel 142 us; one line 52, 52
+ * and 35 us. Only a few double lines near the limit are faster in three passes
+ * (n = 7001: 45 us in one kernel against 37 us up to 32 lines, 46 against 66 us
+ * for 64), both faster than three passes over a power of two (58 us). */
 static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_dim *b, int nb, int src, int dst)
 {
-    int64_t m = 1;
-    while (m < 2 * n - 1) m *= 2;
+    const int mixed = mixed_lines(pl), vb = mixed ? 2 | 8 : 2; /* line_pass bits: tables, mixed-radix tiles */
+    int64_t m = 1, n1 = 0, n2 = 0;
+    int one = 0;
+    if (mixed)
+    {
+        one = (m = fz_mr_blue_len(pl->dtype, n)) > 0;
+        if (!one && (m = fz_mr_blue_split(pl->dtype, n, &n1, &n2)) == 0)
+        {
+            fz_set_error("length %lld has no chirp-z plan", (long long)n);
+            return -1;
+        }
+    }
+    else
+    {
+        while (m < 2 * n - 1) m *= 2;
+        one = m >= 4 && single_pass_ok(pl, m);
+    }
     int64_t pre, post, mid;
     if (fz_bluestein_tables(&pl->blob, pl->dtype, n, m, pl->direction, &pre, &post, &mid)) return -1;
     const int bwd = pl->direction == 1;
-    if (m >= 4 && single_pass_ok(pl, m))
+    if (one)
     {
         fz_pass *p = line_pass(pl, m, ies, oes, b, nb, 0, src, dst,
                                (bwd ? FFTZ_F_CONJ_IN : FFTZ_F_CONJ_OUT) | FFTZ_F_PRE_TAB | FFTZ_F_POST_TAB |
                                    FFTZ_F_MID_TAB,
-                               2 | 4);
+                               vb | 4);
         if (!p) return -1;
         p->k.pre_n = n;
         p->k.pre_es = 1;
@@ -647,8 +669,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
     /* three passes through S0 / S1: A (column FFTs of the chirped, padded
      * input), M (row FFTs, spectrum product, row FFTs of the second FFT_m),
      * D (row FFTs of the second FFT_m, output chirp) */
-    int64_t n1, n2;
-    if (choose_split(pl, m, &n1, &n2)) return -1;
+    if (!mixed && choose_split(pl, m, &n1, &n2)) return -1;
     int64_t lines = lines_of(b, nb);
     const int S0 = new_scratch(pl, m * lines), S1 = new_scratch(pl, m * lines);
     if (S0 < 0 || S1 < 0) return -1;
@@ -668,7 +689,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         so *= b[i].n;
     }
     fz_pass *pa = line_pass(pl, n1, n2 * ies, n2, bb, nb + 1, 1, src, S0,
-                            (bwd ? FFTZ_F_CONJ_IN : 0) | FFTZ_F_PRE_TAB | FFTZ_F_TW4, 2);
+                            (bwd ? FFTZ_F_CONJ_IN : 0) | FFTZ_F_PRE_TAB | FFTZ_F_TW4, vb);
     if (!pa) return -1;
     pa->k.pre_n = n;
     pa->k.pre_es = n2;
@@ -697,7 +718,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         bb[i + 1].os = so;
         so *= b[i].n;
     }
-    fz_pass *pm = line_pass(pl, n2, 1, n1, bb, nb + 1, 1, S0, S1, FFTZ_F_MID_TAB | FFTZ_F_TW4, 2 | 4);
+    fz_pass *pm = line_pass(pl, n2, 1, n1, bb, nb + 1, 1, S0, S1, FFTZ_F_MID_TAB | FFTZ_F_TW4, vb | 4);
     if (!pm) return -1;
     pm->k.mid_cs = n2;
     pm->off_mid = midT;
@@ -720,7 +741,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         so *= b[i].n;
     }
     fz_pass *pd = line_pass(pl, n1, 1, n2 * oes, bb, nb + 1, 1, S1, dst,
-                            (bwd ? 0 : FFTZ_F_CONJ_OUT) | FFTZ_F_POST_TAB, 2);
+                            (bwd ? 0 : FFTZ_F_CONJ_OUT) | FFTZ_F_POST_TAB, vb);
     if (!pd) return -1;
     pd->k.post_n = n;
     pd->k.post_es = n2;

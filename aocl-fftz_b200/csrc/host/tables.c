@@ -46,6 +46,35 @@ static void w_n(int64_t r, int64_t N, double *re, double *im)
     *im = (double)(-s);
 }
 
+/* All N roots exp(-2 pi i r / N), interleaved, by malloc (NULL on failure):
+ * w_n on the part of the circle that the reflections at N / 2, N / 4 and N / 8
+ * leave (each where it divides N), mirrored to the rest. */
+static double *roots(int64_t N)
+{
+    double *w = (double *)malloc(sizeof(double) * 2 * (size_t)N);
+    if (!w) return NULL;
+    const int64_t half = N / 2, quarter = N % 2 == 0 ? N / 4 : half, eighth = N % 4 == 0 ? N / 8 : quarter;
+    for (int64_t r = 0; r <= eighth; r++) w_n(r, N, &w[2 * r], &w[2 * r + 1]);
+    if (N % 4 == 0) /* W^{N/4 - r} = -i conj(W^r) */
+        for (int64_t r = eighth + 1; r <= N / 4; r++)
+        {
+            w[2 * r] = -w[2 * (N / 4 - r) + 1];
+            w[2 * r + 1] = -w[2 * (N / 4 - r)];
+        }
+    if (N % 2 == 0) /* W^{N/2 - r} = -conj(W^r) */
+        for (int64_t r = quarter + 1; r <= half; r++)
+        {
+            w[2 * r] = -w[2 * (half - r)];
+            w[2 * r + 1] = w[2 * (half - r) + 1];
+        }
+    for (int64_t r = half + 1; r < N; r++) /* W^{N - r} = conj(W^r) */
+    {
+        w[2 * r] = w[2 * (N - r)];
+        w[2 * r + 1] = -w[2 * (N - r) + 1];
+    }
+    return w;
+}
+
 int64_t fz_blob_reserve(fz_blob *b, size_t bytes)
 {
     size_t off = (b->len + 255) & ~(size_t)255; /* 256-byte aligned tables */
@@ -101,21 +130,22 @@ int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32
     size_t esz = dtype == 0 ? 8 : 16;
     int64_t off = fz_blob_reserve(b, (size_t)total * esz);
     if (off < 0) return -1;
-    ns = 1;
     put_c(b, off, dtype, 0, 1.0, 0.0);
-    for (int s = 0; s < nstages; s++)
+    if (nstages < 2) return off;
+    /* every W_{Ns*R}^{k*r} is a root of order n = the product of the radices */
+    double *w = roots(ns);
+    if (!w) return -1;
+    const int64_t N = ns;
+    ns = radix[0];
+    for (int s = 1; s < nstages; s++)
     {
-        int64_t R = radix[s];
-        if (s > 0)
-            for (int64_t r = 1; r < R; r++)
-                for (int64_t k = 0; k < ns; k++)
-                {
-                    double re, im;
-                    w_n(k * r, ns * R, &re, &im);
-                    put_c(b, off, dtype, tw_off[s] + (r - 1) * ns + k, re, im);
-                }
+        const int64_t R = radix[s], step = N / (ns * R);
+        for (int64_t r = 1; r < R; r++)
+            for (int64_t k = 0; k < ns; k++)
+                put_c(b, off, dtype, tw_off[s] + (r - 1) * ns + k, w[2 * (k * r * step)], w[2 * (k * r * step) + 1]);
         ns *= R;
     }
+    free(w);
     return off;
 }
 
@@ -151,42 +181,76 @@ int fz_tw4_tables(fz_blob *b, int dtype, int64_t N, int64_t *L, int64_t *off_hi,
     return 0;
 }
 
-/* in-place iterative radix-2 FFT in double (forward), m a power of two */
-static void host_fft_pow2(double *x, int64_t m)
+/* Forward FFT in double, m a product of 2, 3, 5 and 7: Stockham stages of 4 and
+ * the prime factors between x and a second buffer. Returns 0, or -1 on allocation
+ * failure. */
+static int host_fft(double *x, int64_t m)
 {
-    for (int64_t i = 1, j = 0; i < m; i++)
+    double *w = roots(m), *y = (double *)malloc(sizeof(double) * 2 * (size_t)m);
+    double *src = x, *dst = y;
+    if (!w || !y)
     {
-        int64_t bit = m >> 1;
-        for (; j & bit; bit >>= 1) j ^= bit;
-        j ^= bit;
-        if (i < j)
+        free(w);
+        free(y);
+        return -1;
+    }
+    int64_t n = m, st = 1; /* length still to transform, transforms side by side */
+    while (n > 1)
+    {
+        const int p = n % 4 == 0 ? 4 : n % 2 == 0 ? 2 : n % 3 == 0 ? 3 : n % 5 == 0 ? 5 : 7;
+        const int64_t h = n / p;
+        double e[7][2]; /* W_p^j */
+        for (int j = 0; j < p; j++)
         {
-            double t0 = x[2 * i], t1 = x[2 * i + 1];
-            x[2 * i] = x[2 * j];
-            x[2 * i + 1] = x[2 * j + 1];
-            x[2 * j] = t0;
-            x[2 * j + 1] = t1;
+            e[j][0] = w[2 * (j * (m / p))];
+            e[j][1] = w[2 * (j * (m / p)) + 1];
         }
-    }
-    double *w = (double *)malloc(sizeof(double) * (size_t)m);
-    if (!w) return;
-    for (int64_t k = 0; k < m / 2; k++) w_n(k, m, &w[2 * k], &w[2 * k + 1]);
-    for (int64_t len = 2; len <= m; len <<= 1)
-    {
-        int64_t step = m / len;
-        for (int64_t i = 0; i < m; i += len)
-            for (int64_t k = 0; k < len / 2; k++)
+        for (int64_t k = 0; k < h; k++)
+            for (int64_t q = 0; q < st; q++)
             {
-                double wr = w[2 * k * step], wi = w[2 * k * step + 1];
-                double *a = x + 2 * (i + k), *c = x + 2 * (i + k + len / 2);
-                double tr = c[0] * wr - c[1] * wi, ti = c[0] * wi + c[1] * wr;
-                c[0] = a[0] - tr;
-                c[1] = a[1] - ti;
-                a[0] += tr;
-                a[1] += ti;
+                double v[7][2], o[7][2];
+                for (int j = 0; j < p; j++)
+                {
+                    v[j][0] = src[2 * (q + st * (k + j * h))];
+                    v[j][1] = src[2 * (q + st * (k + j * h)) + 1];
+                }
+                if (p == 4)
+                {
+                    const double ar = v[0][0] + v[2][0], ai = v[0][1] + v[2][1], br = v[0][0] - v[2][0],
+                                 bi = v[0][1] - v[2][1], cr = v[1][0] + v[3][0], ci = v[1][1] + v[3][1],
+                                 dr = v[1][0] - v[3][0], di = v[1][1] - v[3][1];
+                    o[0][0] = ar + cr, o[0][1] = ai + ci, o[2][0] = ar - cr, o[2][1] = ai - ci;
+                    o[1][0] = br + di, o[1][1] = bi - dr, o[3][0] = br - di, o[3][1] = bi + dr;
+                }
+                else
+                    for (int r = 0; r < p; r++)
+                    {
+                        o[r][0] = v[0][0];
+                        o[r][1] = v[0][1];
+                        for (int j = 1, i = r; j < p; j++, i = i + r >= p ? i + r - p : i + r)
+                        {
+                            o[r][0] += v[j][0] * e[i][0] - v[j][1] * e[i][1];
+                            o[r][1] += v[j][0] * e[i][1] + v[j][1] * e[i][0];
+                        }
+                    }
+                for (int r = 0; r < p; r++) /* output r of the butterfly, times W_n^{k r} */
+                {
+                    const double *t = w + 2 * (k * r * st);
+                    double *d = dst + 2 * (q + st * (p * k + r));
+                    d[0] = o[r][0] * t[0] - o[r][1] * t[1];
+                    d[1] = o[r][0] * t[1] + o[r][1] * t[0];
+                }
             }
+        double *sw = src;
+        src = dst;
+        dst = sw;
+        st *= p;
+        n = h;
     }
+    if (src != x) memcpy(x, src, sizeof(double) * 2 * (size_t)m);
     free(w);
+    free(y);
+    return 0;
 }
 
 int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int direction, int64_t *off_pre,
@@ -204,11 +268,20 @@ int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int directi
         return -1;
     }
     const int64_t n2 = 2 * n;
+    double *wc = roots(n2);
+    if (!wc)
+    {
+        free(c);
+        free(bb);
+        return -1;
+    }
     for (int64_t j = 0; j < n; j++)
     {
         int64_t sq = (int64_t)(((unsigned __int128)j * (unsigned __int128)j) % (unsigned __int128)n2);
-        w_n(sq, n2, &c[2 * j], &c[2 * j + 1]);
+        c[2 * j] = wc[2 * sq];
+        c[2 * j + 1] = wc[2 * sq + 1];
     }
+    free(wc);
     /* b_j = conj(c_j) at j and m - j, zero between */
     for (int64_t j = 0; j < n; j++)
     {
@@ -220,7 +293,12 @@ int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int directi
             bb[2 * (m - j) + 1] = -c[2 * j + 1];
         }
     }
-    host_fft_pow2(bb, m);
+    if (host_fft(bb, m))
+    {
+        free(c);
+        free(bb);
+        return -1;
+    }
     *off_pre = fz_blob_reserve(b, (size_t)n * esz);
     *off_post = fz_blob_reserve(b, (size_t)n * esz);
     *off_mid = fz_blob_reserve(b, (size_t)m * esz);
@@ -250,12 +328,10 @@ int64_t fz_real_twiddles(fz_blob *b, int dtype, int64_t M)
     size_t esz = dtype == 0 ? 8 : 16;
     int64_t off = fz_blob_reserve(b, (size_t)(M + 1) * esz);
     if (off < 0) return -1;
-    for (int64_t k = 0; k < M; k++)
-    {
-        double re, im;
-        w_n(k, 2 * M, &re, &im);
-        put_c(b, off, dtype, k, re, im);
-    }
+    double *w = roots(2 * M);
+    if (!w) return -1;
+    for (int64_t k = 0; k < M; k++) put_c(b, off, dtype, k, w[2 * k], w[2 * k + 1]);
+    free(w);
     put_c(b, off, dtype, M, -1.0, 0.0);
     return off;
 }
