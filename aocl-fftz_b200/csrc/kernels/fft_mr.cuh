@@ -33,6 +33,7 @@ template <typename T> struct MrTile {
   typename Cplx<T>::type *sd;   // tpc lines, P.sstride apart
   typename Cplx<T>::type *stp;  // four-step factors W^{col nb r}: 16 per line
   const int64_t *s_in, *s_out, *s_col;
+  int nl;                       // lines of the tile that exist (the last tile may be short)
 };
 
 // Four-step factor of output K of column col: col * K < tw4_n, both below
@@ -50,7 +51,6 @@ __device__ __forceinline__ void mr_store(const fftz_pass_t &P, const MrTile<T> &
                                          int p, int K, int nb) {
   typedef typename Cplx<T>::type T2;
   const int64_t col = t.s_col[p];
-  if (col < 0) return;
   const int64_t oes = P.oes;
   T2 *g = (T2 *)P.out + t.s_out[p] + (int64_t)K * oes;
   const int64_t st = (int64_t)nb * oes;
@@ -106,7 +106,7 @@ __device__ __forceinline__ void mr_load(const fftz_pass_t &P, const MrTile<T> &t
     for (int r = 0; r < R; r++) {
       const int li = l0 + r * ls;
       T2 x = zero2<T2>();
-      if (col >= 0 && li < pn) {
+      if (li < pn) {
         x = g[r * st];
         if (cj) x.y = -x.y;
         if (pre) x = cmul(x, __ldg((const T2 *)P.pre_tab + li));
@@ -116,10 +116,8 @@ __device__ __forceinline__ void mr_load(const fftz_pass_t &P, const MrTile<T> &t
   } else {
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      T2 x = zero2<T2>();
-      if (col >= 0) x = g[r * st];
-      if (cj) x.y = -x.y;
-      v[r] = x;
+      v[r] = g[r * st];
+      if (cj) v[r].y = -v[r].y;
     }
   }
 }
@@ -127,7 +125,7 @@ __device__ __forceinline__ void mr_load(const fftz_pass_t &P, const MrTile<T> &t
 // item i of a boundary stage (nb butterflies a line) -> line p, position x
 __device__ __forceinline__ void mr_item(const fftz_pass_t &P, int mode, int i, int nb, uint32_t mnb, int &p, int &x) {
   if (mode == 1) {
-    x = mr_div(i, P.mr.mg_tpc);
+    x = mr_div(i, P.mr.mg_tpc);  // the caller skips p >= nl
     p = i - x * P.tpc;
   } else {
     p = mr_div(i, mnb);
@@ -138,19 +136,26 @@ __device__ __forceinline__ void mr_item(const fftz_pass_t &P, int mode, int i, i
 template <typename T, int R>
 __device__ __forceinline__ void mr_twiddle(const typename Cplx<T>::type *tw, typename Cplx<T>::type (&v)[R], int M,
                                            int rest) {
+  // uniform row pointers plus one 32-bit lane offset
+  const uint32_t o = (uint32_t)rest * (uint32_t)sizeof(*tw);
 #pragma unroll
-  for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(tw + (r - 1) * M + rest));
+  for (int r = 1; r < R; r++) {
+    const char *row = (const char *)(tw + (r - 1) * M);
+    v[r] = cmul(v[r], __ldg((const typename Cplx<T>::type *)(row + o)));
+  }
 }
 
 // Stage 0: HBM -> shared memory (S > 1), or HBM -> HBM (S == 1).
 template <typename T, int R, int FEAT>
 __device__ __forceinline__ void mr_first(const fftz_pass_t &P, const MrTile<T> &t) {
   typedef typename Cplx<T>::type T2;
-  const int M = P.n / R, total = P.tpc * M, S0 = M + P.mr.pad;
+  const int M = P.n / R, S0 = M + P.mr.pad;
   const T2 *tw = (const T2 *)P.tw + P.tw_off[0];
+  const int total = (P.in_mode == 1 ? P.tpc : t.nl) * M;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     int p, rest;
     mr_item(P, P.in_mode, i, M, P.mr.mg_nb[0], p, rest);
+    if (p >= t.nl) continue;
     T2 v[R];
     mr_load<T, R, FEAT>(P, t, v, p, rest, M);
     Dft<R>::template apply<T, T2>(v);
@@ -163,7 +168,7 @@ __device__ __forceinline__ void mr_first(const fftz_pass_t &P, const MrTile<T> &
 template <typename T, int R, int FEAT>
 __device__ __forceinline__ void mr_single(const fftz_pass_t &P, const MrTile<T> &t) {
   typedef typename Cplx<T>::type T2;
-  for (int p = threadIdx.x; p < P.tpc; p += blockDim.x) {
+  for (int p = threadIdx.x; p < t.nl; p += blockDim.x) {
     T2 v[R];
     mr_load<T, R, FEAT>(P, t, v, p, 0, 1);
     Dft<R>::template apply<T, T2>(v);
@@ -175,7 +180,7 @@ __device__ __forceinline__ void mr_single(const fftz_pass_t &P, const MrTile<T> 
 template <typename T, int R, bool DIT>
 __device__ __forceinline__ void mr_mid(const fftz_pass_t &P, const MrTile<T> &t, int s, int M) {
   typedef typename Cplx<T>::type T2;
-  const int nb = P.n / R, total = P.tpc * nb, step = M * (R - 1), pad = P.mr.pad;
+  const int nb = P.n / R, total = t.nl * nb, step = M * (R - 1), pad = P.mr.pad;
   const uint32_t mnb = P.mr.mg_nb[s], mM = P.mr.mg_m[s], mB = P.mr.mg_b[s];
   const T2 *tw = (const T2 *)P.tw + P.tw_off[s];
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
@@ -197,25 +202,27 @@ __device__ __forceinline__ void mr_mid(const fftz_pass_t &P, const MrTile<T> &t,
 
 // Slot of the last stage's butterfly K = k_0 + R_0 (k_1 + R_1 (...)).
 __device__ __forceinline__ int mr_slot(const fftz_pass_t &P, int K) {
-  int M = P.n, o = 0;
-  for (int s = 0; s < P.nstages - 1; s++) {
-    const int R = P.radix[s];
-    M = P.mr.m[s];
-    const int q = mr_div(K, P.mr.mg_r[s]);
-    o += (K - q * R) * (s == 0 ? M + P.mr.pad : M);
-    K = q;
+  const int S0 = P.mr.m[0] + P.mr.pad, S = P.nstages;
+  if (S == 2) return K * S0;
+  int q = mr_div(K, P.mr.mg_r[0]);
+  int o = (K - q * P.radix[0]) * S0;
+  for (int s = 1; s < S - 2; s++) {
+    const int x = mr_div(q, P.mr.mg_r[s]);
+    o += (q - x * P.radix[s]) * P.mr.m[s];
+    q = x;
   }
-  return o;
+  return o + q * P.mr.m[S - 2];
 }
 
 // Last stage: shared memory -> HBM, butterflies in output order.
 template <typename T, int R, int FEAT>
 __device__ __forceinline__ void mr_last(const fftz_pass_t &P, const MrTile<T> &t, int s) {
   typedef typename Cplx<T>::type T2;
-  const int nb = P.n / R, total = P.tpc * nb;
+  const int nb = P.n / R, total = (P.out_mode == 1 ? P.tpc : t.nl) * nb;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     int p, K;
     mr_item(P, P.out_mode, i, nb, P.mr.mg_nb[s], p, K);
+    if (p >= t.nl) continue;
     const T2 *d = t.sd + p * P.sstride + mr_slot(P, K);
     T2 v[R];
 #pragma unroll
@@ -230,7 +237,7 @@ __device__ __forceinline__ void mr_last(const fftz_pass_t &P, const MrTile<T> &t
 template <typename T, int R>
 __device__ __forceinline__ void mr_product(const fftz_pass_t &P, const MrTile<T> &t, int s) {
   typedef typename Cplx<T>::type T2;
-  const int nb = P.n / R, total = P.tpc * nb;
+  const int nb = P.n / R, total = t.nl * nb;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int p = mr_div(i, P.mr.mg_nb[s]);
     const int K = i - p * nb;
@@ -239,8 +246,7 @@ __device__ __forceinline__ void mr_product(const fftz_pass_t &P, const MrTile<T>
 #pragma unroll
     for (int r = 0; r < R; r++) v[r] = d[r];
     Dft<R>::template apply<T, T2>(v);
-    const int64_t col = t.s_col[p] < 0 ? 0 : t.s_col[p];
-    const T2 *mt = (const T2 *)P.mid_tab + col * P.mid_cs + K;
+    const T2 *mt = (const T2 *)P.mid_tab + t.s_col[p] * P.mid_cs + K;
 #pragma unroll
     for (int r = 0; r < R; r++) {
       T2 x = v[r];
@@ -257,11 +263,13 @@ __device__ __forceinline__ void mr_product(const fftz_pass_t &P, const MrTile<T>
 template <typename T, int R, int FEAT>
 __device__ __forceinline__ void mr_dit_last(const fftz_pass_t &P, const MrTile<T> &t) {
   typedef typename Cplx<T>::type T2;
-  const int M = P.n / R, total = P.tpc * M, S0 = M + P.mr.pad;
+  const int M = P.n / R, S0 = M + P.mr.pad;
   const T2 *tw = (const T2 *)P.tw + P.tw_off[0];
+  const int total = (P.out_mode == 1 ? P.tpc : t.nl) * M;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     int p, rest;
     mr_item(P, P.out_mode, i, M, P.mr.mg_nb[0], p, rest);
+    if (p >= t.nl) continue;
     const T2 *d = t.sd + p * P.sstride + rest;
     T2 v[R];
 #pragma unroll
@@ -305,6 +313,7 @@ __device__ __forceinline__ void mr_tile(const fftz_pass_t &P, int64_t blk, unsig
   t.s_in = s_in;
   t.s_out = s_out;
   t.s_col = s_col;
+  t.nl = P.ntf - blk * P.tpc < P.tpc ? (int)(P.ntf - blk * P.tpc) : P.tpc;
   for (int p = threadIdx.x; p < P.tpc; p += blockDim.x)
     batch_offsets(P, blk * P.tpc + p, s_in + p, s_out + p, s_col + p);
   __syncthreads();

@@ -13,13 +13,14 @@ template <typename T, bool BIG> __host__ __device__ constexpr int mr_lb() {
 }
 
 // Measured on B200 against the ping-pong tiles this replaced (two buffers, one
-// prime radix a stage, 153 thread instructions a point at n = 1000; now 94):
-// n = 1000 x 32768 float 242 -> 135 us (2.16 -> 3.89 TB/s read + written),
-// 1920 x 4320 64 -> 49 us, 1080-point columns of four 1920 x 1080 images 117 ->
-// 56 us, 120000 = 375 x 320 in double x 64 (two passes) 307 -> 189 us. ncu at
-// n = 1000: issue 56%, shared-memory wavefronts 58%, DRAM 36% of peak -- issue and
-// the shared-memory pipe together, not HBM, bound it. Lines per CTA at n = 1000: 2
-// 166, 3 136, 4 146, 5 135 (fz_mr_shape's choice), 6 142 us.
+// prime radix a stage, 153 thread instructions a point at n = 1000; now 88):
+// n = 1000 x 32768 float 242 -> 125 us (2.16 -> 4.19 TB/s read + written),
+// four 1920 x 1080 images (rows, then columns) 181 -> 94 us, 120000 = 375 x 320 in
+// double x 64 (two passes) 307 -> 184 us, 77 x 100000 float 45 us. ncu at n = 1000
+// (94 instructions a point): issue 56%, shared-memory wavefronts 58%, DRAM 36% of
+// peak -- issue and the shared-memory pipe together, not HBM, bound it. Lines per
+// CTA at n = 1000, at 94 instructions: 2 166, 3 136, 4 146, 5 135 (fz_mr_shape's
+// choice), 6 142 us.
 template <typename T, int FEAT, bool BIG>
 __global__ void __launch_bounds__(mr_lb<T, BIG>()) fft_mr_kernel(const __grid_constant__ fftz_pass_t P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
