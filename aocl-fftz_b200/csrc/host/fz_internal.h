@@ -30,8 +30,11 @@ extern int64_t fz_inj_alloc_fail;  /* fail this many of the next device allocati
 /* cudaMalloc, or a failure while an injected allocation failure is pending */
 int fz_dev_malloc(void **p, size_t bytes);
 
-/* shared memory a ragged executor tile may use (its CTAs run several per SM) */
+/* shared memory a ragged executor tile may use (its CTAs run several per SM),
+ * the executor's block size and the most lines of a tile */
 int64_t fz_ragged_smem_cap(int dtype);
+#define FZ_RG_THREADS 256
+#define FZ_RG_LINES FFTZ_RG_LINES
 
 /* logical buffers: the caller's in / out, then plan-owned scratch arrays,
  * one per use (four-step intermediates, Bluestein work arrays, the
@@ -153,10 +156,10 @@ int64_t fz_real_twiddles(fz_blob *b, int dtype, int64_t M);
 
 /* ---- mixed-radix lines (mixed.c) ---- */
 int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost);
-int fz_mr_fits(int dtype, int64_t n);
-int64_t fz_mr_blue_len(int dtype, int64_t n);
-int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t *n1, int64_t *n2);
-int fz_mr_shape(fftz_pass_t *k, int want_tpc);
+int fz_mr_fits(int dtype, int64_t n, int64_t cap);
+int64_t fz_mr_blue_len(int dtype, int64_t n, int64_t cap);
+int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t *n2);
+int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap);
 int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k);
 
 /* ---- shared by api.c and ragged.c ---- */

@@ -10,7 +10,7 @@
 static int mr_cost(int R)
 {
     static const int flops[17] = {0, 0, 4, 16, 16, 44, 44, 100, 56, 112, 108, 240, 112, 330, 228, 212, 168};
-    return R >= 2 && R <= 16 ? flops[R] + 10 * R + 12 : 0;
+    return R >= 1 && R <= 16 ? flops[R] + 10 * R + 12 : 0;
 }
 
 typedef struct
@@ -57,6 +57,12 @@ int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost)
     static const int pr[] = {2, 3, 5, 7, 11, 13};
     for (int i = 0; i < 6; i++)
         while (m % pr[i] == 0) m /= pr[i];
+    if (n == 1)
+    {
+        radix[0] = 1; /* a copy */
+        if (cost) *cost = 0;
+        return 1;
+    }
     if (n < 2 || m != 1) return 0;
     mr_try(&q, n, 0, 16, 0.0);
     for (int s = 0; s < q.nbest; s++) radix[s] = q.best[s];
@@ -70,19 +76,19 @@ static uint32_t magic(int64_t d) { return d <= 1 ? 0u : (uint32_t)((0xFFFFFFFFul
 static int64_t mr_span(const fftz_pass_t *k, int pad) { return k->n + (int64_t)pad * (k->nstages > 1 ? k->radix[0] : 0); }
 
 /* Most lines of this length a CTA can hold (0: none). */
-static int64_t mr_lines(const fftz_pass_t *k)
+static int64_t mr_lines(const fftz_pass_t *k, int64_t cap)
 {
     const int64_t esz = k->dtype == 0 ? 8 : 16;
-    const int64_t per = (k->sstride + ((k->flags & FFTZ_F_TW4) ? 16 : 0)) * esz + 24;
-    return fftz_smem_limit() / per;
+    const int64_t per = (k->sstride + ((k->flags & FFTZ_F_TW4) ? 16 : 0)) * esz + 32;
+    return cap / per;
 }
 
-/* 1 if a line of n points fits one CTA as a mixed-radix tile. */
-int fz_mr_fits(int dtype, int64_t n)
+/* 1 if a line of n points fits cap bytes of shared memory as a mixed-radix tile. */
+int fz_mr_fits(int dtype, int64_t n, int64_t cap)
 {
     int32_t r[FFTZ_MR_STAGES];
     const int64_t esz = dtype == 0 ? 8 : 16;
-    if (n < 2 || (n + 1 + 16) * esz + 24 > fftz_smem_limit()) return 0;
+    if (n < 1 || (n + 1 + 16) * esz + 32 > cap) return 0;
     return fz_mr_radices(n, 1, r, NULL) > 0;
 }
 
@@ -102,16 +108,16 @@ static int64_t next_smooth7(int64_t n)
 
 /* Convolution length of a chirp-z transform of n points in one tile: the
  * 7-smooth m >= 2n - 1 with the fewest issue slots over both sweeps (a longer m
- * with fewer stages beats the nearest one); 0 when none fits a CTA. */
-int64_t fz_mr_blue_len(int dtype, int64_t n)
+ * with fewer stages beats the nearest one); 0 when none fits cap bytes. */
+int64_t fz_mr_blue_len(int dtype, int64_t n, int64_t cap)
 {
     int32_t r[FFTZ_MR_STAGES];
     int64_t best = 0;
     double score = 0, c;
     const int64_t need = 2 * n - 1;
-    if (need * (dtype == 0 ? 8 : 16) > fftz_smem_limit()) return 0;
+    if (need * (dtype == 0 ? 8 : 16) > cap) return 0;
     for (int64_t m = next_smooth7(need < 4 ? 4 : need); m <= need + need / 4 + 4; m = next_smooth7(m + 1))
-        if (fz_mr_fits(dtype, m) && fz_mr_radices(m, 2, r, &c) > 1 && (!best || (double)m * c < score))
+        if (fz_mr_fits(dtype, m, cap) && fz_mr_radices(m, 2, r, &c) > 1 && (!best || (double)m * c < score))
         {
             best = m;
             score = (double)m * c;
@@ -122,7 +128,7 @@ int64_t fz_mr_blue_len(int dtype, int64_t n)
 /* Convolution length m = n1 * n2 of a chirp-z transform in three passes: the
  * cheapest of the first 7-smooth lengths from 2n - 1 on, both factors one tile
  * and n2 of at least two stages, within a factor of four of each other. */
-int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t *n1, int64_t *n2)
+int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t *n2)
 {
     int32_t r[FFTZ_MR_STAGES];
     int64_t best = 0, m = 2 * n - 2;
@@ -133,7 +139,7 @@ int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t *n1, int64_t *n2)
         for (int64_t a = 2; a * a <= 4 * m; a++)
         {
             const int64_t b = m / a;
-            if (m % a || a > 4 * b || b > 4 * a || !fz_mr_fits(dtype, a) || !fz_mr_fits(dtype, b)) continue;
+            if (m % a || a > 4 * b || b > 4 * a || !fz_mr_fits(dtype, a, cap) || !fz_mr_fits(dtype, b, cap)) continue;
             if (fz_mr_radices(a, 1, r, &ca) < 1 || fz_mr_radices(b, 2, r, &cb) < 2) continue;
             if (!best || (double)m * (ca + cb) < score)
             {
@@ -152,7 +158,7 @@ int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t *n1, int64_t *n2)
 static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)
 {
     const int S = k->nstages;
-    const int64_t R = k->radix[s], M = k->mr.m[s], nb = k->n / R;
+    const int64_t R = k->radix[s], M = k->mr.st[s].m, nb = k->n / R;
     int64_t p, x;
     if (col)
     {
@@ -171,7 +177,7 @@ static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)
         int64_t o = 0;
         for (int j = 0; j < S - 1; j++)
         {
-            o += (x % k->radix[j]) * (k->mr.m[j] + (j == 0 ? k->mr.pad : 0));
+            o += (x % k->radix[j]) * (k->mr.st[j].m + (j == 0 ? k->mr.pad : 0));
             x /= k->radix[j];
         }
         return base + o;
@@ -220,9 +226,10 @@ static void mr_stride(fftz_pass_t *k, int colmap, int pad)
 }
 
 /* Fills k's mixed-radix launch shape (its lengths, strides, batch and flags are
- * set); want_tpc > 0 fixes the lines per CTA where they fit. Returns 0, or -1
- * when the line does not fit a CTA. */
-int fz_mr_shape(fftz_pass_t *k, int want_tpc)
+ * set); want_tpc > 0 fixes the lines per CTA where they fit, threads > 0 the
+ * block (the ragged executor's, whose tiles keep their size in small batches).
+ * Returns 0, or -1 when the line does not fit cap bytes. */
+int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
 {
     const int two = (k->flags & FFTZ_F_MID_TAB) != 0;
     const int colmap = k->in_mode == 1 || k->out_mode == 1;
@@ -236,23 +243,30 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc)
         const int R = k->radix[s];
         if (R == 11 || R == 13) k->mr.big = 1;
         M /= R;
-        k->mr.m[s] = (int32_t)M;
-        k->mr.mg_nb[s] = magic(k->n / R);
-        k->mr.mg_m[s] = magic(M);
-        k->mr.mg_r[s] = magic(R);
-        k->mr.mg_b[s] = magic(B);
+        fftz_mr_stage_t *st = &k->mr.st[s];
+        st->r = R;
+        st->m = (int32_t)M;
+        st->nb = k->n / R;
+        st->mg_nb = magic(st->nb);
+        st->mg_m = magic(M);
+        st->mg_r = magic(R);
+        st->mg_b = magic(B);
         if (s > 0) B *= R;
     }
     k->tpc = 1;
     mr_stride(k, colmap, 0);
     const int tmax = fftz_mr_max_threads(k->dtype, k->mr.big);
-    int64_t most = mr_lines(k);
+    int64_t most = mr_lines(k, cap);
     if (most < 1) return -1;
     if (most > k->ntf) most = k->ntf;
-    if (most > 256) most = 256;
+    if (most > (threads ? FZ_RG_LINES : 256)) most = threads ? FZ_RG_LINES : 256;
     /* lines per CTA: about 4096 float / 2048 double points of row lines; whole
-     * 64-byte segments (8 float / 4 double neighbours) of column lines */
-    const int64_t pts = k->dtype == 0 ? 4096 : 2048;
+     * 64-byte segments (8 float / 4 double neighbours) of column lines. The
+     * executor's tiles, which wait on memory at their ends, are larger (measured on
+     * B200, 4096 ragged transforms, forward: float 1536 points 888 us, 3072 839, 4096
+     * 809, 6144 805; double 768 2124, 1536 1753, 2048 1459, 3072 1388, and with later
+     * stage forms 2048 1298, 3072 1236, 4096 1187 us) */
+    const int64_t pts = threads ? (k->dtype == 0 ? 6144 : 4096) : (k->dtype == 0 ? 4096 : 2048);
     int64_t lo = 1, hi = most;
     if (want_tpc > 0)
         lo = hi = want_tpc < most ? want_tpc : most;
@@ -261,11 +275,13 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc)
         const int64_t seg = k->dtype == 0 ? 8 : 4;
         lo = hi = seg < most ? seg : most;
         while (hi * 2 <= most && hi * 2 * k->n <= pts && hi < 32) lo = hi = hi * 2;
+        /* the executor's block is fixed: a few more columns where they fill it better */
+        if (threads) hi = lo + lo / 2 <= most ? lo + lo / 2 : most;
     }
     else
     {
         /* fewer lines where whole CTAs would not give every SM two */
-        while (hi > 1 && (hi * k->n > pts + pts / 2 || k->ntf / hi < 2 * 148)) hi--;
+        while (hi > 1 && (hi * k->n > pts + pts / 2 || (threads == 0 && k->ntf / hi < 2 * 148))) hi--;
         lo = hi > 1 ? (hi + 1) / 2 : 1;
     }
     double best = -1;
@@ -275,10 +291,10 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc)
         k->tpc = (int32_t)c;
         mr_stride(k, colmap, 0);
         const int64_t smem = fftz_pass_smem_bytes(k) + 1024;
-        if (smem - 1024 > fftz_smem_limit()) continue;
+        if (smem - 1024 > cap) continue;
         int64_t by_smem = (228 * 1024) / smem;
         if (by_smem > 24) by_smem = 24;
-        for (int t = 64; t <= tmax; t += 32)
+        for (int t = threads ? threads : 64; t <= (threads ? threads : tmax); t += 32)
         {
             int64_t ctas = tmax / t;
             if (ctas > by_smem) ctas = by_smem;
@@ -309,7 +325,7 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc)
     for (int pad = 0; pad < (k->nstages > 1 ? 16 : 1); pad++)
     {
         mr_stride(k, colmap, pad);
-        if (pad > 0 && fftz_pass_smem_bytes(k) > fftz_smem_limit()) break;
+        if (pad > 0 && fftz_pass_smem_bytes(k) > cap) break;
         const int c = mr_conflicts(k);
         if (bp < 0 || c < bc)
         {
@@ -322,7 +338,7 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc)
     k->fuse_load = k->fuse_store = 1;
     k->use_tma = 0;
     k->smem_tw = 0;
-    return fftz_pass_smem_bytes(k) <= fftz_smem_limit() ? 0 : -1;
+    return fftz_pass_smem_bytes(k) <= cap ? 0 : -1;
 }
 
 /* Stage twiddles of a mixed-radix line: stage s multiplies by
@@ -334,6 +350,8 @@ int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k)
     const int S = k->nstages;
     for (int s = 0; s < S; s++) rev[s] = k->radix[S - 1 - s];
     const int64_t o = fz_stage_twiddles(b, k->dtype, k->n, S, rev, off);
-    for (int s = 0; s < S; s++) k->tw_off[s] = off[S - 1 - s];
+    k->ntw = 1;
+    for (int s = 0; s < S; s++) k->ntw += s < S - 1 ? (k->radix[s] - 1) * k->mr.st[s].m : 0;
+    for (int s = 0; s < S; s++) k->mr.st[s].tw = k->tw_off[s] = off[S - 1 - s];
     return o;
 }

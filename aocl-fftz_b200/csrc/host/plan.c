@@ -99,21 +99,16 @@ static int64_t absl(int64_t x) { return x < 0 ? -x : x; }
 /* every pass on the generic kernel (the persistent executor runs only that) */
 static int generic_only(const fz_plan *pl) { return pl->hints.kernel_family == 3; }
 
-/* kernel_family 4: passes for the persistent ragged executor, whose CTAs have
- * 256 threads: compile-time kernels up to length 4096, never the pipelined
- * family */
+/* kernel_family 4: passes for the persistent ragged executor, every line a
+ * mixed-radix tile of its block size within its shared-memory share */
 static int ragged_mode(const fz_plan *pl) { return pl->hints.kernel_family == 4; }
-static int64_t fast_max_n(const fz_plan *pl)
-{
-    const int64_t m = fftz_fast_max_n(pl->dtype);
-    return ragged_mode(pl) && m > 4096 ? 4096 : m;
-}
-static int fast_max_threads(const fz_plan *pl) { return ragged_mode(pl) ? 256 : (pl->dtype == 0 ? 1024 : 512); }
+static int64_t fast_max_n(const fz_plan *pl) { return fftz_fast_max_n(pl->dtype); }
+static int fast_max_threads(const fz_plan *pl) { return pl->dtype == 0 ? 1024 : 512; }
 
-/* Runtime-radix lines run as mixed-radix tiles (one buffer, kernels/fft_mr.cuh);
- * kernel_family 12 keeps the older in-place kernel, the ragged executor its
- * ping-pong tiles. */
-static int mixed_lines(const fz_plan *pl) { return pl->hints.kernel_family != 12 && !ragged_mode(pl); }
+/* Runtime-radix lines run as mixed-radix tiles (kernels/fft_mr.cuh);
+ * kernel_family 12 keeps the older in-place kernel where its threads suffice. */
+static int mixed_lines(const fz_plan *pl) { return pl->hints.kernel_family != 12; }
+static int64_t mixed_cap(const fz_plan *pl) { return ragged_mode(pl) ? fz_ragged_smem_cap(pl->dtype) : fftz_smem_limit(); }
 
 /* Batch dims: optionally sorted by stride (smallest first, so that bdim[0]
  * is the one lanes may run along), then adjacent dims merged when they form
@@ -169,13 +164,6 @@ static int set_batch(fftz_pass_t *k, const fz_dim *b, int nb, int keep_first)
     return 0;
 }
 
-/* shared memory of one ping-pong tile holding one line of n */
-static int64_t pp_one_line_bytes(int dtype, int64_t n)
-{
-    const int64_t esz = dtype == 0 ? 8 : 16;
-    return 2 * (int64_t)fftz_smem_stride(dtype, (int32_t)n) * esz + 24 + 8 * FFTZ_MAX_STAGES;
-}
-
 /* transforms per CTA: enough columns for coalesced column access, enough
  * work per CTA for short rows, bounded by threads and shared memory (two
  * slots for the double-buffered kernels) */
@@ -228,9 +216,10 @@ static void set_modes(fftz_pass_t *k)
     k->out_mode = (k->nbdims > 0 && absl(k->obs[0]) < absl(k->oes)) ? 1 : 0;
 }
 
-/* one complex line pass in the shared-memory kernel; returns the pass */
+/* one complex line pass in the shared-memory kernels (mixed: always a
+ * mixed-radix tile, the only one with tables and two sweeps); returns the pass */
 static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_dim *b, int nb,
-                          int keep_first, int src, int dst, int flags, int variant_bits)
+                          int keep_first, int src, int dst, int flags, int mixed)
 {
     fz_pass *p = push_pass(pl);
     if (!p) return NULL;
@@ -247,7 +236,8 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
     p->dst = dst;
     if (set_batch(k, b, nb, keep_first)) return NULL;
     set_modes(k);
-    const int fast = !generic_only(pl) && is_pow2(n) && n >= 2 && n <= fast_max_n(pl) && !(variant_bits & 8);
+    const int fast = !generic_only(pl) && is_pow2(n) && n >= 2 && n <= fast_max_n(pl) && !mixed &&
+                     !ragged_mode(pl);
     int maxthr;
     if (fast)
     {
@@ -255,21 +245,15 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
         k->tpt = fftz_fast_tpt((int)n);
         maxthr = fast_max_threads(pl);
         if (k->nstages == 1 && k->in_mode != k->out_mode) k->out_mode = k->in_mode;
-        int tabs = (variant_bits & 2) != 0, tw4 = (flags & FFTZ_F_TW4) != 0;
+        const int tw4 = (flags & FFTZ_F_TW4) != 0;
         const int fam = pl->hints.kernel_family;
-        const int pipe_ok = n >= 64 && !tabs && !(variant_bits & 4);
+        const int pipe_ok = n >= 64;
         /* the persistent double-buffered kernel is a tuning option (hint
          * kernel_family = 2); measured on B200 the one-tile-per-CTA kernel is
          * faster for both dtypes and both lane maps, so it is the default */
         const int pipe_default = 0;
         if (pipe_ok && (fam == 2 || (fam == 0 && pipe_default)))
             k->variant = tw4 ? FFTZ_VAR_PIPE_TW4 : FFTZ_VAR_PIPE;
-        else if (variant_bits & 4)
-            k->variant = FFTZ_VAR_FAST_BLUE;
-        else if (tabs && tw4)
-            k->variant = FFTZ_VAR_FAST_TW4_TABS;
-        else if (tabs)
-            k->variant = FFTZ_VAR_FAST_TABS;
         else if (tw4)
             k->variant = FFTZ_VAR_FAST_TW4;
         else
@@ -304,8 +288,8 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
          * the next tile in flight (kernel_family 13) */
         if (k->variant == FFTZ_VAR_FAST && k->in_mode == 0 && fam == 13) k->use_tma = 7;
         /* stage twiddles copied to shared memory by each CTA (hint twiddles = 2) */
-        k->smem_tw = pl->hints.twiddles == 2 && !ragged_mode(pl) && n >= 512;
-        if ((tw4 || tabs) && n < 32 && !(variant_bits & 4))
+        k->smem_tw = pl->hints.twiddles == 2 && n >= 512;
+        if (tw4 && n < 32)
         {
             /* small feature kernels are not instantiated: use the generic one */
             goto generic;
@@ -317,11 +301,12 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
     else
     {
     generic:
-        if (n > 1 && mixed_lines(pl))
+        if (mixed_lines(pl) || mixed)
         {
             k->smem_tw = k->use_tma = 0;
             const int colm = k->in_mode == 1 || k->out_mode == 1;
-            if (fz_mr_shape(k, colm ? pl->hints.tpc_col : pl->hints.tpc_row))
+            if (fz_mr_shape(k, colm ? pl->hints.tpc_col : pl->hints.tpc_row, ragged_mode(pl) ? FZ_RG_THREADS : 0,
+                            mixed_cap(pl)))
             {
                 fz_set_error("length %lld does not fit a mixed-radix tile", (long long)n);
                 return NULL;
@@ -340,10 +325,6 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
         }
         k->tpt = k->nstages ? fftz_threads_per_transform(pl->dtype, (int)n, k->nstages, k->radix) : 1;
         maxthr = fftz_generic_max_threads();
-        /* the executor's lines longer than the in-place tile's thread budget run
-         * as ping-pong tiles (chosen below) */
-        if (k->tpt > maxthr && ragged_mode(pl) && pp_one_line_bytes(pl->dtype, n) <= fftz_smem_limit())
-            k->tpt = maxthr;
         if (k->tpt > maxthr)
         {
             fz_set_error("length %lld exceeds the generic kernel's thread budget", (long long)n);
@@ -368,39 +349,6 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
         finish_launch_shape(pl, k, nslots, maxthr);
     }
     if (k->smem_tw && fftz_pass_smem_bytes(k) > fftz_smem_limit()) k->smem_tw = 0;
-    /* the ragged executor's runtime-radix lines: ping-pong tiles (two
-     * shared-memory buffers, one butterfly per thread at a time, 256 threads)
-     * when both buffers fit */
-    if (k->variant == FFTZ_VAR_GENERIC && ragged_mode(pl))
-    {
-        const int esz = pl->dtype == 0 ? 8 : 16;
-        const int32_t sst = fftz_smem_stride(pl->dtype, nslots);
-        const int colm = (k->in_mode == 1 || k->out_mode == 1);
-        /* about 4096 float (2048 double) elements per CTA: measured on B200,
-         * mixed1000 (N = 1000, batch 32768) 0.618 ms per step with two lines
-         * per CTA, 0.498 with four, 0.732 with eight (one CTA per SM) */
-        int64_t want = (pl->dtype == 0 ? 4096 : 2048) / n;
-        if (colm && want < (pl->dtype == 0 ? 8 : 4)) want = pl->dtype == 0 ? 8 : 4;
-        if (colm && pl->hints.tpc_col > 0) want = pl->hints.tpc_col;
-        if (!colm && pl->hints.tpc_row > 0) want = pl->hints.tpc_row;
-        if (want < 1) want = 1;
-        if (want > 64) want = 64;
-        if (want > k->ntf) want = k->ntf;
-        while (want > 1 && 2 * want * sst * esz + 24 * want + 8 * FFTZ_MAX_STAGES > fftz_smem_limit()) want--;
-        if (2 * want * (int64_t)sst * esz + 24 * want + 8 * FFTZ_MAX_STAGES <= fftz_smem_limit())
-        {
-            k->variant = FFTZ_VAR_GENERIC_PP;
-            k->tpc = (int32_t)want;
-            k->sstride = sst;
-            k->tpt = (int32_t)(256 / want > 0 ? 256 / want : 1);
-            /* complex lines read HBM in their first stage and write it in
-             * their last (the load / store phases stay for the other kinds
-             * and for load-side tables) */
-            k->fuse_load = k->nstages > 0 && k->in_kind == FFTZ_IN_COMPLEX && k->nload == n &&
-                           !(flags & FFTZ_F_PRE_TAB);
-            k->fuse_store = k->nstages > 0 && k->out_kind == FFTZ_OUT_COMPLEX && k->nstore == n;
-        }
-    }
     if (fftz_pass_smem_bytes(k) > fftz_smem_limit())
     {
         fz_set_error("length %lld does not fit shared memory", (long long)n);
@@ -426,9 +374,7 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
         if (p->off_tw < 0) return NULL;
     }
     snprintf(p->what, sizeof(p->what), "%s n=%lld x%lld",
-             k->variant == FFTZ_VAR_GENERIC ? "generic"
-             : k->variant == FFTZ_VAR_GENERIC_PP ? "generic-pp"
-                                                 : (is_pipe_variant(k->variant) ? "pipe" : "fast"),
+             k->variant == FFTZ_VAR_GENERIC ? "generic" : (is_pipe_variant(k->variant) ? "pipe" : "fast"),
              (long long)n, (long long)k->ntf);
     return p;
 }
@@ -436,13 +382,11 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
 static int single_pass_ok(const fz_plan *pl, int64_t n)
 {
     if (n == 1) return 1;
-    if (!generic_only(pl) && is_pow2(n) && n <= fast_max_n(pl)) return 1;
+    if (!generic_only(pl) && !ragged_mode(pl) && is_pow2(n) && n <= fast_max_n(pl)) return 1;
     int32_t r[FFTZ_MAX_STAGES];
     int s = generic_radices(n, r);
     if (s < 0 || n > (1 << 20)) return 0;
-    /* the executor's tiles (ragged batches) are ping-pong tiles within its cap */
-    if (ragged_mode(pl)) return pp_one_line_bytes(pl->dtype, n) <= fz_ragged_smem_cap(pl->dtype);
-    if (mixed_lines(pl)) return fz_mr_fits(pl->dtype, n);
+    if (mixed_lines(pl)) return fz_mr_fits(pl->dtype, n, mixed_cap(pl));
     int tpt = fftz_threads_per_transform(pl->dtype, (int)n, s, r);
     if (tpt < 1 || tpt > fftz_generic_max_threads()) return 0;
     int64_t esz = pl->dtype == 0 ? 8 : 16;
@@ -617,10 +561,8 @@ static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_d
 }
 
 /* Bluestein (chirp-z) over a 7-smooth m >= 2n - 1 on mixed-radix tiles (the
- * reference pads to a 13-smooth m, core/common/bluestein_utils.c:39-67). The
- * ragged executor and kernel_family 12 keep a power of two, whose
- * sub-transforms run on the compile-time kernels. A convolution that fits a
- * CTA (m up to 28672 float, 14400 double) is one kernel, which reads and writes
+ * reference pads to a 13-smooth m, core/common/bluestein_utils.c:39-67). A
+ * convolution that fits a CTA (m up to 28672 float, 14400 double) is one kernel, which reads and writes
  * HBM once: measured on B200, n = 10007 float x 512, m = 32768 in three passes 452
  * us, m = 20736 in three passes 317 us, in one kernel 142 us; one line 52, 52
  * and 35 us. Only a few double lines near the limit are faster in three passes
@@ -628,22 +570,12 @@ static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_d
  * for 64), both faster than three passes over a power of two (58 us). */
 static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_dim *b, int nb, int src, int dst)
 {
-    const int mixed = mixed_lines(pl), vb = mixed ? 2 | 8 : 2; /* line_pass bits: tables, mixed-radix tiles */
-    int64_t m = 1, n1 = 0, n2 = 0;
-    int one = 0;
-    if (mixed)
+    int64_t n1 = 0, n2 = 0, m = fz_mr_blue_len(pl->dtype, n, mixed_cap(pl));
+    const int one = m > 0;
+    if (!one && (m = fz_mr_blue_split(pl->dtype, n, mixed_cap(pl), &n1, &n2)) == 0)
     {
-        one = (m = fz_mr_blue_len(pl->dtype, n)) > 0;
-        if (!one && (m = fz_mr_blue_split(pl->dtype, n, &n1, &n2)) == 0)
-        {
-            fz_set_error("length %lld has no chirp-z plan", (long long)n);
-            return -1;
-        }
-    }
-    else
-    {
-        while (m < 2 * n - 1) m *= 2;
-        one = m >= 4 && single_pass_ok(pl, m);
+        fz_set_error("length %lld has no chirp-z plan", (long long)n);
+        return -1;
     }
     int64_t pre, post, mid;
     if (fz_bluestein_tables(&pl->blob, pl->dtype, n, m, pl->direction, &pre, &post, &mid)) return -1;
@@ -653,7 +585,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         fz_pass *p = line_pass(pl, m, ies, oes, b, nb, 0, src, dst,
                                (bwd ? FFTZ_F_CONJ_IN : FFTZ_F_CONJ_OUT) | FFTZ_F_PRE_TAB | FFTZ_F_POST_TAB |
                                    FFTZ_F_MID_TAB,
-                               vb | 4);
+                               1);
         if (!p) return -1;
         p->k.pre_n = n;
         p->k.pre_es = 1;
@@ -669,7 +601,6 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
     /* three passes through S0 / S1: A (column FFTs of the chirped, padded
      * input), M (row FFTs, spectrum product, row FFTs of the second FFT_m),
      * D (row FFTs of the second FFT_m, output chirp) */
-    if (!mixed && choose_split(pl, m, &n1, &n2)) return -1;
     int64_t lines = lines_of(b, nb);
     const int S0 = new_scratch(pl, m * lines), S1 = new_scratch(pl, m * lines);
     if (S0 < 0 || S1 < 0) return -1;
@@ -689,7 +620,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         so *= b[i].n;
     }
     fz_pass *pa = line_pass(pl, n1, n2 * ies, n2, bb, nb + 1, 1, src, S0,
-                            (bwd ? FFTZ_F_CONJ_IN : 0) | FFTZ_F_PRE_TAB | FFTZ_F_TW4, vb);
+                            (bwd ? FFTZ_F_CONJ_IN : 0) | FFTZ_F_PRE_TAB | FFTZ_F_TW4, 1);
     if (!pa) return -1;
     pa->k.pre_n = n;
     pa->k.pre_es = n2;
@@ -718,7 +649,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         bb[i + 1].os = so;
         so *= b[i].n;
     }
-    fz_pass *pm = line_pass(pl, n2, 1, n1, bb, nb + 1, 1, S0, S1, FFTZ_F_MID_TAB | FFTZ_F_TW4, vb | 4);
+    fz_pass *pm = line_pass(pl, n2, 1, n1, bb, nb + 1, 1, S0, S1, FFTZ_F_MID_TAB | FFTZ_F_TW4, 1);
     if (!pm) return -1;
     pm->k.mid_cs = n2;
     pm->off_mid = midT;
@@ -741,7 +672,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         so *= b[i].n;
     }
     fz_pass *pd = line_pass(pl, n1, 1, n2 * oes, bb, nb + 1, 1, S1, dst,
-                            (bwd ? 0 : FFTZ_F_CONJ_OUT) | FFTZ_F_POST_TAB, vb);
+                            (bwd ? 0 : FFTZ_F_CONJ_OUT) | FFTZ_F_POST_TAB, 1);
     if (!pd) return -1;
     pd->k.post_n = n;
     pd->k.post_es = n2;

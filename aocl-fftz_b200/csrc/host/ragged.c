@@ -6,7 +6,7 @@
  * back to back (AOCL-FFTZ executes each plan's solver tree,
  * core/executor.c:17-44). Here the transforms are grouped by length; each
  * group is planned once by the ordinary planner (in its executor mode:
- * 256-thread tiles, compile-time kernels up to length 4096) as a batch whose
+ * mixed-radix tiles of the executor's block) as a batch whose
  * transform dimension is indirect, so the group's transforms keep their own
  * offsets in the packed buffers. The passes are flattened into a table of CTA
  * tiles (pass, tile, predecessor pass) and the persistent executor
@@ -76,67 +76,16 @@ static void resolve(int id, int64_t io_off_bytes, const int64_t *soff, int32_t *
     }
 }
 
-#define RG_THREADS 256
-
-/* The executor's shared memory per CTA is the largest of its passes', so
- * every tile shape stays within 44 KB (float: five CTAs per SM, the
- * executor's register bound) or 100 KB (double: two CTAs per SM). Measured on
- * B200 (4096 float transforms): float ping-pong tiles of up to 72 KB made the
- * whole launch 1.353 -> 1.688 ms although their own class got faster. */
-int64_t fz_ragged_smem_cap(int dtype) { return dtype == 0 ? 44 * 1024 : 100 * 1024; }
-
-/* Launch shape of one pass inside the executor (256-thread CTAs): a
- * compile-time tile with tpc * tpt == 256 where the executor has one,
- * otherwise the generic tile with as many transforms as fit (loads and stores
- * through the generic phases, which know every table and bound). */
-static int ragged_shape(fftz_pass_t *k, int dtype, int64_t smem_cap)
-{
-    const int nslots = k->n > k->nload ? k->n : k->nload;
-    const int colmap = k->in_mode == 1 || k->out_mode == 1;
-    const int fastv = k->variant == FFTZ_VAR_FAST || k->variant == FFTZ_VAR_FAST_TW4 ||
-                      k->variant == FFTZ_VAR_FAST_TABS || k->variant == FFTZ_VAR_FAST_TW4_TABS ||
-                      k->variant == FFTZ_VAR_FAST_BLUE;
-    if (fastv && fftz_ragged_fast_ok(k->n, k->variant) && k->tpt <= RG_THREADS && RG_THREADS % k->tpt == 0)
-    {
-        fftz_pass_t t = *k;
-        t.tpc = RG_THREADS / t.tpt;
-        t.sstride = colmap ? fftz_smem_stride_cols(dtype, nslots, t.tpc) : fftz_smem_stride(dtype, nslots);
-        if (fftz_pass_smem_bytes(&t) <= smem_cap)
-        {
-            *k = t;
-            return 0;
-        }
-    }
-    /* everything else runs as a ping-pong tile (the same radix list and
-     * twiddle table; tables and other element kinds through its load / store
-     * phases): as many lines as fit the cap, up to about 4096 elements */
-    if (k->variant != FFTZ_VAR_GENERIC_PP)
-    {
-        k->variant = FFTZ_VAR_GENERIC_PP;
-        k->fuse_load = k->nstages > 0 && k->in_kind == FFTZ_IN_COMPLEX && k->nload == k->n &&
-                       !(k->flags & FFTZ_F_PRE_TAB);
-        k->fuse_store = k->nstages > 0 && k->out_kind == FFTZ_OUT_COMPLEX && k->nstore == k->n;
-    }
-    int tpc = (int)((dtype == 0 ? 4096 : 2048) / k->n);
-    if (colmap && tpc < (dtype == 0 ? 8 : 4)) tpc = dtype == 0 ? 8 : 4;
-    if (tpc < 1) tpc = 1;
-    if (tpc > 64) tpc = 64;
-    if (tpc > k->ntf) tpc = (int)k->ntf;
-    for (; tpc >= 1; tpc--)
-    {
-        k->tpc = tpc;
-        k->sstride = fftz_smem_stride(dtype, nslots);
-        k->tpt = RG_THREADS / tpc > 0 ? RG_THREADS / tpc : 1;
-        if (fftz_pass_smem_bytes(k) <= smem_cap) return 0;
-    }
-    return -1;
-}
+/* A quarter of an SM's shared memory a tile (float: four CTAs of 256 threads
+ * and 64 registers), half of it for double (two CTAs, 128 registers), less the
+ * executor's own pass descriptors and twiddle copies. */
+int64_t fz_ragged_smem_cap(int dtype) { return dtype == 0 ? 42 * 1024 : 91 * 1024; }
 
 typedef struct
 {
     fz_plan *pl;
     int dtype, direction;
-    int64_t csz, smem_cap;
+    int64_t csz;
     int64_t npass, cap_pass, cap_aux, nitem, cap_item, scratch_total, nind, cap_ind;
     fftz_pass_t *passes;
     int64_t (*toff)[7];  /* per pass: table offsets in the merged blob */
@@ -266,9 +215,10 @@ static int add_group(rg_build *B, int64_t n, int64_t c, const int64_t *tin, cons
         k.ind_dim = inddim[j] >= 0 ? inddim[j] : 0;
         k.ind_in = NULL;
         k.ind_out = NULL;
-        if (ragged_shape(&k, B->dtype, B->smem_cap))
+        if (k.nstages == 1 && (k.flags & (FFTZ_F_TW4 | FFTZ_F_PRE_TAB | FFTZ_F_POST_TAB)))
         {
-            fz_set_error("ragged setup: a pass of length %d does not fit the executor", k.n);
+            /* the executor's one-stage tiles are whole lines (every split has longer factors) */
+            fz_set_error("ragged setup: a pass of length %d has no tile form", k.n);
             rc = -1;
             break;
         }
@@ -356,7 +306,6 @@ FFTZ_VOID *aoclfftz_gpu_ragged_setup(FFTZ_INT32 dtype, FFTZ_INT32 direction, FFT
     B.dtype = dtype;
     B.direction = direction;
     B.csz = dtype == 0 ? 8 : 16;
-    B.smem_cap = fz_ragged_smem_cap(dtype);
     int64_t next_in = 0, next_out = 0;
     for (int64_t i = 0; i < count; i++)
     {
@@ -452,7 +401,7 @@ FFTZ_VOID *aoclfftz_gpu_ragged_setup(FFTZ_INT32 dtype, FFTZ_INT32 direction, FFT
     if (rg->grid > B.nitem) rg->grid = (int)B.nitem;
     snprintf(rg->summary, sizeof(rg->summary),
              "ragged: %lld transforms in %lld length groups, %lld passes, %lld tiles, grid %d x %d, %d B smem",
-             (long long)count, (long long)rg->ngroups, (long long)B.npass, (long long)B.nitem, rg->grid, RG_THREADS,
+             (long long)count, (long long)rg->ngroups, (long long)B.npass, (long long)B.nitem, rg->grid, FZ_RG_THREADS,
              rg->smem);
     pl->in_bytes = rg->in_elems * B.csz;
     pl->out_bytes = rg->out_elems * B.csz;

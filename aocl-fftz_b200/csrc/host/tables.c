@@ -128,7 +128,7 @@ int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32
     }
     (void)n;
     size_t esz = dtype == 0 ? 8 : 16;
-    int64_t off = fz_blob_reserve(b, (size_t)total * esz);
+    int64_t off = fz_blob_reserve(b, (size_t)(total + (total & 1)) * esz); /* whole 16-byte words */
     if (off < 0) return -1;
     put_c(b, off, dtype, 0, 1.0, 0.0);
     if (nstages < 2) return off;

@@ -39,6 +39,10 @@ template <int N1, int N2> struct DftPfa {
   }
 };
 
+template <> struct Dft<1> {  // one-point lines
+  template <typename T, typename T2>
+  static __device__ __forceinline__ void apply(T2 (&)[1]) {}
+};
 template <> struct Dft<6> : DftPfa<2, 3> {};
 template <> struct Dft<10> : DftPfa<2, 5> {};
 template <> struct Dft<12> : DftPfa<4, 3> {};

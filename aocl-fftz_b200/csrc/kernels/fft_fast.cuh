@@ -20,11 +20,7 @@
 // (mode 1, columns) on the HBM side, which keeps both row and column accesses
 // coalesced. Feature bits (template FEAT) add:
 //   FEAT_TW4   output k of column c times W_{tw4_n}^{c k} (four-step twiddle,
-//              FP64 factors);
-//   FEAT_TABS  load-side bound and table product (Bluestein pre-chirp and zero
-//              padding) and store-side table product, bound and scale;
-//   FEAT_SWEEP2 two sweeps of the stages with v = conj(v) * mid_tab[e] between
-//              them (the spectrum product of a one-kernel Bluestein transform).
+//              FP64 factors).
 #pragma once
 #include "fft_common.cuh"
 
@@ -64,45 +60,7 @@ template <typename T> __host__ __device__ constexpr int ct_lb() { return sizeof(
 // registers a thread) unless one transform needs more.
 __host__ __device__ constexpr int ct_pipe_lb(int n) { return ct_tpt(n) > 512 ? ct_tpt(n) : 512; }
 
-enum { FEAT_TW4 = 1, FEAT_TABS = 2, FEAT_SWEEP2 = 4 };
-
-// Epilogue of one output element kk (the destination pointer already points
-// at it).
-template <typename T, int FEAT>
-__device__ __forceinline__ void store_fast(const fftz_pass_t &P, typename Cplx<T>::type v, int kk, int64_t col,
-                                           int64_t obase) {
-  typedef typename Cplx<T>::type T2;
-  if (FEAT & FEAT_TABS) {
-    store_complex<T>(P, v, kk, col, obase);
-    return;
-  }
-  if (FEAT & FEAT_TW4) v = cmul(v, tw4<T>(P, col, kk));
-  if (P.flags & FFTZ_F_CONJ_OUT) v.y = -v.y;
-  T2 *o = (T2 *)P.out + obase;
-  if (P.oes == 1)
-    o[kk] = v;
-  else
-    o[(int64_t)kk * P.oes] = v;
-}
-
-template <typename T, int FEAT>
-__device__ __forceinline__ typename Cplx<T>::type load_fast(const fftz_pass_t &P, const typename Cplx<T>::type *gin,
-                                                            int e, int64_t col, bool valid) {
-  typedef typename Cplx<T>::type T2;
-  T2 x = zero2<T2>();
-  if (FEAT & FEAT_TABS) {
-    const int64_t li = (int64_t)e * P.pre_es + col * P.pre_cs;
-    if (valid && (P.pre_n == 0 || li < P.pre_n)) {
-      x = gin[(int64_t)e * P.ies];
-      if (P.flags & FFTZ_F_CONJ_IN) x.y = -x.y;
-      if (P.flags & FFTZ_F_PRE_TAB) x = cmul(x, __ldg((const T2 *)P.pre_tab + li));
-    }
-  } else {
-    if (valid) x = (P.ies == 1) ? gin[e] : gin[(int64_t)e * P.ies];
-    if (P.flags & FFTZ_F_CONJ_IN) x.y = -x.y;
-  }
-  return x;
-}
+enum { FEAT_TW4 = 1 };
 
 // One Stockham stage. FROMG: the stage reads its inputs from HBM (otherwise
 // from shared memory). LAST: it writes its outputs to HBM. MAPFIRST /
@@ -188,22 +146,17 @@ __device__ __forceinline__ void fast_stage(const fftz_pass_t &P, typename Cplx<T
     for (int q = 0; q < NB; q++) {
       const int b = j + q * TPT;
       if (ALLV || b < NBF) {
-        if constexpr ((FEAT & FEAT_TABS) != 0) {
+        // one 64-bit product per butterfly, constant multiples after it
+        const int64_t ies = P.ies;
+        const T2 *gb = gin + (int64_t)b * ies;
+        const int64_t st = (int64_t)NBF * ies;
+        const bool cj = (P.flags & FFTZ_F_CONJ_IN) != 0;
 #pragma unroll
-          for (int r = 0; r < R; r++) v[q][r] = load_fast<T, FEAT>(P, gin, b + r * NBF, col, valid);
-        } else {
-          // one 64-bit product per butterfly, constant multiples after it
-          const int64_t ies = P.ies;
-          const T2 *gb = gin + (int64_t)b * ies;
-          const int64_t st = (int64_t)NBF * ies;
-          const bool cj = (P.flags & FFTZ_F_CONJ_IN) != 0;
-#pragma unroll
-          for (int r = 0; r < R; r++) {
-            T2 x = zero2<T2>();
-            if (valid) x = gb[r * st];
-            if (cj) x.y = -x.y;
-            v[q][r] = x;
-          }
+        for (int r = 0; r < R; r++) {
+          T2 x = zero2<T2>();
+          if (valid) x = gb[r * st];
+          if (cj) x.y = -x.y;
+          v[q][r] = x;
         }
       }
     }
@@ -250,34 +203,29 @@ __device__ __forceinline__ void fast_stage(const fftz_pass_t &P, typename Cplx<T
       const int d0 = (b - k) * R + k;
       if (LAST) {
         if (valid) {
-          if constexpr ((FEAT & FEAT_TABS) != 0) {
+          const int64_t oes = P.oes;
+          T2 *ob = (T2 *)P.out + s_out[p] + (int64_t)d0 * oes;
+          const int64_t st = (int64_t)NS * oes;
+          const bool cj = (P.flags & FFTZ_F_CONJ_OUT) != 0;
+          // four-step factor of output d0 + r NS: W^{col d0} (W^{col NS})^r,
+          // two table products per chain start and one for the step, then
+          // a chain of at most CH - 1 products (CH = 8 for radix 16)
+          constexpr int CH = R > 8 ? R / 2 : R;
+          T2 w = zero2<T2>(), stp = zero2<T2>();
+          if constexpr ((FEAT & FEAT_TW4) != 0) {
+            stp = tw4<T>(P, col, NS);
+            w = tw4<T>(P, col, d0);
+          }
 #pragma unroll
-            for (int r = 0; r < R; r++) store_fast<T, FEAT>(P, v[q][r], d0 + r * NS, col, s_out[p]);
-          } else {
-            const int64_t oes = P.oes;
-            T2 *ob = (T2 *)P.out + s_out[p] + (int64_t)d0 * oes;
-            const int64_t st = (int64_t)NS * oes;
-            const bool cj = (P.flags & FFTZ_F_CONJ_OUT) != 0;
-            // four-step factor of output d0 + r NS: W^{col d0} (W^{col NS})^r,
-            // two table products per chain start and one for the step, then
-            // a chain of at most CH - 1 products (CH = 8 for radix 16)
-            constexpr int CH = R > 8 ? R / 2 : R;
-            T2 w = zero2<T2>(), stp = zero2<T2>();
+          for (int r = 0; r < R; r++) {
+            T2 y = v[q][r];
             if constexpr ((FEAT & FEAT_TW4) != 0) {
-              stp = tw4<T>(P, col, NS);
-              w = tw4<T>(P, col, d0);
+              if (r > 0 && r % CH == 0) w = tw4<T>(P, col, d0 + r * NS);
+              y = cmul(y, w);
+              if ((r + 1) % CH != 0) w = cmul(w, stp);
             }
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-              T2 y = v[q][r];
-              if constexpr ((FEAT & FEAT_TW4) != 0) {
-                if (r > 0 && r % CH == 0) w = tw4<T>(P, col, d0 + r * NS);
-                y = cmul(y, w);
-                if ((r + 1) % CH != 0) w = cmul(w, stp);
-              }
-              if (cj) y.y = -y.y;
-              ob[r * st] = y;
-            }
+            if (cj) y.y = -y.y;
+            ob[r * st] = y;
           }
         }
       } else if constexpr (NS % PAD == 0) {
@@ -340,25 +288,7 @@ __device__ __forceinline__ void fast_tile(const fftz_pass_t &P, int64_t tf0, uns
     for (int i = threadIdx.x; i < ct_tw_total(N); i += blockDim.x) twb[i] = __ldg(g + i);
   }
   __syncthreads();
-  if (FEAT & FEAT_SWEEP2) {
-    constexpr int SH = Cplx<T>::PADSH;
-    FastStages<T, N, 0, ct_nstages(N), 0, 2, FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
-    const T2 *mt = (const T2 *)P.mid_tab;
-    for (int i = threadIdx.x; i < P.tpc * N; i += blockDim.x) {
-      const int p = i / N;
-      const int e = i - p * N;
-      const int64_t c = s_col[p];
-      if (c < 0) continue;
-      T2 *a = sdata + (size_t)p * P.sstride + phys<SH>(e);
-      T2 v = *a;
-      v.y = -v.y;
-      *a = cmul(v, __ldg(mt + e + c * P.mid_cs));
-    }
-    __syncthreads();
-    FastStages<T, N, 0, ct_nstages(N), 1, 2, FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
-  } else {
-    FastStages<T, N, 0, ct_nstages(N), 0, 1, FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
-  }
+  FastStages<T, N, 0, ct_nstages(N), 0, 1, FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
 }
 
 template <typename T, int N, int FEAT>

@@ -6,9 +6,7 @@
 extern "C" {
 
 const void *fftz_fast_f32_a(int log2n, int feat);
-const void *fftz_fast_f32_b(int log2n, int feat);
 const void *fftz_fast_f64_a(int log2n, int feat);
-const void *fftz_fast_f64_b(int log2n, int feat);
 const void *fftz_fast_f32_c(int log2n, int feat);
 const void *fftz_fast_f64_c(int log2n, int feat);
 const void *fftz_fast_real_kernel(int dtype, int log2n);
@@ -18,18 +16,13 @@ static const void *fast_kernel(int dtype, int log2n, int variant) {
   switch (variant) {
     case FFTZ_VAR_FAST: feat = 0; break;
     case FFTZ_VAR_FAST_TW4: feat = fftz::FEAT_TW4; break;
-    case FFTZ_VAR_FAST_TABS: feat = fftz::FEAT_TABS; break;
-    case FFTZ_VAR_FAST_TW4_TABS: feat = fftz::FEAT_TW4 | fftz::FEAT_TABS; break;
-    case FFTZ_VAR_FAST_BLUE: feat = fftz::FEAT_TABS | fftz::FEAT_SWEEP2; break;
     case FFTZ_VAR_PIPE: feat = 16; break;
     case FFTZ_VAR_PIPE_TW4: feat = 16 | fftz::FEAT_TW4; break;
     case FFTZ_VAR_FAST_REAL: return fftz_fast_real_kernel(dtype, log2n);
     default: return 0;
   }
   if (feat >= 16) return dtype == 0 ? fftz_fast_f32_c(log2n, feat) : fftz_fast_f64_c(log2n, feat);
-  const void *f = dtype == 0 ? fftz_fast_f32_a(log2n, feat) : fftz_fast_f64_a(log2n, feat);
-  if (!f) f = dtype == 0 ? fftz_fast_f32_b(log2n, feat) : fftz_fast_f64_b(log2n, feat);
-  return f;
+  return dtype == 0 ? fftz_fast_f32_a(log2n, feat) : fftz_fast_f64_a(log2n, feat);
 }
 
 int fftz_max_smem_n(int dtype) { return dtype == 0 ? 16384 : 8192; }
@@ -106,11 +99,9 @@ int32_t fftz_fast_tw_entries(int n) {
 int64_t fftz_pass_smem_bytes(const fftz_pass_t *p) {
   if (p->variant == FFTZ_VAR_TC) return fftz_tc_smem_bytes();
   const int64_t esz = p->dtype == 0 ? 8 : 16;
-  if (p->variant == FFTZ_VAR_GENERIC_PP)
-    return 2 * (int64_t)p->tpc * p->sstride * esz + 3 * 8 * (int64_t)p->tpc + 8 * FFTZ_MAX_STAGES;
   if (p->variant == FFTZ_VAR_MR)
-    return (int64_t)p->tpc * p->sstride * esz + ((p->flags & FFTZ_F_TW4) ? 16 * esz * p->tpc : 0) +
-           3 * 8 * (int64_t)p->tpc;
+    return (((int64_t)p->tpc * p->sstride * esz + 15) & ~(int64_t)15) +
+           ((p->flags & FFTZ_F_TW4) ? 16 * esz * p->tpc : 0) + 32 * (int64_t)p->tpc;
   if (is_pipe(p)) return 2 * (int64_t)p->tpc * p->sstride * esz + 9 * 8 * (int64_t)p->tpc;
   int64_t b = (int64_t)p->tpc * p->sstride * esz + 3 * 8 * (int64_t)p->tpc;
   if (p->smem_tw) b += 16 + (int64_t)fftz_fast_tw_entries(p->n) * esz;  // shared copy of the stage twiddles
@@ -136,12 +127,10 @@ int fftz_launch_pass(const fftz_pass_t *p, void *stream) {
   if (p->variant == FFTZ_VAR_GENERIC) {
     fn = p->dtype == 0 ? (const void *)&fftz::fft_smem_kernel_occ3<float>
                        : (const void *)&fftz::fft_smem_kernel<double>;
-  } else if (p->variant == FFTZ_VAR_GENERIC_PP) {
-    fn = p->dtype == 0 ? (const void *)&fftz::fft_pp_kernel<float> : (const void *)&fftz::fft_pp_kernel<double>;
   } else if (p->variant == FFTZ_VAR_MR) {
-    int feat = (p->flags & FFTZ_F_TW4) ? 1 : 0;
-    if ((p->flags & (FFTZ_F_PRE_TAB | FFTZ_F_POST_TAB | FFTZ_F_SCALE)) || p->pre_n || p->post_n) feat = 2;
-    if (p->flags & FFTZ_F_MID_TAB) feat = 2 | 4;
+    const int f = p->flags;
+    const int feat = ((f & FFTZ_F_TW4) ? 1 : 0) | ((f & FFTZ_F_PRE_TAB) ? 2 : 0) | ((f & FFTZ_F_POST_TAB) ? 4 : 0) |
+                     ((f & FFTZ_F_MID_TAB) ? 8 : 0);
     fn = p->dtype == 0 ? fftz_mr_kernel_f32(feat, p->mr.big) : fftz_mr_kernel_f64(feat, p->mr.big);
   } else {
     fn = fast_kernel(p->dtype, fftz::ct_log2(p->n), p->variant);
@@ -155,9 +144,7 @@ int fftz_launch_pass(const fftz_pass_t *p, void *stream) {
     if (e != cudaSuccess) return (int)e;
     if (nopted[dev] < 96) opted[dev][nopted[dev]++] = fn;
   }
-  const dim3 block(p->variant == FFTZ_VAR_GENERIC_PP ? 256u
-                   : p->variant == FFTZ_VAR_MR       ? (unsigned)p->threads
-                                                     : (unsigned)(p->tpc * p->tpt));
+  const dim3 block(p->variant == FFTZ_VAR_MR ? (unsigned)p->threads : (unsigned)(p->tpc * p->tpt));
   const size_t smem = (size_t)fftz_pass_smem_bytes(p);
   dim3 grid((unsigned)nblk);
   if (is_pipe(p)) {

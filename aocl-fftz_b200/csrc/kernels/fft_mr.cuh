@@ -3,7 +3,7 @@
 //
 // A line of n = R_0 R_1 ... R_{S-1} points sits in shared memory in its natural
 // digit order, position sum_s d_s M_s with M_s = R_{s+1} ... R_{S-1} (plus
-// mr_pad slots per step of digit 0). Stage s transforms digit s in place
+// mr.pad slots per step of digit 0). Stage s transforms digit s in place
 // (decimation in frequency): a butterfly reads its R_s values M_s apart,
 // transforms them, multiplies by W_{R_s M_s}^{k r} (r = position below digit s)
 // and writes them back to the same slots, so one buffer and one barrier a
@@ -15,6 +15,10 @@
 // stage in registers: the second sweep runs the stages backwards (decimation
 // in time), from digit-reversed to natural order, with the same twiddles.
 //
+// What a stage reads of its pass is copied to locals before its loop: in the
+// ragged executor the pass lies in shared memory, where the loop's own stores
+// would force every field to be read again for each butterfly.
+//
 // What bounds it: HBM for long batches, instruction issue otherwise; see the
 // measurements beside fft_mr_kernel.
 #pragma once
@@ -23,69 +27,98 @@
 
 namespace fftz {
 
-enum { FEAT_MR_TW4 = 1, FEAT_MR_TABS = 2, FEAT_MR_BLUE = 4 };
+// Features of a pass, all compile-time: a form for every combination the planner
+// makes. (One form with run-time flags for the table passes spent most of its time
+// waiting for instructions: 11 of 19 stall cycles an instruction in a 256-point
+// chirp pass.) TW4: output k of column c times W_{tw4_n}^{c k}. PRE / POST: bound
+// and table product on the load / store side. BLUE: two sweeps around mid_tab.
+enum { FEAT_MR_TW4 = 1, FEAT_MR_PRE = 2, FEAT_MR_POST = 4, FEAT_MR_BLUE = 8 };
 
 // x / d by the host's m = ceil(2^32 / d) (0 for d = 1); exact while x d < 2^32
 __device__ __forceinline__ int mr_div(int x, uint32_t m) { return m ? (int)__umulhi((uint32_t)x, m) : x; }
 
-// Per-tile view shared by the stages.
-template <typename T> struct MrTile {
-  typename Cplx<T>::type *sd;   // tpc lines, P.sstride apart
-  typename Cplx<T>::type *stp;  // four-step factors W^{col nb r}: 16 per line
-  const int64_t *s_in, *s_out, *s_col;
-  int nl;                       // lines of the tile that exist (the last tile may be short)
+// Offset of a line on one HBM side, and its column.
+struct __align__(16) MrLine {
+  int64_t off, col;
 };
 
-// Four-step factor of output K of column col: col * K < tw4_n, both below
-// 2^28 elements, so no reduction and 32 bits are enough.
-template <typename T>
-__device__ __forceinline__ typename Cplx<T>::type mr_tw4(const fftz_pass_t &P, uint32_t r) {
-  typedef typename Cplx<T>::type T2;
-  const int sh = 31 - __clz((int)P.tw4_l);
-  return cmul(__ldg((const T2 *)P.tw4_hi + (r >> sh)), __ldg((const T2 *)P.tw4_lo + (r & ((1u << sh) - 1u))));
+// A tile's shared memory: tpc lines P.sstride apart, the four-step factors
+// W^{col nb r} (16 per line), the lines' places on the input and output side, a
+// copy of the stage twiddles in the executor (otherwise they are read through L1);
+// nl of the lines exist (the last tile of a pass may be short).
+template <typename T> struct MrTile {
+  typename Cplx<T>::type *sd, *stp;
+  const MrLine *in, *out;
+  int nl;
+  bool has_tw;                       // tw holds the stage twiddles
+  const typename Cplx<T>::type *tw;  // (a shared-memory array: never NULL, since the
+                                     // compiler's shared-memory address of NULL is not)
+};
+
+// W_{tw4_n}^r from the two factor tables: r = column * output < tw4_n, both
+// below 2^28 elements, so no reduction and 32 bits are enough.
+template <typename T2> struct MrTw4 {
+  const T2 *hi, *lo;
+  int sh;
+  __device__ __forceinline__ T2 operator()(uint32_t r) const {
+    return cmul(__ldg(hi + (r >> sh)), __ldg(lo + (r & ((1u << sh) - 1u))));
+  }
+};
+
+template <typename T2> __device__ __forceinline__ MrTw4<T2> mr_tw4(const fftz_pass_t &P) {
+  const int l = (int)P.tw4_l;
+  return MrTw4<T2>{(const T2 *)P.tw4_hi, (const T2 *)P.tw4_lo, 31 - __clz(l)};
 }
 
 // Outputs K + r nb (r < R) of line p.
-template <typename T, int R, int FEAT>
-__device__ __forceinline__ void mr_store(const fftz_pass_t &P, const MrTile<T> &t, const typename Cplx<T>::type (&v)[R],
-                                         int p, int K, int nb) {
-  typedef typename Cplx<T>::type T2;
-  const int64_t col = t.s_col[p];
-  const int64_t oes = P.oes;
-  T2 *g = (T2 *)P.out + t.s_out[p] + (int64_t)K * oes;
-  const int64_t st = (int64_t)nb * oes;
-  const bool cj = (P.flags & FFTZ_F_CONJ_OUT) != 0;
-  const bool tw4 = (FEAT & FEAT_MR_TW4) || ((FEAT & FEAT_MR_TABS) && (P.flags & FFTZ_F_TW4));
-  T2 w = zero2<T2>();
-  if (tw4) w = mr_tw4<T>(P, (uint32_t)col * (uint32_t)K);
-  const T2 *stp = t.stp + p * 16;
-  if constexpr ((FEAT & FEAT_MR_TABS) != 0) {
-    const int pes = (int)P.post_es, pn = P.post_n > 0 ? (int)P.post_n : 0x7fffffff;
-    const int l0 = (int)(col * P.post_cs) + K * pes, ls = nb * pes;
-    const bool post = (P.flags & FFTZ_F_POST_TAB) != 0, sc = (P.flags & FFTZ_F_SCALE) != 0;
+// Table factors in flight beside R values: as many as the registers hold (float
+// 64, double 128).
+template <int R> __host__ __device__ constexpr int mr_chunk() { return R <= 8 ? R : R <= 12 ? 6 : 4; }
+
+// v[r] *= tab[min(l0 + r ls, last)], C factors in flight
+template <typename T2, int R>
+__device__ __forceinline__ void mr_table(T2 (&v)[R], const T2 *tab, int l0, int ls, int last) {
+  constexpr int C = mr_chunk<R>();
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      T2 y = v[r];
-      if (tw4) y = cmul(y, r ? cmul(w, stp[r]) : w);
-      if (cj) y.y = -y.y;
-      const int li = l0 + r * ls;
-      if (li < pn) {
-        if (post) y = cmul(y, __ldg((const T2 *)P.post_tab + li));
-        if (sc) {
-          y.x = (T)(y.x * P.scale);
-          y.y = (T)(y.y * P.scale);
-        }
-        g[r * st] = y;
-      }
-    }
+  for (int q = 0; q < R; q += C) {
+    T2 w[C];
+#pragma unroll
+    for (int r = q; r < R && r < q + C; r++) w[r - q] = __ldg(tab + min(l0 + r * ls, last));
+#pragma unroll
+    for (int r = q; r < R && r < q + C; r++) v[r] = cmul(v[r], w[r - q]);
+  }
+}
+
+// Outputs K + r nb (r < R) of line p (v is used up).
+template <typename T, int R, int FEAT>
+__device__ __forceinline__ void mr_store(const fftz_pass_t &P, const MrTile<T> &t, typename Cplx<T>::type (&v)[R], int p,
+                                         int K, int nb) {
+  typedef typename Cplx<T>::type T2;
+  const MrLine L = t.out[p];
+  const int64_t oes = P.oes;
+  T2 *g = (T2 *)P.out + L.off + (int64_t)K * oes;
+  const int64_t st = (int64_t)nb * oes;
+  if constexpr ((FEAT & FEAT_MR_TW4) != 0) {
+    const T2 w = mr_tw4<T2>(P)((uint32_t)L.col * (uint32_t)K);
+    const T2 *stp = t.stp + p * 16;
+    v[0] = cmul(v[0], w);
+#pragma unroll
+    for (int r = 1; r < R; r++) v[r] = cmul(v[r], cmul(w, stp[r]));
+  }
+  if (P.flags & FFTZ_F_CONJ_OUT) {
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r].y = -v[r].y;
+  }
+  if constexpr ((FEAT & FEAT_MR_POST) != 0) {
+    const int pes = (int)P.post_es, pn = (int)P.post_n;
+    const int l0 = (int)(L.col * P.post_cs) + K * pes, ls = nb * pes;
+    mr_table<T2, R>(v, (const T2 *)P.post_tab, l0, ls, pn - 1);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (l0 + r * ls < pn) g[r * st] = v[r];
   } else {
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      T2 y = v[r];
-      if (tw4) y = cmul(y, r ? cmul(w, stp[r]) : w);
-      if (cj) y.y = -y.y;
-      g[r * st] = y;
-    }
+    for (int r = 0; r < R; r++) g[r * st] = v[r];
   }
 }
 
@@ -94,73 +127,93 @@ template <typename T, int R, int FEAT>
 __device__ __forceinline__ void mr_load(const fftz_pass_t &P, const MrTile<T> &t, typename Cplx<T>::type (&v)[R], int p,
                                         int rest, int nb) {
   typedef typename Cplx<T>::type T2;
-  const int64_t col = t.s_col[p];
-  const T2 *g = (const T2 *)P.in + t.s_in[p] + (int64_t)rest * P.ies;
-  const int64_t st = (int64_t)nb * P.ies;
+  const MrLine L = t.in[p];
+  const int64_t ies = P.ies;
+  const T2 *g = (const T2 *)P.in + L.off + (int64_t)rest * ies;
+  const int64_t st = (int64_t)nb * ies;
   const bool cj = (P.flags & FFTZ_F_CONJ_IN) != 0;
-  if constexpr ((FEAT & FEAT_MR_TABS) != 0) {
-    const int pes = (int)P.pre_es, pn = P.pre_n > 0 ? (int)P.pre_n : 0x7fffffff;
-    const int l0 = (int)(col * P.pre_cs) + rest * pes, ls = nb * pes;
-    const bool pre = (P.flags & FFTZ_F_PRE_TAB) != 0;
+  if constexpr ((FEAT & FEAT_MR_PRE) != 0) {
+    const int pes = (int)P.pre_es, pn = (int)P.pre_n;
+    const int l0 = (int)(L.col * P.pre_cs) + rest * pes, ls = nb * pes;
+    // every load first, then the table factors, at an index clamped to the table
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      const int li = l0 + r * ls;
-      T2 x = zero2<T2>();
-      if (li < pn) {
-        x = g[r * st];
-        if (cj) x.y = -x.y;
-        if (pre) x = cmul(x, __ldg((const T2 *)P.pre_tab + li));
-      }
-      v[r] = x;
+      v[r] = zero2<T2>();
+      if (l0 + r * ls < pn) v[r] = g[r * st];
     }
+    if (cj) {
+#pragma unroll
+      for (int r = 0; r < R; r++) v[r].y = -v[r].y;
+    }
+    mr_table<T2, R>(v, (const T2 *)P.pre_tab, l0, ls, pn - 1);
   } else {
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      v[r] = g[r * st];
-      if (cj) v[r].y = -v[r].y;
+    for (int r = 0; r < R; r++) v[r] = g[r * st];
+    if (cj) {
+#pragma unroll
+      for (int r = 0; r < R; r++) v[r].y = -v[r].y;
     }
   }
 }
 
-// item i of a boundary stage (nb butterflies a line) -> line p, position x
-__device__ __forceinline__ void mr_item(const fftz_pass_t &P, int mode, int i, int nb, uint32_t mnb, int &p, int &x) {
-  if (mode == 1) {
-    x = mr_div(i, P.mr.mg_tpc);  // the caller skips p >= nl
-    p = i - x * P.tpc;
-  } else {
-    p = mr_div(i, mnb);
-    x = i - p * nb;
+// item i of a boundary stage (nb butterflies a line) -> line p, position x;
+// with lanes along lines (mode 1) items of lines p >= nl are skipped
+struct MrItems {
+  int mode, tpc, nb, total;
+  uint32_t mg;
+  __device__ __forceinline__ MrItems(const fftz_pass_t &P, int mode_, int nb_, uint32_t mnb, int nl)
+      : mode(mode_), tpc(P.tpc), nb(nb_) {
+    total = (mode == 1 ? tpc : nl) * nb;
+    mg = mode == 1 ? P.mr.mg_tpc : mnb;
   }
-}
+  __device__ __forceinline__ void at(int i, int &p, int &x) const {
+    const int q = mr_div(i, mg);
+    if (mode == 1) {
+      x = q;
+      p = i - q * tpc;
+    } else {
+      p = q;
+      x = i - q * nb;
+    }
+  }
+};
 
+// v[r] *= tw[(r - 1) M + rest], from the table's shared-memory copy sh where the
+// tile has one.
 template <typename T, int R>
-__device__ __forceinline__ void mr_twiddle(const typename Cplx<T>::type *tw, typename Cplx<T>::type (&v)[R], int M,
-                                           int rest) {
+__device__ __forceinline__ void mr_twiddle(const typename Cplx<T>::type *tw, const typename Cplx<T>::type *sh, bool has,
+                                           typename Cplx<T>::type (&v)[R], int M, int rest) {
+  typedef typename Cplx<T>::type T2;
+  if (has) {
+#pragma unroll
+    for (int r = 1; r < R; r++) v[r] = cmul(v[r], sh[(r - 1) * M + rest]);
+    return;
+  }
   // uniform row pointers plus one 32-bit lane offset
-  const uint32_t o = (uint32_t)rest * (uint32_t)sizeof(*tw);
+  const uint32_t o = (uint32_t)rest * (uint32_t)sizeof(T2);
 #pragma unroll
   for (int r = 1; r < R; r++) {
     const char *row = (const char *)(tw + (r - 1) * M);
-    v[r] = cmul(v[r], __ldg((const typename Cplx<T>::type *)(row + o)));
+    v[r] = cmul(v[r], __ldg((const T2 *)(row + o)));
   }
 }
 
 // Stage 0: HBM -> shared memory (S > 1), or HBM -> HBM (S == 1).
 template <typename T, int R, int FEAT>
-__device__ __forceinline__ void mr_first(const fftz_pass_t &P, const MrTile<T> &t) {
+__device__ __forceinline__ void mr_first(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
   typedef typename Cplx<T>::type T2;
-  const int M = P.n / R, S0 = M + P.mr.pad;
-  const T2 *tw = (const T2 *)P.tw + P.tw_off[0];
-  const int total = (P.in_mode == 1 ? P.tpc : t.nl) * M;
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+  const int M = st.m, S0 = M + P.mr.pad, sst = P.sstride;
+  const T2 *tw = (const T2 *)P.tw + st.tw, *sh = t.tw + st.tw;
+  const MrItems it(P, P.in_mode, M, st.mg_nb, t.nl);
+  for (int i = threadIdx.x; i < it.total; i += blockDim.x) {
     int p, rest;
-    mr_item(P, P.in_mode, i, M, P.mr.mg_nb[0], p, rest);
+    it.at(i, p, rest);
     if (p >= t.nl) continue;
     T2 v[R];
     mr_load<T, R, FEAT>(P, t, v, p, rest, M);
     Dft<R>::template apply<T, T2>(v);
-    mr_twiddle<T, R>(tw, v, M, rest);
-    T2 *d = t.sd + p * P.sstride + rest;
+    mr_twiddle<T, R>(tw, sh, t.has_tw, v, M, rest);
+    T2 *d = t.sd + p * sst + rest;
 #pragma unroll
     for (int r = 0; r < R; r++) d[r * S0] = v[r];
   }
@@ -178,52 +231,52 @@ __device__ __forceinline__ void mr_single(const fftz_pass_t &P, const MrTile<T> 
 
 // Stage 0 < s < S - 1 in place; DIT: twiddles before the butterfly (second sweep).
 template <typename T, int R, bool DIT>
-__device__ __forceinline__ void mr_mid(const fftz_pass_t &P, const MrTile<T> &t, int s, int M) {
+__device__ __forceinline__ void mr_mid(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
   typedef typename Cplx<T>::type T2;
-  const int nb = P.n / R, total = t.nl * nb, step = M * (R - 1), pad = P.mr.pad;
-  const uint32_t mnb = P.mr.mg_nb[s], mM = P.mr.mg_m[s], mB = P.mr.mg_b[s];
-  const T2 *tw = (const T2 *)P.tw + P.tw_off[s];
+  const int M = st.m, nb = st.nb, total = t.nl * nb, step = M * (R - 1), pad = P.mr.pad, sst = P.sstride;
+  const uint32_t mnb = st.mg_nb, mM = st.mg_m, mB = st.mg_b;
+  const T2 *tw = (const T2 *)P.tw + st.tw, *sh = t.tw + st.tw;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int p = mr_div(i, mnb);
     const int j = i - p * nb;
     const int b = mr_div(j, mM);
     const int rest = j - b * M;
-    T2 *d = t.sd + p * P.sstride + j + b * step + mr_div(b, mB) * pad;
+    T2 *d = t.sd + p * sst + j + b * step + mr_div(b, mB) * pad;
     T2 v[R];
 #pragma unroll
     for (int r = 0; r < R; r++) v[r] = d[r * M];
-    if (DIT) mr_twiddle<T, R>(tw, v, M, rest);
+    if (DIT) mr_twiddle<T, R>(tw, sh, t.has_tw, v, M, rest);
     Dft<R>::template apply<T, T2>(v);
-    if (!DIT) mr_twiddle<T, R>(tw, v, M, rest);
+    if (!DIT) mr_twiddle<T, R>(tw, sh, t.has_tw, v, M, rest);
 #pragma unroll
     for (int r = 0; r < R; r++) d[r * M] = v[r];
   }
 }
 
 // Slot of the last stage's butterfly K = k_0 + R_0 (k_1 + R_1 (...)).
-__device__ __forceinline__ int mr_slot(const fftz_pass_t &P, int K) {
-  const int S0 = P.mr.m[0] + P.mr.pad, S = P.nstages;
+__device__ __forceinline__ int mr_slot(const fftz_pass_t &P, int S, int S0, int K) {
   if (S == 2) return K * S0;
-  int q = mr_div(K, P.mr.mg_r[0]);
-  int o = (K - q * P.radix[0]) * S0;
+  int q = mr_div(K, P.mr.st[0].mg_r);
+  int o = (K - q * P.mr.st[0].r) * S0;
   for (int s = 1; s < S - 2; s++) {
-    const int x = mr_div(q, P.mr.mg_r[s]);
-    o += (q - x * P.radix[s]) * P.mr.m[s];
+    const int x = mr_div(q, P.mr.st[s].mg_r);
+    o += (q - x * P.mr.st[s].r) * P.mr.st[s].m;
     q = x;
   }
-  return o + q * P.mr.m[S - 2];
+  return o + q * P.mr.st[S - 2].m;
 }
 
 // Last stage: shared memory -> HBM, butterflies in output order.
 template <typename T, int R, int FEAT>
-__device__ __forceinline__ void mr_last(const fftz_pass_t &P, const MrTile<T> &t, int s) {
+__device__ __forceinline__ void mr_last(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
   typedef typename Cplx<T>::type T2;
-  const int nb = P.n / R, total = (P.out_mode == 1 ? P.tpc : t.nl) * nb;
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+  const int nb = st.nb, S = P.nstages, S0 = P.mr.st[0].m + P.mr.pad, sst = P.sstride;
+  const MrItems it(P, P.out_mode, nb, st.mg_nb, t.nl);
+  for (int i = threadIdx.x; i < it.total; i += blockDim.x) {
     int p, K;
-    mr_item(P, P.out_mode, i, nb, P.mr.mg_nb[s], p, K);
+    it.at(i, p, K);
     if (p >= t.nl) continue;
-    const T2 *d = t.sd + p * P.sstride + mr_slot(P, K);
+    const T2 *d = t.sd + p * sst + mr_slot(P, S, S0, K);
     T2 v[R];
 #pragma unroll
     for (int r = 0; r < R; r++) v[r] = d[r];
@@ -235,24 +288,24 @@ __device__ __forceinline__ void mr_last(const fftz_pass_t &P, const MrTile<T> &t
 // Two-sweep passes: last stage of the first FFT, v = conj(v) * mid_tab, first
 // stage of the second FFT, in place.
 template <typename T, int R>
-__device__ __forceinline__ void mr_product(const fftz_pass_t &P, const MrTile<T> &t, int s) {
+__device__ __forceinline__ void mr_product(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
   typedef typename Cplx<T>::type T2;
-  const int nb = P.n / R, total = t.nl * nb;
+  const int nb = st.nb, total = t.nl * nb, S = P.nstages, S0 = P.mr.st[0].m + P.mr.pad, sst = P.sstride;
+  const uint32_t mnb = st.mg_nb;
+  const T2 *mid = (const T2 *)P.mid_tab;
+  const int64_t mid_cs = P.mid_cs;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
-    const int p = mr_div(i, P.mr.mg_nb[s]);
+    const int p = mr_div(i, mnb);
     const int K = i - p * nb;
-    T2 *d = t.sd + p * P.sstride + mr_slot(P, K);
+    T2 *d = t.sd + p * sst + mr_slot(P, S, S0, K);
     T2 v[R];
 #pragma unroll
     for (int r = 0; r < R; r++) v[r] = d[r];
     Dft<R>::template apply<T, T2>(v);
-    const T2 *mt = (const T2 *)P.mid_tab + t.s_col[p] * P.mid_cs + K;
+    const T2 *mt = mid + t.in[p].col * mid_cs + K;
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      T2 x = v[r];
-      x.y = -x.y;
-      v[r] = cmul(x, __ldg(mt + r * nb));
-    }
+    for (int r = 0; r < R; r++) v[r].y = -v[r].y;
+    mr_table<T2, R>(v, mt, 0, nb, 0x7fffffff);
     Dft<R>::template apply<T, T2>(v);
 #pragma unroll
     for (int r = 0; r < R; r++) d[r] = v[r];
@@ -261,96 +314,101 @@ __device__ __forceinline__ void mr_product(const fftz_pass_t &P, const MrTile<T>
 
 // Second sweep's last stage (digit 0): shared memory -> HBM, natural order.
 template <typename T, int R, int FEAT>
-__device__ __forceinline__ void mr_dit_last(const fftz_pass_t &P, const MrTile<T> &t) {
+__device__ __forceinline__ void mr_dit_last(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
   typedef typename Cplx<T>::type T2;
-  const int M = P.n / R, S0 = M + P.mr.pad;
-  const T2 *tw = (const T2 *)P.tw + P.tw_off[0];
-  const int total = (P.out_mode == 1 ? P.tpc : t.nl) * M;
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+  const int M = st.m, S0 = M + P.mr.pad, sst = P.sstride;
+  const T2 *tw = (const T2 *)P.tw + st.tw, *sh = t.tw + st.tw;
+  const MrItems it(P, P.out_mode, M, st.mg_nb, t.nl);
+  for (int i = threadIdx.x; i < it.total; i += blockDim.x) {
     int p, rest;
-    mr_item(P, P.out_mode, i, M, P.mr.mg_nb[0], p, rest);
+    it.at(i, p, rest);
     if (p >= t.nl) continue;
-    const T2 *d = t.sd + p * P.sstride + rest;
+    const T2 *d = t.sd + p * sst + rest;
     T2 v[R];
 #pragma unroll
     for (int r = 0; r < R; r++) v[r] = d[r * S0];
-    mr_twiddle<T, R>(tw, v, M, rest);
+    mr_twiddle<T, R>(tw, sh, t.has_tw, v, M, rest);
     Dft<R>::template apply<T, T2>(v);
     mr_store<T, R, FEAT>(P, t, v, p, rest, M);
   }
 }
 
-// BIG: radices 11 and 13 too (their butterflies hold more live values).
-#define FZ_MR_SWITCH(R_, BIG, CALL)                       \
-  switch (R_) {                                           \
-    case 2: { constexpr int R = 2; CALL; } break;         \
-    case 3: { constexpr int R = 3; CALL; } break;         \
-    case 4: { constexpr int R = 4; CALL; } break;         \
-    case 5: { constexpr int R = 5; CALL; } break;         \
-    case 6: { constexpr int R = 6; CALL; } break;         \
-    case 7: { constexpr int R = 7; CALL; } break;         \
-    case 8: { constexpr int R = 8; CALL; } break;         \
-    case 9: { constexpr int R = 9; CALL; } break;         \
-    case 10: { constexpr int R = 10; CALL; } break;       \
-    case 11: if constexpr (BIG) { constexpr int R = 11; CALL; } break; \
-    case 12: { constexpr int R = 12; CALL; } break;       \
-    case 13: if constexpr (BIG) { constexpr int R = 13; CALL; } break; \
-    case 14: { constexpr int R = 14; CALL; } break;       \
-    case 15: { constexpr int R = 15; CALL; } break;       \
-    case 16: { constexpr int R = 16; CALL; } break;       \
+// Radix sets: MR_SMOOTH without 11 and 13 (whose butterflies hold more live
+// values) and MR_ALL.
+enum { MR_SMOOTH = 0, MR_ALL = 1 };
+__host__ __device__ constexpr bool mr_has(int set, int R) {
+  return set == MR_ALL || (R != 11 && R != 13);
+}
+#define FZ_MR_CASE(SET, R_, CALL) \
+  case R_:                        \
+    if constexpr (mr_has(SET, R_)) { constexpr int R = R_; CALL; } \
+    break;
+#define FZ_MR_SWITCH(R_, SET, CALL)                                                                             \
+  switch (R_) {                                                                                                 \
+    FZ_MR_CASE(SET, 2, CALL) FZ_MR_CASE(SET, 3, CALL) FZ_MR_CASE(SET, 4, CALL) FZ_MR_CASE(SET, 5, CALL)         \
+    FZ_MR_CASE(SET, 6, CALL) FZ_MR_CASE(SET, 7, CALL) FZ_MR_CASE(SET, 8, CALL) FZ_MR_CASE(SET, 9, CALL)         \
+    FZ_MR_CASE(SET, 10, CALL) FZ_MR_CASE(SET, 11, CALL) FZ_MR_CASE(SET, 12, CALL) FZ_MR_CASE(SET, 13, CALL)     \
+    FZ_MR_CASE(SET, 14, CALL) FZ_MR_CASE(SET, 15, CALL) FZ_MR_CASE(SET, 16, CALL)                               \
   }
 
+// Four-step factors W^{col nb r} of the final butterflies of radix Rl (outputs
+// nb apart), formed per line; read after the caller's next barrier.
+template <typename T> __device__ __forceinline__ void mr_steps(const fftz_pass_t &P, const MrTile<T> &t, int Rl) {
+  typedef typename Cplx<T>::type T2;
+  const uint32_t nb = (uint32_t)(P.n / Rl);
+  const MrTw4<T2> w = mr_tw4<T2>(P);
+  for (int i = threadIdx.x; i < 16 * t.nl; i += blockDim.x) {
+    const int p = i >> 4, r = i & 15;
+    if (r < Rl) t.stp[i] = w((uint32_t)t.out[p].col * (nb * (uint32_t)r));
+  }
+}
+
 // One CTA-worth of a pass: transforms [blk * tpc, (blk + 1) * tpc).
-template <typename T, int FEAT, bool BIG>
+template <typename T, int FEAT, int SET>
 __device__ __forceinline__ void mr_tile(const fftz_pass_t &P, int64_t blk, unsigned char *smem_raw) {
   typedef typename Cplx<T>::type T2;
-  constexpr bool TW4 = (FEAT & (FEAT_MR_TW4 | FEAT_MR_TABS)) != 0;
+  const int S = P.nstages, tpc = P.tpc;
   MrTile<T> t;
   t.sd = (T2 *)smem_raw;
-  t.stp = t.sd + (size_t)P.tpc * P.sstride;
-  int64_t *s_in = (int64_t *)(t.stp + ((P.flags & FFTZ_F_TW4) ? 16 * P.tpc : 0));
-  int64_t *s_out = s_in + P.tpc, *s_col = s_out + P.tpc;
-  t.s_in = s_in;
-  t.s_out = s_out;
-  t.s_col = s_col;
-  t.nl = P.ntf - blk * P.tpc < P.tpc ? (int)(P.ntf - blk * P.tpc) : P.tpc;
-  for (int p = threadIdx.x; p < P.tpc; p += blockDim.x)
-    batch_offsets(P, blk * P.tpc + p, s_in + p, s_out + p, s_col + p);
+  t.stp = (T2 *)(smem_raw + (((size_t)tpc * P.sstride * sizeof(T2) + 15) & ~(size_t)15));
+  MrLine *in = (MrLine *)(t.stp + ((FEAT & FEAT_MR_TW4) ? 16 * tpc : 0)), *out = in + tpc;
+  t.has_tw = false;
+  t.tw = t.sd;
+  t.in = in;
+  t.out = out;
+  t.nl = P.ntf - blk * tpc < tpc ? (int)(P.ntf - blk * tpc) : tpc;
+  for (int p = threadIdx.x; p < t.nl; p += blockDim.x) {
+    batch_offsets(P, blk * tpc + p, &in[p].off, &out[p].off, &in[p].col);
+    out[p].col = in[p].col;
+  }
   __syncthreads();
-  const int S = P.nstages;
-  if (TW4 && (P.flags & FFTZ_F_TW4)) {
-    // W^{col nb r} of the final butterflies (outputs nb apart), formed per line
-    const int Rl = (FEAT & FEAT_MR_BLUE) ? P.radix[0] : P.radix[S - 1];
-    const int nb = P.n / Rl;
-    for (int i = threadIdx.x; i < 16 * P.tpc; i += blockDim.x) {
-      const int p = i >> 4, r = i & 15;
-      const int64_t col = s_col[p];
-      if (col >= 0 && r < Rl) t.stp[i] = mr_tw4<T>(P, (uint32_t)col * (uint32_t)(nb * r));
-    }
+  if constexpr ((FEAT & FEAT_MR_TW4) != 0) {
+    mr_steps<T>(P, t, (FEAT & FEAT_MR_BLUE) ? P.mr.st[0].r : P.mr.st[S - 1].r);
     if (S == 1) __syncthreads();
   }
   if (S == 1) {
-    if constexpr ((FEAT & FEAT_MR_BLUE) == 0) FZ_MR_SWITCH(P.radix[0], BIG, (mr_single<T, R, FEAT>(P, t)));
+    if constexpr ((FEAT & FEAT_MR_BLUE) == 0) {
+      if (P.n == 1) mr_single<T, 1, FEAT>(P, t);
+      FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_single<T, R, FEAT>(P, t)));
+    }
     return;
   }
-  FZ_MR_SWITCH(P.radix[0], BIG, (mr_first<T, R, FEAT>(P, t)));
+  FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_first<T, R, FEAT>(P, t, P.mr.st[0])));
   __syncthreads();
   for (int s = 1; s < S - 1; s++) {
-    const int M = P.mr.m[s];
-    FZ_MR_SWITCH(P.radix[s], BIG, (mr_mid<T, R, false>(P, t, s, M)));
+    FZ_MR_SWITCH(P.mr.st[s].r, SET, (mr_mid<T, R, false>(P, t, P.mr.st[s])));
     __syncthreads();
   }
   if constexpr ((FEAT & FEAT_MR_BLUE) != 0) {
-    FZ_MR_SWITCH(P.radix[S - 1], BIG, (mr_product<T, R>(P, t, S - 1)));
+    FZ_MR_SWITCH(P.mr.st[S - 1].r, SET, (mr_product<T, R>(P, t, P.mr.st[S - 1])));
     __syncthreads();
     for (int s = S - 2; s > 0; s--) {
-      const int M = P.mr.m[s];
-      FZ_MR_SWITCH(P.radix[s], BIG, (mr_mid<T, R, true>(P, t, s, M)));
+      FZ_MR_SWITCH(P.mr.st[s].r, SET, (mr_mid<T, R, true>(P, t, P.mr.st[s])));
       __syncthreads();
     }
-    FZ_MR_SWITCH(P.radix[0], BIG, (mr_dit_last<T, R, FEAT>(P, t)));
+    FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_dit_last<T, R, FEAT>(P, t, P.mr.st[0])));
   } else {
-    FZ_MR_SWITCH(P.radix[S - 1], BIG, (mr_last<T, R, FEAT>(P, t, S - 1)));
+    FZ_MR_SWITCH(P.mr.st[S - 1].r, SET, (mr_last<T, R, FEAT>(P, t, P.mr.st[S - 1])));
   }
 }
 

@@ -24,7 +24,7 @@ template <typename T, bool BIG> __host__ __device__ constexpr int mr_lb() {
 template <typename T, int FEAT, bool BIG>
 __global__ void __launch_bounds__(mr_lb<T, BIG>()) fft_mr_kernel(const __grid_constant__ fftz_pass_t P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  mr_tile<T, FEAT, BIG>(P, (int64_t)blockIdx.x, smem_raw);
+  mr_tile<T, FEAT, BIG ? MR_ALL : MR_SMOOTH>(P, (int64_t)blockIdx.x, smem_raw);
 }
 
 }  // namespace fftz
@@ -32,16 +32,16 @@ __global__ void __launch_bounds__(mr_lb<T, BIG>()) fft_mr_kernel(const __grid_co
 /* The mixed-radix kernel for a feature set (FEAT_MR_*), or NULL. */
 extern "C" const void *FZ_MR_GET(int feat, int big) {
   using namespace fftz;
-  if (big) switch (feat) {
-      case 0: return (const void *)&fft_mr_kernel<FZ_MR_T, 0, true>;
-      case FEAT_MR_TW4: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TW4, true>;
-      default: return 0;
+#define FZ_MR_K(F, BIG) \
+  case (F): return (const void *)&fft_mr_kernel<FZ_MR_T, (F), BIG>;
+  if (big) switch (feat) { FZ_MR_K(0, true) FZ_MR_K(FEAT_MR_TW4, true) }
+  else switch (feat) {
+      FZ_MR_K(0, false)
+      FZ_MR_K(FEAT_MR_TW4, false)
+      FZ_MR_K(FEAT_MR_PRE | FEAT_MR_TW4, false)                   // three-pass chirp: columns,
+      FZ_MR_K(FEAT_MR_BLUE | FEAT_MR_TW4, false)                  // rows,
+      FZ_MR_K(FEAT_MR_POST, false)                                // columns of the second FFT
+      FZ_MR_K(FEAT_MR_PRE | FEAT_MR_POST | FEAT_MR_BLUE, false)   // one-kernel chirp
     }
-  switch (feat) {
-    case 0: return (const void *)&fft_mr_kernel<FZ_MR_T, 0, false>;
-    case FEAT_MR_TW4: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TW4, false>;
-    case FEAT_MR_TABS: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TABS, false>;
-    case FEAT_MR_TABS | FEAT_MR_BLUE: return (const void *)&fft_mr_kernel<FZ_MR_T, FEAT_MR_TABS | FEAT_MR_BLUE, false>;
-    default: return 0;
-  }
+  return 0;
 }

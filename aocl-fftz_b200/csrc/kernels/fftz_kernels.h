@@ -46,14 +46,10 @@ enum fftz_out_kind {
 #define FFTZ_VAR_GENERIC 0 /* runtime radix list, any element kind, <= 256 threads   */
 #define FFTZ_VAR_FAST    1 /* compile-time power-of-two shape, complex in/out fused  */
 #define FFTZ_VAR_FAST_TW4 2 /* as FAST with the four-step twiddle epilogue          */
-#define FFTZ_VAR_FAST_TABS 3 /* as FAST with load/store tables, bounds and scale     */
-#define FFTZ_VAR_FAST_TW4_TABS 4 /* both of the above                               */
-#define FFTZ_VAR_FAST_BLUE 5 /* tables plus two sweeps around a mid-table product   */
 #define FFTZ_VAR_PIPE 6      /* persistent, cp.async double-buffered, complex in/out */
 #define FFTZ_VAR_PIPE_TW4 7  /* as PIPE with the four-step twiddle epilogue         */
 #define FFTZ_VAR_TC 8        /* 4096-point rows as two radix-64 tensor-core GEMM stages */
 #define FFTZ_VAR_FAST_REAL 9 /* packed real line: generic load/store phases, compile-time stages */
-#define FFTZ_VAR_GENERIC_PP 10 /* runtime radix list over two shared-memory buffers, 256 threads */
 #define FFTZ_VAR_MR 11       /* runtime radix list (2..16) in place in one shared-memory buffer */
 #define FFTZ_MR_STAGES 8     /* most stages of a mixed-radix line */
 
@@ -70,19 +66,26 @@ enum fftz_out_kind {
 #define FFTZ_F_BLK4_OUT   0x80  /* the pass writes its output blocked */
 #define FFTZ_F_BLK4_IN    0x100 /* the pass reads its input blocked (rows = k) */
 
-/* Mixed-radix line (FFTZ_VAR_MR): digit strides M_s, the slots added per step
- * of digit 0, and ceil(2^32 / d) (0 for d = 1) of the divisors that the
- * stages' index maps need */
+/* Mixed-radix line (FFTZ_VAR_MR): one stage's numbers and ceil(2^32 / d) (0
+ * for d = 1) of the divisors its index map needs, two 16-byte words that a
+ * thread reads together */
+typedef struct fftz_mr_stage
+{
+    int32_t r, m;    /* radix R_s; M_s = R_{s+1} ... R_{S-1} */
+    int32_t nb, tw;  /* butterflies of a line, n / R_s; twiddle block offset */
+    uint32_t mg_nb;  /* d = nb */
+    uint32_t mg_m;   /* d = M_s */
+    uint32_t mg_b;   /* d = R_1 ... R_{s-1}: blocks per digit-0 step */
+    uint32_t mg_r;   /* d = R_s */
+} fftz_mr_stage_t;
+
 typedef struct fftz_mr
 {
-    int32_t pad;                     /* slots between digit-0 blocks beyond M_0 */
-    int32_t m[FFTZ_MR_STAGES];       /* M_s = R_{s+1} ... R_{S-1} */
-    uint32_t mg_nb[FFTZ_MR_STAGES];  /* d = n / R_s: butterflies of a line */
-    uint32_t mg_m[FFTZ_MR_STAGES];   /* d = M_s */
-    uint32_t mg_b[FFTZ_MR_STAGES];   /* d = R_1 ... R_{s-1}: blocks per digit-0 step */
-    uint32_t mg_r[FFTZ_MR_STAGES];   /* d = R_s */
-    uint32_t mg_tpc;                 /* d = tpc */
-    int32_t big;                     /* a radix of 11 or 13 among them */
+    fftz_mr_stage_t st[FFTZ_MR_STAGES];
+    int32_t pad;     /* slots between digit-0 blocks beyond M_0 */
+    uint32_t mg_tpc; /* d = tpc */
+    int32_t big;     /* a radix of 11 or 13 among them */
+    int32_t pad_;
 } fftz_mr_t;
 
 typedef struct fftz_pass
@@ -136,13 +139,17 @@ typedef struct fftz_pass
     int32_t test_tx_short;              /* fault injection (tests): TMA tiles expect this many bytes more
                                            than their copies deliver, so the bounded tile wait runs out */
     const int64_t *ind_in, *ind_out;
+    fftz_mr_t mr;                       /* FFTZ_VAR_MR */
     int32_t threads;                    /* FFTZ_VAR_MR: block size */
-    fftz_mr_t mr;
+    int32_t ntw;                        /* FFTZ_VAR_MR: entries of the stage-twiddle table */
+    int32_t pad2_[2];                   /* a multiple of 16 bytes: the ragged executor copies passes in 16-byte words */
 } fftz_pass_t;
 
 /* Persistent DAG executor (fft_ragged.cu): one launch runs the CTA tiles of
  * many passes; a tile of a pass with a predecessor waits until every tile of
  * the predecessor has completed. */
+#define FFTZ_RG_LINES 64 /* most lines of a tile */
+#define FFTZ_RG_TW 512   /* stage twiddles a tile keeps in shared memory (longer tables stay in L2) */
 #define FFTZ_RBUF_IN 0
 #define FFTZ_RBUF_OUT 1
 #define FFTZ_RBUF_SCRATCH 2
@@ -174,9 +181,6 @@ typedef struct fftz_ragged
 } fftz_ragged_t;
 
 int fftz_launch_ragged(const fftz_ragged_t *r, int grid, void *stream);
-/* 1 if the executor has a compile-time tile for a pass of length n and
- * FFTZ_VAR_FAST* variant (its tpc * tpt must then be 256). */
-int fftz_ragged_fast_ok(int n, int variant);
 /* CTAs of the persistent executor that fit on the device at once. */
 int fftz_ragged_grid(int dtype, int smem_bytes);
 
@@ -251,8 +255,9 @@ int32_t fftz_smem_stride_cols(int dtype, int32_t nslots, int32_t tpc);
 /* Maximum dynamic SMEM bytes per CTA the kernels may use. */
 int64_t fftz_smem_limit(void);
 
-/* Mixed-radix kernel of one dtype for a feature set (1 four-step twiddles,
- * 2 tables, 4 two sweeps; 2 and 4 without radices 11 and 13), or NULL. */
+/* Mixed-radix kernel of one dtype for a feature set (1 four-step twiddles, 2 / 4
+ * table and bound on the load / store side, 8 two sweeps; 2, 4 and 8 without
+ * radices 11 and 13), or NULL. */
 const void *fftz_mr_kernel_f32(int feat, int big);
 const void *fftz_mr_kernel_f64(int feat, int big);
 /* Largest block of those kernels. */

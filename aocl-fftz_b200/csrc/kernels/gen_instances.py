@@ -7,7 +7,6 @@ returning the kernel for that shape, or NULL.
 """
 GROUPS = {
     "a": [(0, 1), (1, 5)],            # (FEAT, smallest log2 n): plain, four-step twiddle
-    "b": [(2, 2), (3, 5), (6, 2)],    # tables, twiddle+tables, two-sweep Bluestein
     "c": [(16, 6), (17, 6)],          # pipelined (FEAT 16 + bits): plain, four-step twiddle
 }
 DTYPES = {"f32": ("float", 14), "f64": ("double", 13)}

@@ -115,7 +115,7 @@ CANDIDATES = [
     dict(fourstep_n1=256), dict(fourstep_n1=1024), dict(fourstep_n1=4096),
     dict(algorithm=2),                        # force a four-step split where possible
     dict(kernel_family=9),                    # 16 x 256 split tiles for every 4096-point float pass
-    dict(kernel_family=12),                   # in-place runtime-radix kernel instead of ping-pong tiles
+    dict(kernel_family=12),                   # in-place runtime-radix kernel instead of mixed-radix tiles
 ]
 
 

@@ -15,9 +15,13 @@ MAXS, MAXB, MRS = 12, 8, 8
 VAR_MR, F_TW4, F_MID = 11, 0x04, 0x40
 
 
+class Stage(C.Structure):
+    _fields_ = [("r", I32), ("m", I32), ("nb", I32), ("tw", I32), ("mg_nb", U32), ("mg_m", U32), ("mg_b", U32),
+                ("mg_r", U32)]
+
+
 class Mr(C.Structure):
-    _fields_ = [("pad", I32), ("m", I32 * MRS), ("mg_nb", U32 * MRS), ("mg_m", U32 * MRS), ("mg_b", U32 * MRS),
-                ("mg_r", U32 * MRS), ("mg_tpc", U32), ("big", I32)]
+    _fields_ = [("st", Stage * MRS), ("pad", I32), ("mg_tpc", U32), ("big", I32), ("pad_", I32)]
 
 
 class Pass(C.Structure):
@@ -31,19 +35,20 @@ class Pass(C.Structure):
                 ("scale", C.c_double), ("in_", VP), ("out", VP), ("tw", VP), ("tw4_hi", VP), ("tw4_lo", VP),
                 ("pre_tab", VP), ("post_tab", VP), ("mid_tab", VP), ("rtw", VP), ("src_buf", I32), ("dst_buf", I32),
                 ("ind_dim", I32), ("use_tma", I32), ("smem_tw", I32), ("test_tx_short", I32), ("ind_in", VP),
-                ("ind_out", VP), ("threads", I32), ("mr", Mr)]
+                ("ind_out", VP), ("mr", Mr), ("threads", I32), ("ntw", I32), ("pad2_", I32 * 2)]
 
 
-def shape(n, dtype=0, col=False, two=False, tw4=False, ntf=100000, tpc=0):
+def shape(n, dtype=0, col=False, two=False, tw4=False, ntf=100000, tpc=0, threads=0, cap=0):
     lib = aoclfftz_b200.load()
     lib.fftz_pass_smem_bytes.restype = I64
     lib.fftz_smem_limit.restype = I64
     p = Pass(n=n, dtype=dtype, ntf=ntf, in_mode=int(col), out_mode=int(col), nbdims=1,
              flags=(F_MID if two else 0) | (F_TW4 if tw4 else 0))
-    assert lib.fz_mr_shape(C.byref(p), tpc) == 0
+    assert lib.fz_mr_shape(C.byref(p), tpc, threads, I64(cap or lib.fftz_smem_limit())) == 0
     assert p.variant == VAR_MR and 1 <= p.tpc <= ntf and 1 <= p.threads <= lib.fftz_mr_max_threads(dtype, p.mr.big)
     assert lib.fftz_pass_smem_bytes(C.byref(p)) <= lib.fftz_smem_limit()
     assert int(np.prod(p.radix[: p.nstages])) == n
+    assert [(st.r, st.nb) for st in p.mr.st[: p.nstages]] == [(R, n // R) for R in p.radix[: p.nstages]]
     return p
 
 
@@ -64,26 +69,26 @@ def items(p, s, col):
     if col:
         x = exact_div(i, p.mr.mg_tpc, p.tpc)
         return i - x * p.tpc, x
-    q = exact_div(i, p.mr.mg_nb[s], nb)
+    q = exact_div(i, p.mr.st[s].mg_nb, nb)
     return q, i - q * nb
 
 
 def mid_slots(p, s):
-    R, M = p.radix[s], p.mr.m[s]
+    R, M = p.radix[s], p.mr.st[s].m
     nb = p.n // R
     i = np.arange(p.tpc * nb)
-    q = exact_div(i, p.mr.mg_nb[s], nb)
+    q = exact_div(i, p.mr.st[s].mg_nb, nb)
     j = i - q * nb
-    b = exact_div(j, p.mr.mg_m[s], M)
+    b = exact_div(j, p.mr.st[s].mg_m, M)
     B = int(np.prod(p.radix[1:s]))
-    return q * p.sstride + j + b * M * (R - 1) + exact_div(b, p.mr.mg_b[s], B) * p.mr.pad, j - b * M
+    return q * p.sstride + j + b * M * (R - 1) + exact_div(b, p.mr.st[s].mg_b, B) * p.mr.pad, j - b * M
 
 
 def last_slots(p, line, K):
     o, q = np.zeros_like(K), K
     for s in range(p.nstages - 1):
-        R, M = p.radix[s], p.mr.m[s]
-        nxt = exact_div(q, p.mr.mg_r[s], R)
+        R, M = p.radix[s], p.mr.st[s].m
+        nxt = exact_div(q, p.mr.st[s].mg_r, R)
         o, q = o + (q - nxt * R) * (M + p.mr.pad if s == 0 else M), nxt
     return line * p.sstride + o
 
@@ -115,7 +120,7 @@ def simulate(p, x, mid=None):
     check_slots(p, first)
     sd[first] = v
     for s in range(1, S - 1):
-        Rs, Ms = p.radix[s], p.mr.m[s]
+        Rs, Ms = p.radix[s], p.mr.st[s].m
         base, rs = mid_slots(p, s)
         a = base + np.arange(Rs)[:, None] * Ms
         check_slots(p, a)
@@ -131,7 +136,7 @@ def simulate(p, x, mid=None):
         return y
     sd[a] = dft(np.conj(v) * mid[K + np.arange(Rl)[:, None] * nb])
     for s in range(S - 2, 0, -1):
-        Rs, Ms = p.radix[s], p.mr.m[s]
+        Rs, Ms = p.radix[s], p.mr.st[s].m
         base, rs = mid_slots(p, s)
         a = base + np.arange(Rs)[:, None] * Ms
         sd[a] = dft(sd[a] * twiddle(Rs, Ms, rs))
@@ -151,7 +156,7 @@ SIZES = [3, 11, 13, 14, 15, 16, 18, 35, 77, 100, 169, 360, 375, 1000, 1080, 1920
 @pytest.mark.parametrize("n", SIZES)
 def test_tile_is_the_transform(n, dtype, col):
     lib = aoclfftz_b200.load()
-    if not lib.fz_mr_fits(dtype, I64(n)):
+    if not lib.fz_mr_fits(dtype, I64(n), I64(227 * 1024)):
         assert n * (8 if dtype == 0 else 16) > 220 * 1024
         return
     p = shape(n, dtype, col)
@@ -178,3 +183,14 @@ def test_lines_per_cta_follow_the_batch_and_the_hint(ntf, tpc):
     p = shape(360, ntf=ntf, tpc=tpc, tw4=True)
     assert p.tpc <= ntf and (tpc == 0 or p.tpc == tpc)
     assert p.tpc == 1 or ntf // p.tpc >= 296 or tpc
+
+
+@pytest.mark.parametrize("n,dtype,ntf,least", [(2, 0, 5000, 64), (144, 0, 40, 14), (5250, 0, 3, 1), (5600, 1, 2, 1), (1, 0, 9, 1)])
+def test_executor_tiles_keep_their_block_and_share(n, dtype, ntf, least):
+    """The ragged executor's tiles: 256 threads, within its share of shared memory, small batches not cut up."""
+    lib = aoclfftz_b200.load()
+    lib.fz_ragged_smem_cap.restype = I64
+    cap = lib.fz_ragged_smem_cap(dtype)
+    p = shape(n, dtype, ntf=ntf, threads=256, cap=cap)
+    assert p.threads == 256 and lib.fftz_pass_smem_bytes(C.byref(p)) <= cap
+    assert least <= p.tpc <= ntf
