@@ -155,7 +155,7 @@ int64_t fz_tc64_tables(fz_blob *b);
 int64_t fz_real_twiddles(fz_blob *b, int dtype, int64_t M);
 
 /* ---- mixed-radix lines (mixed.c) ---- */
-int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost);
+int fz_mr_radices(int64_t n, int min_stages, int pair, int32_t *radix, double *cost);
 int fz_mr_fits(int dtype, int64_t n, int64_t cap);
 int64_t fz_mr_blue_len(int dtype, int64_t n, int64_t cap);
 int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t *n2);

@@ -16,7 +16,7 @@ static int mr_cost(int R)
 typedef struct
 {
     int64_t n; /* the whole line */
-    int min_stages;
+    int min_stages, pair;
     int cur[FFTZ_MR_STAGES], best[FFTZ_MR_STAGES];
     int nbest;
     double score;
@@ -26,6 +26,7 @@ static void mr_try(mr_search *q, int64_t rest, int depth, int top, double cost)
 {
     if (rest == 1)
     {
+        if (q->pair && depth > 1 && q->cur[depth - 1] > 8) return;
         if (depth >= q->min_stages && (q->nbest == 0 || cost < q->score))
         {
             q->score = cost;
@@ -45,14 +46,16 @@ static void mr_try(mr_search *q, int64_t rest, int depth, int top, double cost)
 }
 
 /* Radices (largest first) of the cheapest split of n into at least min_stages
- * stages; returns their number, 0 when n has a prime factor above 13. cost
- * (may be NULL): issue slots a point. */
-int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost)
+ * stages, the last of at most 8 for pair (real lines, whose last stage holds two
+ * butterflies a thread); returns their number, 0 when n has a prime factor above
+ * 13. cost (may be NULL): issue slots a point. */
+int fz_mr_radices(int64_t n, int min_stages, int pair, int32_t *radix, double *cost)
 {
     mr_search q;
     memset(&q, 0, sizeof(q));
     q.n = n;
     q.min_stages = min_stages;
+    q.pair = pair;
     int64_t m = n;
     static const int pr[] = {2, 3, 5, 7, 11, 13};
     for (int i = 0; i < 6; i++)
@@ -65,6 +68,11 @@ int fz_mr_radices(int64_t n, int min_stages, int32_t *radix, double *cost)
     }
     if (n < 2 || m != 1) return 0;
     mr_try(&q, n, 0, 16, 0.0);
+    if (!q.nbest && pair) /* nothing but 11 and 13 */
+    {
+        q.pair = 0;
+        mr_try(&q, n, 0, 16, 0.0);
+    }
     for (int s = 0; s < q.nbest; s++) radix[s] = q.best[s];
     if (cost) *cost = q.score;
     return q.nbest;
@@ -89,7 +97,7 @@ int fz_mr_fits(int dtype, int64_t n, int64_t cap)
     int32_t r[FFTZ_MR_STAGES];
     const int64_t esz = dtype == 0 ? 8 : 16;
     if (n < 1 || (n + 1 + 16) * esz + 32 > cap) return 0;
-    return fz_mr_radices(n, 1, r, NULL) > 0;
+    return fz_mr_radices(n, 1, 0, r, NULL) > 0;
 }
 
 /* the smallest product of 2, 3, 5 and 7 that is at least n */
@@ -117,7 +125,7 @@ int64_t fz_mr_blue_len(int dtype, int64_t n, int64_t cap)
     const int64_t need = 2 * n - 1;
     if (need * (dtype == 0 ? 8 : 16) > cap) return 0;
     for (int64_t m = next_smooth7(need < 4 ? 4 : need); m <= need + need / 4 + 4; m = next_smooth7(m + 1))
-        if (fz_mr_fits(dtype, m, cap) && fz_mr_radices(m, 2, r, &c) > 1 && (!best || (double)m * c < score))
+        if (fz_mr_fits(dtype, m, cap) && fz_mr_radices(m, 2, 0, r, &c) > 1 && (!best || (double)m * c < score))
         {
             best = m;
             score = (double)m * c;
@@ -140,7 +148,7 @@ int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t
         {
             const int64_t b = m / a;
             if (m % a || a > 4 * b || b > 4 * a || !fz_mr_fits(dtype, a, cap) || !fz_mr_fits(dtype, b, cap)) continue;
-            if (fz_mr_radices(a, 1, r, &ca) < 1 || fz_mr_radices(b, 2, r, &cb) < 2) continue;
+            if (fz_mr_radices(a, 1, 0, r, &ca) < 1 || fz_mr_radices(b, 2, 0, r, &cb) < 2) continue;
             if (!best || (double)m * (ca + cb) < score)
             {
                 best = m;
@@ -233,8 +241,18 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
 {
     const int two = (k->flags & FFTZ_F_MID_TAB) != 0;
     const int colmap = k->in_mode == 1 || k->out_mode == 1;
-    k->nstages = fz_mr_radices(k->n, two ? 2 : 1, k->radix, NULL);
+    /* packed real lines: mirrored butterflies in the last (r2c) or first (c2r) stage */
+    const int r2c = k->in_kind == FFTZ_IN_REAL_PAIRS, c2r = k->in_kind == FFTZ_IN_HERM_SEPARATE;
+    k->nstages = fz_mr_radices(k->n, two ? 2 : 1, r2c || c2r, k->radix, NULL);
     if (k->nstages <= 0) return -1;
+    const int ps = r2c ? k->nstages - 1 : c2r ? 0 : -1; /* the paired stage */
+    if (c2r)
+        for (int s = 0; s < k->nstages / 2; s++)
+        {
+            const int32_t x = k->radix[s];
+            k->radix[s] = k->radix[k->nstages - 1 - s];
+            k->radix[k->nstages - 1 - s] = x;
+        }
     k->variant = FFTZ_VAR_MR;
     k->mr.big = 0;
     int64_t M = k->n, B = 1;
@@ -261,7 +279,9 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     if (most > k->ntf) most = k->ntf;
     if (most > (threads ? FZ_RG_LINES : 256)) most = threads ? FZ_RG_LINES : 256;
     /* lines per CTA: about 4096 float / 2048 double points of row lines; whole
-     * 64-byte segments (8 float / 4 double neighbours) of column lines. The
+     * 64-byte segments (8 float / 4 double neighbours) of column lines. Of equal
+ * choices the smaller tile (512-point double r2c rows x 262144: 2 lines 588, 4 521,
+ * 6 591, 8 546 us). The
      * executor's tiles, which wait on memory at their ends, are larger (measured on
      * B200, 4096 ragged transforms, forward: float 1536 points 888 us, 3072 839, 4096
      * 809, 6144 805; double 768 2124, 1536 1753, 2048 1459, 3072 1388, and with later
@@ -282,7 +302,7 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     {
         /* fewer lines where whole CTAs would not give every SM two */
         while (hi > 1 && (hi * k->n > pts + pts / 2 || (threads == 0 && k->ntf / hi < 2 * 148))) hi--;
-        lo = hi > 1 ? (hi + 1) / 2 : 1;
+        lo = hi > 3 ? hi / 3 : 1;
     }
     double best = -1;
     int btpc = 1, bthr = 32;
@@ -301,9 +321,10 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
             double used = 0, spent = 0;
             for (int s = 0; s < k->nstages; s++)
             {
-                const int64_t items = c * (k->n / k->radix[s]);
-                used += (double)items * mr_cost(k->radix[s]);
-                spent += (double)((items + t - 1) / t * t) * mr_cost(k->radix[s]);
+                const int64_t nb = k->n / k->radix[s], items = c * (s == ps ? (nb + 1) / 2 : nb);
+                const int w = mr_cost(k->radix[s]) * (s == ps ? 2 : 1);
+                used += (double)items * w;
+                spent += (double)((items + t - 1) / t * t) * w;
             }
             /* lanes at work, times warps in flight (half weight), times the
              * overlap of independent CTAs' phases */
@@ -335,6 +356,7 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     }
     mr_stride(k, colmap, bp);
     k->mr.mg_tpc = magic(k->tpc);
+    if (ps >= 0) k->mr.mg_pair = magic((k->n / k->radix[ps] + 1) / 2);
     k->fuse_load = k->fuse_store = 1;
     k->use_tma = 0;
     k->smem_tw = 0;

@@ -193,10 +193,6 @@ static void finish_launch_shape(fz_plan *pl, fftz_pass_t *k, int nslots, int max
         int64_t per = pipe ? 4096 : (pl->dtype == 0 ? 4096 : 2048); /* complex elements per CTA */
         want = (int)((per + k->n - 1) / k->n);
         if (want * k->tpt < 128) want = (128 + k->tpt - 1) / k->tpt;
-        /* double real lines in the compile-time real kernel: two lines per CTA
-         * (measured on B200, fp64 512^3 real: r2c 0.95 -> 0.79 ms, c2r 0.79 ->
-         * 0.70 ms against eight lines of 256 points; 1024-point lines equal) */
-        if (k->variant == FFTZ_VAR_FAST_REAL && pl->dtype == 1) want = 2;
     }
     if (colmap && pl->hints.tpc_col > 0) want = pl->hints.tpc_col;
     if (!colmap && pl->hints.tpc_row > 0) want = pl->hints.tpc_row;
@@ -765,7 +761,8 @@ static int plan_c2c(fz_plan *pl, int rank, const fz_dim *dims, int vrank, const 
     return 0;
 }
 
-/* real line along dims[0]: r2c (forward) or c2r (backward) in one generic pass */
+/* real line along dims[0]: r2c (forward) or c2r (backward) in one mixed-radix
+ * pass (kernel_family 12: the older in-place kernel) */
 static fz_pass *real_pass(fz_plan *pl, int64_t n0, int64_t ies, int64_t oes, const fz_dim *b, int nb, int src,
                           int dst)
 {
@@ -800,30 +797,29 @@ static fz_pass *real_pass(fz_plan *pl, int64_t n0, int64_t ies, int64_t oes, con
     int64_t es_out = (k->out_kind == FFTZ_OUT_REAL_PAIRS) ? 2 * oes : oes;
     k->in_mode = (k->nbdims > 0 && absl(k->ibs[0]) < absl(es_in)) ? 1 : 0;
     k->out_mode = (k->nbdims > 0 && absl(k->obs[0]) < absl(es_out)) ? 1 : 0;
-    /* power-of-two packed lines: compile-time stages between the generic
-     * load and store phases (measured on B200, fp64 512^3 r2c: the 512-point
-     * row pass at 1.14 TB/s with the generic kernel) */
-    const int fast = packed && !generic_only(pl) && is_pow2(n) && n <= fast_max_n(pl) &&
-                     !(k->flags & FFTZ_F_CONJ_IN) && fftz_fast_real_kernel(pl->dtype, ilog2i(n)) != NULL;
-    int maxthr = fftz_generic_max_threads();
-    if (fast)
+    if (mixed_lines(pl))
     {
-        k->variant = FFTZ_VAR_FAST_REAL;
-        k->nstages = fftz_fast_radices((int)n, k->radix);
-        k->tpt = fftz_fast_tpt((int)n);
-        maxthr = fast_max_threads(pl);
-    }
-    else
-    {
-        k->variant = FFTZ_VAR_GENERIC;
-        k->nstages = n > 1 ? generic_radices(n, k->radix) : 0;
-        if (k->nstages < 0)
+        const int colm = k->in_mode == 1 || k->out_mode == 1;
+        if (fz_mr_shape(k, colm ? pl->hints.tpc_col : pl->hints.tpc_row, 0, mixed_cap(pl)))
         {
-            fz_set_error("real length %lld has no radix decomposition", (long long)n0);
+            fz_set_error("real length %lld does not fit a mixed-radix tile", (long long)n0);
             return NULL;
         }
-        k->tpt = k->nstages ? fftz_threads_per_transform(pl->dtype, (int)n, k->nstages, k->radix) : 1;
+        p->off_tw = fz_mr_twiddles(&pl->blob, k);
+        if (p->off_tw < 0 || (packed && (p->off_rtw = fz_real_twiddles(&pl->blob, pl->dtype, n)) < 0)) return NULL;
+        snprintf(p->what, sizeof(p->what), "%s n=%lld x%lld", pl->direction ? "c2r" : "r2c", (long long)n0,
+                 (long long)k->ntf);
+        return p;
     }
+    const int maxthr = fftz_generic_max_threads();
+    k->variant = FFTZ_VAR_GENERIC;
+    k->nstages = n > 1 ? generic_radices(n, k->radix) : 0;
+    if (k->nstages < 0)
+    {
+        fz_set_error("real length %lld has no radix decomposition", (long long)n0);
+        return NULL;
+    }
+    k->tpt = k->nstages ? fftz_threads_per_transform(pl->dtype, (int)n, k->nstages, k->radix) : 1;
     if (k->tpt < 1 || k->tpt > maxthr)
     {
         fz_set_error("real length %lld exceeds the one-pass real kernel", (long long)n0);
@@ -856,6 +852,7 @@ static int real_pass_ok(const fz_plan *pl, int64_t n0)
     const int packed = (n0 % 2 == 0) && n0 >= 2;
     const int64_t n = packed ? n0 / 2 : n0;
     if (n == 1) return 1;
+    if (mixed_lines(pl)) return fz_mr_fits(pl->dtype, n, mixed_cap(pl));
     int32_t r[FFTZ_MAX_STAGES];
     int s = generic_radices(n, r);
     if (s < 0) return 0;

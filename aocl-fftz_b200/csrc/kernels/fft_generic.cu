@@ -9,7 +9,6 @@ const void *fftz_fast_f32_a(int log2n, int feat);
 const void *fftz_fast_f64_a(int log2n, int feat);
 const void *fftz_fast_f32_c(int log2n, int feat);
 const void *fftz_fast_f64_c(int log2n, int feat);
-const void *fftz_fast_real_kernel(int dtype, int log2n);
 
 static const void *fast_kernel(int dtype, int log2n, int variant) {
   int feat;
@@ -18,7 +17,6 @@ static const void *fast_kernel(int dtype, int log2n, int variant) {
     case FFTZ_VAR_FAST_TW4: feat = fftz::FEAT_TW4; break;
     case FFTZ_VAR_PIPE: feat = 16; break;
     case FFTZ_VAR_PIPE_TW4: feat = 16 | fftz::FEAT_TW4; break;
-    case FFTZ_VAR_FAST_REAL: return fftz_fast_real_kernel(dtype, log2n);
     default: return 0;
   }
   if (feat >= 16) return dtype == 0 ? fftz_fast_f32_c(log2n, feat) : fftz_fast_f64_c(log2n, feat);
@@ -131,7 +129,15 @@ int fftz_launch_pass(const fftz_pass_t *p, void *stream) {
     const int f = p->flags;
     const int feat = ((f & FFTZ_F_TW4) ? 1 : 0) | ((f & FFTZ_F_PRE_TAB) ? 2 : 0) | ((f & FFTZ_F_POST_TAB) ? 4 : 0) |
                      ((f & FFTZ_F_MID_TAB) ? 8 : 0);
-    fn = p->dtype == 0 ? fftz_mr_kernel_f32(feat, p->mr.big) : fftz_mr_kernel_f64(feat, p->mr.big);
+    const int real = p->in_kind == FFTZ_IN_REAL_PAIRS     ? 16
+                     : p->in_kind == FFTZ_IN_HERM_SEPARATE ? 32
+                     : p->in_kind == FFTZ_IN_REAL          ? 64
+                     : p->in_kind == FFTZ_IN_HERM_FULL     ? 128
+                                                           : 0;
+    if (real)
+      fn = p->dtype == 0 ? fftz_mr_real_kernel_f32(real, p->mr.big) : fftz_mr_real_kernel_f64(real, p->mr.big);
+    else
+      fn = p->dtype == 0 ? fftz_mr_kernel_f32(feat, p->mr.big) : fftz_mr_kernel_f64(feat, p->mr.big);
   } else {
     fn = fast_kernel(p->dtype, fftz::ct_log2(p->n), p->variant);
   }

@@ -32,7 +32,13 @@ namespace fftz {
 // waiting for instructions: 11 of 19 stall cycles an instruction in a 256-point
 // chirp pass.) TW4: output k of column c times W_{tw4_n}^{c k}. PRE / POST: bound
 // and table product on the load / store side. BLUE: two sweeps around mid_tab.
-enum { FEAT_MR_TW4 = 1, FEAT_MR_PRE = 2, FEAT_MR_POST = 4, FEAT_MR_BLUE = 8 };
+// R2C / C2R: real lines of 2 n points packed as n complex ones, with the Hermitian
+// recombination in the last stage's registers / the separation in the first
+// stage's. RFULL / CFULL: real lines of n points as n complex ones (odd lengths).
+enum {
+  FEAT_MR_TW4 = 1, FEAT_MR_PRE = 2, FEAT_MR_POST = 4, FEAT_MR_BLUE = 8,
+  FEAT_MR_R2C = 16, FEAT_MR_C2R = 32, FEAT_MR_RFULL = 64, FEAT_MR_CFULL = 128
+};
 
 // x / d by the host's m = ceil(2^32 / d) (0 for d = 1); exact while x d < 2^32
 __device__ __forceinline__ int mr_div(int x, uint32_t m) { return m ? (int)__umulhi((uint32_t)x, m) : x; }
@@ -96,8 +102,41 @@ __device__ __forceinline__ void mr_store(const fftz_pass_t &P, const MrTile<T> &
   typedef typename Cplx<T>::type T2;
   const MrLine L = t.out[p];
   const int64_t oes = P.oes;
+  if constexpr ((FEAT & FEAT_MR_C2R) != 0) {
+    // value k is the pair (out[2k], out[2k + 1]), conjugated
+    T *x = (T *)P.out + L.off;
+    if (oes == 1 && ((uintptr_t)x & (sizeof(T2) - 1)) == 0) {
+      T2 *g = (T2 *)x + K;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        v[r].y = -v[r].y;
+        g[r * nb] = v[r];
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        T *g = x + 2 * (int64_t)(K + r * nb) * oes;
+        g[0] = v[r].x;
+        g[oes] = -v[r].y;
+      }
+    }
+    return;
+  }
+  if constexpr ((FEAT & FEAT_MR_CFULL) != 0) {
+    T *g = (T *)P.out + L.off + (int64_t)K * oes;
+#pragma unroll
+    for (int r = 0; r < R; r++) g[(int64_t)r * nb * oes] = v[r].x;
+    return;
+  }
   T2 *g = (T2 *)P.out + L.off + (int64_t)K * oes;
   const int64_t st = (int64_t)nb * oes;
+  if constexpr ((FEAT & FEAT_MR_RFULL) != 0) {
+    const int half = P.n / 2;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (K + r * nb <= half) g[r * st] = v[r];
+    return;
+  }
   if constexpr ((FEAT & FEAT_MR_TW4) != 0) {
     const T2 w = mr_tw4<T2>(P)((uint32_t)L.col * (uint32_t)K);
     const T2 *stp = t.stp + p * 16;
@@ -129,6 +168,46 @@ __device__ __forceinline__ void mr_load(const fftz_pass_t &P, const MrTile<T> &t
   typedef typename Cplx<T>::type T2;
   const MrLine L = t.in[p];
   const int64_t ies = P.ies;
+  if constexpr ((FEAT & FEAT_MR_R2C) != 0) {
+    // value e is the pair (in[2e], in[2e + 1])
+    const T *x = (const T *)P.in + L.off;
+    if (ies == 1 && ((uintptr_t)x & (sizeof(T2) - 1)) == 0) {
+      const T2 *g = (const T2 *)x + rest;
+#pragma unroll
+      for (int r = 0; r < R; r++) v[r] = g[r * nb];
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const T *g = x + 2 * (int64_t)(rest + r * nb) * ies;
+        v[r].x = g[0];
+        v[r].y = g[ies];
+      }
+    }
+    return;
+  }
+  if constexpr ((FEAT & FEAT_MR_RFULL) != 0) {
+    const T *g = (const T *)P.in + L.off + (int64_t)rest * ies;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      v[r].x = g[(int64_t)r * nb * ies];
+      v[r].y = 0;
+    }
+    return;
+  }
+  if constexpr ((FEAT & FEAT_MR_CFULL) != 0) {
+    // bins above n / 2 are the conjugates of those below; the backward
+    // transform's conjugation included
+    const T2 *g = (const T2 *)P.in + L.off;
+    const int n = P.n;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int e = rest + r * nb;
+      const bool up = 2 * e > n;
+      v[r] = g[(int64_t)(up ? n - e : e) * ies];
+      if (!up) v[r].y = -v[r].y;
+    }
+    return;
+  }
   const T2 *g = (const T2 *)P.in + L.off + (int64_t)rest * ies;
   const int64_t st = (int64_t)nb * ies;
   const bool cj = (P.flags & FFTZ_F_CONJ_IN) != 0;
@@ -333,11 +412,191 @@ __device__ __forceinline__ void mr_dit_last(const fftz_pass_t &P, const MrTile<T
   }
 }
 
+// Real lines pair bin k with bin n - k. Butterfly A of a boundary stage (nb of
+// them, values A + r nb) mirrors butterfly nb - A, value r against value R - 1 -
+// r, so a thread that holds both recombines in registers. Item 0 holds the two
+// butterflies that mirror themselves: 0 (value r against R - r) and, for even nb,
+// nb / 2 (r against R - 1 - r).
+__device__ __forceinline__ int mr_mirror(int q, int nb) { return q ? nb - q : (nb & 1 ? 0 : nb >> 1); }
+
+// X_k and X_{n-k} from Z_k, Z_{n-k} and w = W_{2n}^k: with E = (Z_k + conj
+// Z_{n-k}) / 2, O = -i (Z_k - conj Z_{n-k}) / 2, X_k = E + w O, X_{n-k} = conj(E - w O).
+template <typename T2> __device__ __forceinline__ void mr_recombine(T2 &zk, T2 &zm, T2 w) {
+  typedef decltype(zk.x) T;
+  const T er = T(0.5) * (zk.x + zm.x), ei = T(0.5) * (zk.y - zm.y);
+  const T orr = T(0.5) * (zk.y + zm.y), oi = T(0.5) * (zm.x - zk.x);
+  const T tr = w.x * orr - w.y * oi, ti = w.x * oi + w.y * orr;
+  zk.x = er + tr;
+  zk.y = ei + ti;
+  zm.x = er - tr;
+  zm.y = ti - ei;
+}
+// 2 conj Z_k and 2 conj Z_{n-k} from X_k, X_{n-k}.
+template <typename T2> __device__ __forceinline__ void mr_separate(T2 &xk, T2 &xm, T2 w) {
+  typedef decltype(xk.x) T;
+  const T dr = xk.x - xm.x, di = xk.y + xm.y, s = xk.x + xm.x, d = xk.y - xm.y;
+  const T er = w.x * dr + w.y * di, ei = w.x * di - w.y * dr;  // conj(w) (X_k - conj X_{n-k})
+  xk.x = s - ei;
+  xk.y = -(d + er);
+  xm.x = s + ei;
+  xm.y = d - er;
+}
+
+// Bins of butterflies A (a) and B = mr_mirror(q, nb) (b) to HBM.
+template <typename T, int R>
+__device__ __forceinline__ void mr_store_half(const fftz_pass_t &P, const MrTile<T> &t, typename Cplx<T>::type (&a)[R],
+                                              typename Cplx<T>::type (&b)[R], int p, int q, int nb) {
+  typedef typename Cplx<T>::type T2;
+  const int64_t oes = P.oes;
+  const int n = P.n;
+  T2 *g = (T2 *)P.out + t.out[p].off;
+  const T2 *rtw = (const T2 *)P.rtw;
+  if (q) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int k = q + r * nb;
+      mr_recombine(a[r], b[R - 1 - r], __ldg(rtw + k));
+      g[k * oes] = a[r];
+      g[(n - k) * oes] = b[R - 1 - r];
+    }
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r <= R / 2; r++) {
+    const int k = r * nb;
+    T2 zk = a[r], zm = a[(R - r) % R];
+    mr_recombine(zk, zm, __ldg(rtw + k));
+    g[k * oes] = zk;
+    if (2 * r != R) g[(n - k) * oes] = zm;
+  }
+  if (nb & 1) return;
+#pragma unroll
+  for (int r = 0; r <= (R - 1) / 2; r++) {
+    const int k = (nb >> 1) + r * nb;
+    T2 zk = b[r], zm = b[R - 1 - r];
+    mr_recombine(zk, zm, __ldg(rtw + k));
+    g[k * oes] = zk;
+    if (r != R - 1 - r) g[(n - k) * oes] = zm;
+  }
+}
+
+// The same two butterflies' inputs from the half spectrum in HBM.
+template <typename T, int R>
+__device__ __forceinline__ void mr_load_half(const fftz_pass_t &P, const MrTile<T> &t, typename Cplx<T>::type (&a)[R],
+                                             typename Cplx<T>::type (&b)[R], int p, int q, int nb) {
+  typedef typename Cplx<T>::type T2;
+  const int64_t ies = P.ies;
+  const int n = P.n;
+  const T2 *g = (const T2 *)P.in + t.in[p].off;
+  const T2 *rtw = (const T2 *)P.rtw;
+  if (q) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int k = q + r * nb;
+      a[r] = g[k * ies];
+      b[R - 1 - r] = g[(n - k) * ies];
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) mr_separate(a[r], b[R - 1 - r], __ldg(rtw + q + r * nb));
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r <= R / 2; r++) {
+    const int k = r * nb;
+    T2 xk = g[k * ies], xm = g[(n - k) * ies];
+    mr_separate(xk, xm, __ldg(rtw + k));
+    a[r] = xk;
+    if (r > 0 && 2 * r != R) a[R - r] = xm;
+  }
+  if (nb & 1) {
+#pragma unroll
+    for (int r = 0; r < R; r++) b[r] = zero2<T2>();
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r <= (R - 1) / 2; r++) {
+    const int k = (nb >> 1) + r * nb;
+    T2 xk = g[k * ies], xm = g[(n - k) * ies];
+    mr_separate(xk, xm, __ldg(rtw + k));
+    b[r] = xk;
+    if (r != R - 1 - r) b[R - 1 - r] = xm;
+  }
+}
+
+// Last stage of a packed r2c line: shared memory -> half spectrum in HBM.
+template <typename T, int R>
+__device__ __forceinline__ void mr_last_r2c(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
+  typedef typename Cplx<T>::type T2;
+  const int nb = st.nb, S = P.nstages, S0 = P.mr.st[0].m + P.mr.pad, sst = P.sstride;
+  const MrItems it(P, P.out_mode, (nb + 1) >> 1, P.mr.mg_pair, t.nl);
+  for (int i = threadIdx.x; i < it.total; i += blockDim.x) {
+    int p, q;
+    it.at(i, p, q);
+    if (p >= t.nl) continue;
+    const T2 *da = t.sd + p * sst + mr_slot(P, S, S0, q), *db = t.sd + p * sst + mr_slot(P, S, S0, mr_mirror(q, nb));
+    T2 a[R], b[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      a[r] = da[r];
+      b[r] = db[r];
+    }
+    Dft<R>::template apply<T, T2>(a);
+    Dft<R>::template apply<T, T2>(b);
+    mr_store_half<T, R>(P, t, a, b, p, q, nb);
+  }
+}
+
+// Stage 0 of a packed c2r line: half spectrum in HBM -> shared memory.
+template <typename T, int R>
+__device__ __forceinline__ void mr_first_c2r(const fftz_pass_t &P, const MrTile<T> &t, const fftz_mr_stage_t &st) {
+  typedef typename Cplx<T>::type T2;
+  const int M = st.m, S0 = M + P.mr.pad, sst = P.sstride;
+  const T2 *tw = (const T2 *)P.tw + st.tw, *sh = t.tw + st.tw;
+  const MrItems it(P, P.in_mode, (M + 1) >> 1, P.mr.mg_pair, t.nl);
+  for (int i = threadIdx.x; i < it.total; i += blockDim.x) {
+    int p, q;
+    it.at(i, p, q);
+    if (p >= t.nl) continue;
+    const int B = mr_mirror(q, M);
+    T2 a[R], b[R];
+    mr_load_half<T, R>(P, t, a, b, p, q, M);
+    T2 *d = t.sd + p * sst;
+    Dft<R>::template apply<T, T2>(a);
+    mr_twiddle<T, R>(tw, sh, t.has_tw, a, M, q);
+#pragma unroll
+    for (int r = 0; r < R; r++) d[q + r * S0] = a[r];
+    if (B == q) continue;  // odd M: butterfly 0 alone
+    Dft<R>::template apply<T, T2>(b);
+    mr_twiddle<T, R>(tw, sh, t.has_tw, b, M, B);
+#pragma unroll
+    for (int r = 0; r < R; r++) d[B + r * S0] = b[r];
+  }
+}
+
+// Packed lines of one stage (n <= 16): a thread a line.
+template <typename T, int R, int FEAT>
+__device__ __forceinline__ void mr_single_real(const fftz_pass_t &P, const MrTile<T> &t) {
+  typedef typename Cplx<T>::type T2;
+  for (int p = threadIdx.x; p < t.nl; p += blockDim.x) {
+    T2 a[R], b[R];
+    if constexpr ((FEAT & FEAT_MR_C2R) != 0)
+      mr_load_half<T, R>(P, t, a, b, p, 0, 1);
+    else
+      mr_load<T, R, FEAT>(P, t, a, p, 0, 1);
+    Dft<R>::template apply<T, T2>(a);
+    if constexpr ((FEAT & FEAT_MR_C2R) != 0)
+      mr_store<T, R, FEAT>(P, t, a, p, 0, 1);
+    else
+      mr_store_half<T, R>(P, t, a, b, p, 0, 1);
+  }
+}
+
 // Radix sets: MR_SMOOTH without 11 and 13 (whose butterflies hold more live
-// values) and MR_ALL.
-enum { MR_SMOOTH = 0, MR_ALL = 1 };
+// values), MR_ALL, and those of the stage that holds mirrored butterflies (two
+// of them in a thread: at most 8, or 11 and 13 where a line has nothing else).
+enum { MR_SMOOTH = 0, MR_ALL = 1, MR_PAIR = 2 };
 __host__ __device__ constexpr bool mr_has(int set, int R) {
-  return set == MR_ALL || (R != 11 && R != 13);
+  return set == MR_ALL || (set == MR_PAIR ? R <= 8 || R == 11 || R == 13 : R != 11 && R != 13);
 }
 #define FZ_MR_CASE(SET, R_, CALL) \
   case R_:                        \
@@ -387,13 +646,20 @@ __device__ __forceinline__ void mr_tile(const fftz_pass_t &P, int64_t blk, unsig
     if (S == 1) __syncthreads();
   }
   if (S == 1) {
-    if constexpr ((FEAT & FEAT_MR_BLUE) == 0) {
+    if constexpr ((FEAT & (FEAT_MR_R2C | FEAT_MR_C2R)) != 0) {
+      if (P.n == 1) mr_single_real<T, 1, FEAT>(P, t);
+      FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_single_real<T, R, FEAT>(P, t)));
+    } else if constexpr ((FEAT & FEAT_MR_BLUE) == 0) {
       if (P.n == 1) mr_single<T, 1, FEAT>(P, t);
       FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_single<T, R, FEAT>(P, t)));
     }
     return;
   }
-  FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_first<T, R, FEAT>(P, t, P.mr.st[0])));
+  if constexpr ((FEAT & FEAT_MR_C2R) != 0) {
+    FZ_MR_SWITCH(P.mr.st[0].r, MR_PAIR, (mr_first_c2r<T, R>(P, t, P.mr.st[0])));
+  } else {
+    FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_first<T, R, FEAT>(P, t, P.mr.st[0])));
+  }
   __syncthreads();
   for (int s = 1; s < S - 1; s++) {
     FZ_MR_SWITCH(P.mr.st[s].r, SET, (mr_mid<T, R, false>(P, t, P.mr.st[s])));
@@ -407,6 +673,8 @@ __device__ __forceinline__ void mr_tile(const fftz_pass_t &P, int64_t blk, unsig
       __syncthreads();
     }
     FZ_MR_SWITCH(P.mr.st[0].r, SET, (mr_dit_last<T, R, FEAT>(P, t, P.mr.st[0])));
+  } else if constexpr ((FEAT & FEAT_MR_R2C) != 0) {
+    FZ_MR_SWITCH(P.mr.st[S - 1].r, MR_PAIR, (mr_last_r2c<T, R>(P, t, P.mr.st[S - 1])));
   } else {
     FZ_MR_SWITCH(P.mr.st[S - 1].r, SET, (mr_last<T, R, FEAT>(P, t, P.mr.st[S - 1])));
   }

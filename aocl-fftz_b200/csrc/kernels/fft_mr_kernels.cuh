@@ -21,6 +21,11 @@ template <typename T, bool BIG> __host__ __device__ constexpr int mr_lb() {
 // peak -- issue and the shared-memory pipe together, not HBM, bound it. Lines per
 // CTA at n = 1000, at 94 instructions: 2 166, 3 136, 4 146, 5 135 (fz_mr_shape's
 // choice), 6 142 us.
+// Real lines, against the kernels that loaded, transformed and recombined in
+// separate sweeps of shared memory (r2c / c2r us, before -> after): 2048 x 8192
+// float 56 / 54 -> 41 / 42, 512 x 262144 double 730 / 642 -> 521 / 460, 1024 x 65536
+// double 329 / 351 -> 247 / 273, 256 x 65536 float 133 / 133 -> 42 / 40, 1000 x 16000
+// float 203 / 204 -> 43 / 41, 44100 x 200 float (four passes before) 311 / 309 -> 51 / 47.
 template <typename T, int FEAT, bool BIG>
 __global__ void __launch_bounds__(mr_lb<T, BIG>()) fft_mr_kernel(const __grid_constant__ fftz_pass_t P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -30,6 +35,15 @@ __global__ void __launch_bounds__(mr_lb<T, BIG>()) fft_mr_kernel(const __grid_co
 }  // namespace fftz
 
 /* The mixed-radix kernel for a feature set (FEAT_MR_*), or NULL. */
+#ifdef FZ_MR_REAL
+extern "C" const void *FZ_MR_GET(int feat, int big) {
+  using namespace fftz;
+#define FZ_MR_K(F) \
+  case (F): return big ? (const void *)&fft_mr_kernel<FZ_MR_T, (F), true> : (const void *)&fft_mr_kernel<FZ_MR_T, (F), false>;
+  switch (feat) { FZ_MR_K(FEAT_MR_R2C) FZ_MR_K(FEAT_MR_C2R) FZ_MR_K(FEAT_MR_RFULL) FZ_MR_K(FEAT_MR_CFULL) }
+  return 0;
+}
+#else
 extern "C" const void *FZ_MR_GET(int feat, int big) {
   using namespace fftz;
 #define FZ_MR_K(F, BIG) \
@@ -45,3 +59,4 @@ extern "C" const void *FZ_MR_GET(int feat, int big) {
     }
   return 0;
 }
+#endif

@@ -49,7 +49,6 @@ enum fftz_out_kind {
 #define FFTZ_VAR_PIPE 6      /* persistent, cp.async double-buffered, complex in/out */
 #define FFTZ_VAR_PIPE_TW4 7  /* as PIPE with the four-step twiddle epilogue         */
 #define FFTZ_VAR_TC 8        /* 4096-point rows as two radix-64 tensor-core GEMM stages */
-#define FFTZ_VAR_FAST_REAL 9 /* packed real line: generic load/store phases, compile-time stages */
 #define FFTZ_VAR_MR 11       /* runtime radix list (2..16) in place in one shared-memory buffer */
 #define FFTZ_MR_STAGES 8     /* most stages of a mixed-radix line */
 
@@ -85,7 +84,7 @@ typedef struct fftz_mr
     int32_t pad;     /* slots between digit-0 blocks beyond M_0 */
     uint32_t mg_tpc; /* d = tpc */
     int32_t big;     /* a radix of 11 or 13 among them */
-    int32_t pad_;
+    uint32_t mg_pair; /* real lines: d = items of the stage with mirrored butterflies, (nb + 1) / 2 */
 } fftz_mr_t;
 
 typedef struct fftz_pass
@@ -229,9 +228,6 @@ int fftz_fast_tpt(int n);
 int fftz_fast_max_n(int dtype);
 /* Radix list used by the compile-time kernel for length n (returns stages). */
 int fftz_fast_radices(int n, int32_t *radix);
-/* compile-time packed real-line kernel for complex length 2^log2n (NULL if
- * not instantiated) */
-const void *fftz_fast_real_kernel(int dtype, int log2n);
 /* Threads per CTA the generic kernel may use; the persistent kernels' bound. */
 int fftz_generic_max_threads(void);
 int fftz_pipe_max_threads(int n);
@@ -260,6 +256,9 @@ int64_t fftz_smem_limit(void);
  * radices 11 and 13), or NULL. */
 const void *fftz_mr_kernel_f32(int feat, int big);
 const void *fftz_mr_kernel_f64(int feat, int big);
+/* The same for real lines: 16 / 32 packed r2c / c2r, 64 / 128 unpacked (odd). */
+const void *fftz_mr_real_kernel_f32(int feat, int big);
+const void *fftz_mr_real_kernel_f64(int feat, int big);
 /* Largest block of those kernels. */
 int fftz_mr_max_threads(int dtype, int big);
 

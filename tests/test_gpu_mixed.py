@@ -1,11 +1,14 @@
 """GPU parity of the mixed-radix line kernel (csrc/kernels/fft_mr.cuh) against the
 FP64 oracle at the edges of its shapes: one, two and more stages, every
 composite radix, a last CTA that is not full, the longest line of each dtype,
-row and column lane maps, non-unit strides, in place, four-step passes.
+row and column lane maps, non-unit strides, in place, four-step passes, real lines
+with mirrored butterflies (odd and even butterfly counts, one stage, 11 and 13
+alone) and unpacked odd ones.
 Bound: rel-L2 <= 4 log2(n) eps of the working dtype (oracle.tol)."""
 import pytest
 
 from test_gpu_c2c import check_c2c
+from test_gpu_real import check_real
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +41,17 @@ def test_strides_and_mixed_maps(dtype):
 @pytest.mark.parametrize("dtype,n,b", [("f32", 250047, 2), ("f64", 120000, 1), ("f32", 30030, 3)])
 def test_four_step(dtype, n, b):
     check_c2c(dtype, [(n, 1, 1)], [(b, n, n)], direction=b & 1, seed=5, compare_ref=False)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("shape,batch", [((2,), 5), ((3,), 300), ((6,), 70), ((13,), 9), ((32,), 131), ((36,), 3), ((50,), 40),
+                                         ((98,), 7), ((242,), 5), ((286,), 3), ((338,), 2), ((441,), 9), ((480,), 33),
+                                         ((2048,), 5), ((14406,), 2), ((6, 9, 10), 2), ((17, 24), 3)])
+def test_real_lines(shape, batch, dtype):
+    check_real(dtype, shape, batch=batch, compare_ref=False)
+    check_real(dtype, shape, batch=1, inplace=len(shape) > 1, compare_ref=False)
+
+
+def test_longest_real_lines():
+    check_real("f32", (56000,), batch=2, compare_ref=False)
+    check_real("f64", (28800,), batch=1, compare_ref=False)

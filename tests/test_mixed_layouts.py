@@ -21,7 +21,7 @@ class Stage(C.Structure):
 
 
 class Mr(C.Structure):
-    _fields_ = [("st", Stage * MRS), ("pad", I32), ("mg_tpc", U32), ("big", I32), ("pad_", I32)]
+    _fields_ = [("st", Stage * MRS), ("pad", I32), ("mg_tpc", U32), ("big", I32), ("mg_pair", U32)]
 
 
 class Pass(C.Structure):
@@ -38,11 +38,11 @@ class Pass(C.Structure):
                 ("ind_out", VP), ("mr", Mr), ("threads", I32), ("ntw", I32), ("pad2_", I32 * 2)]
 
 
-def shape(n, dtype=0, col=False, two=False, tw4=False, ntf=100000, tpc=0, threads=0, cap=0):
+def shape(n, dtype=0, col=False, two=False, tw4=False, ntf=100000, tpc=0, threads=0, cap=0, in_kind=0):
     lib = aoclfftz_b200.load()
     lib.fftz_pass_smem_bytes.restype = I64
     lib.fftz_smem_limit.restype = I64
-    p = Pass(n=n, dtype=dtype, ntf=ntf, in_mode=int(col), out_mode=int(col), nbdims=1,
+    p = Pass(n=n, dtype=dtype, ntf=ntf, in_kind=in_kind, in_mode=int(col), out_mode=int(col), nbdims=1,
              flags=(F_MID if two else 0) | (F_TW4 if tw4 else 0))
     assert lib.fz_mr_shape(C.byref(p), tpc, threads, I64(cap or lib.fftz_smem_limit())) == 0
     assert p.variant == VAR_MR and 1 <= p.tpc <= ntf and 1 <= p.threads <= lib.fftz_mr_max_threads(dtype, p.mr.big)
@@ -194,3 +194,44 @@ def test_executor_tiles_keep_their_block_and_share(n, dtype, ntf, least):
     p = shape(n, dtype, ntf=ntf, threads=256, cap=cap)
     assert p.threads == 256 and lib.fftz_pass_smem_bytes(C.byref(p)) <= cap
     assert least <= p.tpc <= ntf
+
+
+IN_PAIRS, IN_SEPARATE = 1, 4  # fftz_in_kind
+
+
+def pair_items(p, s):
+    """(line, butterfly, mirrored butterfly) of every item of the stage that holds mirrored butterflies."""
+    nb = p.n // p.radix[s]
+    items_ = (nb + 1) // 2
+    i = np.arange(p.tpc * items_)
+    if p.in_mode:
+        q = exact_div(i, p.mr.mg_tpc, p.tpc)
+        line = i - q * p.tpc
+    else:
+        line = exact_div(i, p.mr.mg_pair, items_)
+        q = i - line * items_
+    return line, q, np.where(q > 0, nb - q, 0 if nb & 1 else nb // 2)
+
+
+@pytest.mark.parametrize("col", [False, True])
+@pytest.mark.parametrize("n", [2, 16, 18, 25, 77, 121, 143, 240, 256, 1000, 1024, 2401, 22050, 28000])
+def test_mirrored_butterflies_cover_each_bin_once(n, col):
+    """r2c / c2r: the paired stage's items hold every butterfly of every line once, and bin k of one is bin n - k of the
+    other; the stage's radix is one its two-butterfly form exists for."""
+    for kind in (IN_PAIRS, IN_SEPARATE):
+        p = shape(n, col=col, in_kind=kind)
+        if p.nstages == 1:
+            assert n <= 16
+            continue
+        s = p.nstages - 1 if kind == IN_PAIRS else 0
+        R, nb = p.radix[s], n // p.radix[s]
+        assert R <= 8 or R in (11, 13)
+        line, a, b = pair_items(p, s)
+        own = np.concatenate([line * nb + a, (line * nb + b)[a != b]])
+        assert np.array_equal(np.sort(own), np.arange(p.tpc * nb))
+        r = np.arange(R)[:, None]
+        ordinary = a > 0
+        assert np.all((a + r * nb + b + (R - 1 - r) * nb)[:, ordinary] == n)
+        x = np.random.default_rng(n).standard_normal((p.tpc, n)) + 0j
+        if kind == IN_PAIRS:
+            assert np.linalg.norm(simulate(p, x) - np.fft.fft(x, axis=1)) <= 1e-13 * np.linalg.norm(x) * np.sqrt(n)
