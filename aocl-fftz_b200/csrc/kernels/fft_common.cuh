@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "codelets.cuh"
+#include "fft_launch.cuh"
 #include "fftz_kernels.h"
 
 namespace fftz {

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fft_launch.cuh"
 #include "fftz_kernels.h"
 
 namespace fftz {
@@ -29,6 +30,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) elem_kernel(const __grid_constant__ fftz_elem_t E) {
   typedef typename C2T<T>::type T2;
   const int64_t total = E.nlines * E.nout;
+  pdl_begin();
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
     const int64_t line = g / E.nout;
     const int64_t e = g - line * E.nout;
@@ -118,5 +120,5 @@ extern "C" int fftz_launch_elem(const fftz_elem_t *e, void *stream) {
   if (blocks > 148 * 64) blocks = 148 * 64;
   void *args[1] = {(void *)e};
   const void *fn = e->dtype == 0 ? (const void *)&fftz::elem_kernel<float> : (const void *)&fftz::elem_kernel<double>;
-  return (int)cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(256), args, 0, (cudaStream_t)stream);
+  return fz_launch_pdl(fn, dim3((unsigned)blocks), dim3(256), args, 0, stream);
 }

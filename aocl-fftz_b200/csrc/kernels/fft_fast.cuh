@@ -287,6 +287,7 @@ __device__ __forceinline__ void fast_tile(const fftz_pass_t &P, int64_t tf0, uns
     const T2 *g = (const T2 *)P.tw;
     for (int i = threadIdx.x; i < ct_tw_total(N); i += blockDim.x) twb[i] = __ldg(g + i);
   }
+  pdl_begin();
   __syncthreads();
   FastStages<T, N, 0, ct_nstages(N), 0, 1, FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
 }
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(ct_pipe_lb(N), 1) fft_pipe_kernel(const __grid
   int64_t *offs = (int64_t *)(slot0 + 2 * slot_elems);  // 3 rotating sets of {in, out, col}
   const int64_t ntiles = (P.ntf + P.tpc - 1) / P.tpc;
   int64_t tile = blockIdx.x;
+  pdl_begin();
   if (tile >= ntiles) return;
 #define FZ_OFF(bf, a) (offs + (size_t)((bf)*3 + (a)) * P.tpc)
   tile_offsets(P, tile * P.tpc, FZ_OFF(0, 0), FZ_OFF(0, 1), FZ_OFF(0, 2));

@@ -178,7 +178,7 @@ int fftz_launch_pass(const fftz_pass_t *p, void *stream) {
     grid.x = (unsigned)(nblk < cap ? nblk : cap);
   }
   void *args[1] = {(void *)p};
-  return (int)cudaLaunchKernel(fn, grid, block, args, smem, (cudaStream_t)stream);
+  return fz_launch_pdl(fn, grid, block, args, smem, stream);
 }
 
 }  // extern "C"

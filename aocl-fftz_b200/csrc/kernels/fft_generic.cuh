@@ -314,6 +314,7 @@ __device__ __forceinline__ void generic_tile(const fftz_pass_t &P, int64_t blk, 
   int64_t *s_col = s_out + P.tpc;
   const int64_t tf0 = blk * P.tpc;
   for (int p = threadIdx.x; p < P.tpc; p += blockDim.x) batch_offsets(P, tf0 + p, s_in + p, s_out + p, s_col + p);
+  pdl_begin();
   __syncthreads();
 
   const int nsweeps = (P.flags & FFTZ_F_MID_TAB) ? 2 : 1;

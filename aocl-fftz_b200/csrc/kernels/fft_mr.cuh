@@ -640,6 +640,7 @@ __device__ __forceinline__ void mr_tile(const fftz_pass_t &P, int64_t blk, unsig
     batch_offsets(P, blk * tpc + p, &in[p].off, &out[p].off, &in[p].col);
     out[p].col = in[p].col;
   }
+  pdl_begin();
   __syncthreads();
   if constexpr ((FEAT & FEAT_MR_TW4) != 0) {
     mr_steps<T>(P, t, (FEAT & FEAT_MR_BLUE) ? P.mr.st[0].r : P.mr.st[S - 1].r);

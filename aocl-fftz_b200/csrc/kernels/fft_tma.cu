@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(ct_lb<T>()) fft_tma_kernel(const __grid_consta
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  pdl_begin();
   __syncthreads();
   if (threadIdx.x == 0) {
     mbar_expect_tx(&bar, (unsigned)(N * tpc * sizeof(T2) + P.test_tx_short));
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(ct_lb<T>(), 1) fft_tma_pipe_kernel(const __gri
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  pdl_begin();
   __syncthreads();
   int64_t tile = blockIdx.x;
   if (threadIdx.x == 0 && tile < ntiles) issue(tile);
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(ct_lb<T>()) fft_tma_stream_kernel(const __grid
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  pdl_begin();
   __syncthreads();
   int64_t tile = blockIdx.x;
   if (threadIdx.x == 0) {
@@ -525,6 +528,7 @@ __global__ void __launch_bounds__(ct_lb<T>(), 1) fft_tma_rr_kernel(const __grid_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  pdl_begin();
   __syncthreads();
   int64_t tile = blockIdx.x;
   if (threadIdx.x == 0 && tile < ntiles) issue(tile);
@@ -763,6 +767,7 @@ __global__ void __launch_bounds__(1024, 1) fft_tma_split_kernel(const __grid_con
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (XM == 2) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  pdl_begin();
   __syncthreads();
   if (XM == 2) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   // this warp's stash columns (round-1 reader warps, four per lane quarter)
@@ -1049,7 +1054,7 @@ int launch_stream(const fftz_pass_t *p, void *stream) {
   const int64_t cap = (int64_t)occ * (nsm[dev] > 0 ? nsm[dev] : 148);
   const dim3 grid((unsigned)(ntiles < cap ? ntiles : cap));
   void *args[2] = {(void *)p, (void *)&ntiles};
-  return (int)cudaLaunchKernel(fn, grid, block, args, smem, (cudaStream_t)stream);
+  return fz_launch_pdl(fn, grid, block, args, smem, stream);
 }
 
 template <int XM> const void *split_pick(int tw4, int mode, int omode) {
@@ -1168,7 +1173,7 @@ int launch_split(const fftz_pass_t *p, void *stream) {
   const int64_t cap = nsm[dev] > 0 ? nsm[dev] : 148;
   const dim3 grid((unsigned)(ntiles < cap ? ntiles : cap)), block(1024);
   void *args[3] = {(void *)p, (void *)&map, (void *)&ntiles};
-  return (int)cudaLaunchKernel(fn, grid, block, args, smem, (cudaStream_t)stream);
+  return fz_launch_pdl(fn, grid, block, args, smem, stream);
 }
 
 const void *tma_kernel(int dtype, int n, int tw4, int mode) {
@@ -1286,7 +1291,7 @@ int fftz_launch_pass_tma(const fftz_pass_t *p, void *stream) {
     grid.x = (unsigned)(ntiles < cap ? ntiles : cap);
   }
   void *args[3] = {(void *)p, (void *)&map, (void *)&ntiles};
-  return (int)cudaLaunchKernel(fn, grid, block, args, smem, (cudaStream_t)stream);
+  return fz_launch_pdl(fn, grid, block, args, smem, stream);
 }
 
 /* 1 if some TMA tile gave up waiting for its copies since the last call (and
