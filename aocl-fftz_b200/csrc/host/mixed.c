@@ -91,13 +91,17 @@ static int64_t mr_lines(const fftz_pass_t *k, int64_t cap)
     return cap / per;
 }
 
-/* 1 if a line of n points fits cap bytes of shared memory as a mixed-radix tile. */
+/* 1 if a line of n points fits cap bytes of shared memory as a mixed-radix tile
+ * (a product of the primes up to 13 that fits never needs more stages than there
+ * are: 5^6 takes six). */
 int fz_mr_fits(int dtype, int64_t n, int64_t cap)
 {
-    int32_t r[FFTZ_MR_STAGES];
     const int64_t esz = dtype == 0 ? 8 : 16;
     if (n < 1 || (n + 1 + 16) * esz + 32 > cap) return 0;
-    return fz_mr_radices(n, 1, 0, r, NULL) > 0;
+    static const int pr[] = {2, 3, 5, 7, 11, 13};
+    for (int i = 0; i < 6; i++)
+        while (n % pr[i] == 0) n /= pr[i];
+    return n == 1;
 }
 
 /* the smallest product of 2, 3, 5 and 7 that is at least n */
@@ -163,11 +167,11 @@ int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t
 
 /* Slot of item i (of one line, or of tpc lines when col) of stage s; first /
  * last are the maps of the HBM-side stages. */
-static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)
+static int mr_addr(const fftz_pass_t *k, int s, int i, int col)
 {
     const int S = k->nstages;
-    const int64_t R = k->radix[s], M = k->mr.st[s].m, nb = k->n / R;
-    int64_t p, x;
+    const int R = k->radix[s], M = k->mr.st[s].m, nb = k->n / R;
+    int p, x;
     if (col)
     {
         x = i / k->tpc;
@@ -178,11 +182,11 @@ static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)
         p = i / nb;
         x = i % nb;
     }
-    const int64_t base = p * k->sstride;
+    const int base = p * k->sstride;
     if (s == 0) return base + x;
     if (s == S - 1)
     {
-        int64_t o = 0;
+        int o = 0;
         for (int j = 0; j < S - 1; j++)
         {
             o += (x % k->radix[j]) * (k->mr.st[j].m + (j == 0 ? k->mr.pad : 0));
@@ -190,28 +194,29 @@ static int64_t mr_addr(const fftz_pass_t *k, int s, int64_t i, int col)
         }
         return base + o;
     }
-    const int64_t b = x / M;
-    int64_t B = 1;
+    const int b = x / M;
+    int B = 1;
     for (int j = 1; j < s; j++) B *= k->radix[j];
     return base + x + b * M * (R - 1) + (b / B) * k->mr.pad;
 }
 
 /* Shared-memory wavefronts per lane group (16 float or 8 double slots span all
- * banks) over the first groups of every stage, for the pad and stride in k. */
-static int mr_conflicts(const fftz_pass_t *k)
+ * banks) over the first groups of every stage, for the pad and stride in k; stops
+ * counting at most. */
+static int mr_conflicts(const fftz_pass_t *k, int most)
 {
     const int W = k->dtype == 0 ? 16 : 8;
     int tot = 0;
     for (int s = 0; s < k->nstages; s++)
     {
         const int col = (s == 0 && k->in_mode == 1) || (s == k->nstages - 1 && k->out_mode == 1);
-        const int64_t items = (int64_t)k->tpc * (k->n / k->radix[s]);
-        for (int g = 0; g < 8 && (int64_t)g * W < items; g++)
+        const int items = k->tpc * (k->n / k->radix[s]);
+        for (int g = 0; g < 8 && g * W < items && tot < most; g++)
         {
             int cnt[16] = {0}, worst = 0;
-            for (int l = 0; l < W && (int64_t)g * W + l < items; l++)
+            for (int l = 0; l < W && g * W + l < items; l++)
             {
-                int c = ++cnt[mr_addr(k, s, (int64_t)g * W + l, col) % W];
+                int c = ++cnt[mr_addr(k, s, g * W + l, col) % W];
                 if (c > worst) worst = c;
             }
             tot += worst * k->radix[s] * (s > 0 && s < k->nstages - 1 ? 2 : 1);
@@ -279,7 +284,7 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     if (most > k->ntf) most = k->ntf;
     if (most > (threads ? FZ_RG_LINES : 256)) most = threads ? FZ_RG_LINES : 256;
     /* lines per CTA: about 4096 float / 2048 double points of row lines; whole
-     * 64-byte segments (8 float / 4 double neighbours) of column lines. Of equal
+     * segments of neighbouring lines where lanes run across them. Of equal
  * choices the smaller tile (512-point double r2c rows x 262144: 2 lines 588, 4 521,
  * 6 591, 8 546 us). The
      * executor's tiles, which wait on memory at their ends, are larger (measured on
@@ -292,9 +297,14 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
         lo = hi = want_tpc < most ? want_tpc : most;
     else if (colmap)
     {
-        const int64_t seg = k->dtype == 0 ? 8 : 4;
+        /* 8 neighbours (double lines above 440 points, whose 8 would leave fewer than
+         * four CTAs an SM: 4), doubled while a tile stays small. Measured on B200, lines a tile 4 / 6 / 8 / 12 / 16: 120000 x 64 double
+         * (375 and 320 points) 178 / 160 / 154 / 191 / 183 us, 60000 x 64 float (250 and
+         * 240) 56 / 51 / 49 / 58 / 54, 1080-point float columns 66 / 56 / 51 / 56 / 51;
+         * 65521 x 32 double (512-point rows of its middle pass) 161 with 4, 182 with 8 */
+        const int64_t seg = k->dtype == 0 || k->n <= 440 ? 8 : 4, room = threads ? pts : pts / 2;
         lo = hi = seg < most ? seg : most;
-        while (hi * 2 <= most && hi * 2 * k->n <= pts && hi < 32) lo = hi = hi * 2;
+        while (hi * 2 <= most && hi * 2 * k->n <= room && hi < 32) lo = hi = hi * 2;
         /* the executor's block is fixed: a few more columns where they fill it better */
         if (threads) hi = lo + lo / 2 <= most ? lo + lo / 2 : most;
     }
@@ -347,7 +357,7 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     {
         mr_stride(k, colmap, pad);
         if (pad > 0 && fftz_pass_smem_bytes(k) > cap) break;
-        const int c = mr_conflicts(k);
+        const int c = mr_conflicts(k, bp < 0 ? 0x7fffffff : bc);
         if (bp < 0 || c < bc)
         {
             bp = pad;
