@@ -235,6 +235,15 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
     const int fast = !generic_only(pl) && is_pow2(n) && n >= 2 && n <= fast_max_n(pl) && !mixed &&
                      !ragged_mode(pl);
     int maxthr;
+    /* short rows: the compile-time kernel's threads hold 16 points each, here a
+     * whole line or half of one, and read it in steps of the line's length. The
+     * mixed-radix tile's two short stages read whole sectors (measured on B200,
+     * compile-time / mixed-radix us: 16 x 10^6 float 140 / 63, 8 x 500000 23 / 21, 32 x
+     * 200000 37 / 25, 64 x 100000 30 / 23, 16 x 500000 double 87 / 53, 8 x 500000 46 / 31;
+     * 4 x 500000 float 14 / 16, 256 x 65536 50 / 52) */
+    if (fast && pl->hints.kernel_family == 0 && k->in_mode == 0 && k->out_mode == 0 && n >= 8 && n <= 64 &&
+        !(flags & FFTZ_F_TW4))
+        goto generic;
     if (fast)
     {
         k->nstages = fftz_fast_radices((int)n, k->radix);

@@ -2,17 +2,19 @@
 // (programmatic dependent launch). Every kernel launched through fz_launch_pdl
 // calls pdl_begin before its first access to memory that earlier work of the
 // stream may write or read (its inputs, outputs and scratch; tables are written
-// at setup): it lets the next such kernel be brought onto the device once this
-// one's last CTA has started, then waits until everything before it in the stream
-// is complete and visible. What overlaps is the launch itself, the first CTAs'
-// set-up and the first instruction fetches.
+// at setup): it waits until everything before it in the stream is complete and
+// visible, then lets the next such kernel be brought onto the device once this
+// one's last CTA has come this far. What overlaps is the launch itself, the first
+// CTAs' set-up and the first instruction fetches: two dependent 512-point launches
+// took 12.28 us a pair, 6.33 with the next kernel let in before the wait, 6.05 after
+// it; 4096 x 1024 float forward and backward 43.9 -> 38.8.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace fftz {
 __device__ __forceinline__ void pdl_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 }  // namespace fftz
 

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", ["f32", "f64"])
-@pytest.mark.parametrize("n,b", [(6, 700), (9, 1), (13, 33), (14, 129), (15, 7), (18, 65), (26, 50), (60, 301), (100, 41),
+@pytest.mark.parametrize("n,b", [(4, 5), (6, 700), (8, 1001), (9, 1), (10, 300), (16, 4097), (32, 77), (64, 3), (13, 33), (14, 129), (15, 7), (18, 65), (26, 50), (60, 301), (100, 41),
                                  (143, 9), (360, 14), (1000, 11), (1080, 3), (2187, 5), (11011, 2), (14400, 2)])
 def test_rows(n, b, dtype):
     check_c2c(dtype, [(n, 1, 1)], [(b, n, n)], direction=n & 1, seed=n, compare_ref=False)
