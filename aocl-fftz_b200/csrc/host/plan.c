@@ -29,13 +29,6 @@
 
 static int is_pow2(int64_t n) { return n > 0 && (n & (n - 1)) == 0; }
 
-static int ilog2i(int64_t n)
-{
-    int k = 0;
-    while (((int64_t)1 << k) < n) k++;
-    return k;
-}
-
 static int smooth13(int64_t n)
 {
     static const int64_t pr[] = {2, 3, 5, 7, 11, 13};
