@@ -238,6 +238,14 @@ static void mr_stride(fftz_pass_t *k, int colmap, int pad)
     k->sstride = (int32_t)s;
 }
 
+/* shared memory of a tile of c lines, without padding */
+static int64_t mr_tile_bytes(fftz_pass_t *k, int colmap, int64_t c)
+{
+    k->tpc = (int32_t)c;
+    mr_stride(k, colmap, 0);
+    return fftz_pass_smem_bytes(k);
+}
+
 /* Fills k's mixed-radix launch shape (its lengths, strides, batch and flags are
  * set); want_tpc > 0 fixes the lines per CTA where they fit, threads > 0 the
  * block (the ragged executor's, whose tiles keep their size in small batches).
@@ -289,11 +297,10 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     if (most > k->ntf) most = k->ntf;
     if (most > (threads ? FZ_RG_LINES : 256)) most = threads ? FZ_RG_LINES : 256;
     /* lines per CTA: about 4096 float / 2048 double points of row lines; whole
-     * segments of neighbouring lines where lanes run across them. Of equal
- * choices the smaller tile (512-point double r2c rows x 262144: 2 lines 588, 4 521,
- * 6 591, 8 546 us). The
-     * executor's tiles, which wait on memory at their ends, are larger (measured on
-     * B200, 4096 ragged transforms, forward: float 1536 points 888 us, 3072 839, 4096
+     * segments of neighbouring lines where lanes run across them. Of equal choices
+     * the smaller tile (512-point double r2c rows x 262144: 2 lines 588, 4 521, 6 591,
+     * 8 546 us). The executor's tiles, which wait on memory at their ends, are larger
+     * (measured on B200, 4096 ragged transforms, forward: float 1536 points 888 us, 3072 839, 4096
      * 809, 6144 805; double 768 2124, 1536 1753, 2048 1459, 3072 1388, and with later
      * stage forms 2048 1298, 3072 1236, 4096 1187 us) */
     const int64_t pts = threads ? (k->dtype == 0 ? 6144 : 4096) : (k->dtype == 0 ? 4096 : 2048);
@@ -319,13 +326,15 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
         while (hi > 1 && (hi * k->n > pts + pts / 2 || (threads == 0 && k->ntf / hi < 2 * 148))) hi--;
         lo = hi > 3 ? hi / 3 : 1;
     }
+    /* `most` counts lines at the distance that a tile of one has; several are
+     * further apart */
+    while (hi > 1 && mr_tile_bytes(k, colmap, hi) > cap) hi--;
+    if (lo > hi) lo = hi;
     double best = -1;
     int btpc = 1, bthr = 32;
     for (int64_t c = lo; c <= hi; c++)
     {
-        k->tpc = (int32_t)c;
-        mr_stride(k, colmap, 0);
-        const int64_t smem = fftz_pass_smem_bytes(k) + 1024;
+        const int64_t smem = mr_tile_bytes(k, colmap, c) + 1024;
         if (smem - 1024 > cap) continue;
         int64_t by_smem = (228 * 1024) / smem;
         if (by_smem > 24) by_smem = 24;

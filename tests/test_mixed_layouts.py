@@ -13,6 +13,7 @@ import aoclfftz_b200
 I32, I64, U32, VP = C.c_int32, C.c_int64, C.c_uint32, C.c_void_p
 MAXS, MAXB, MRS = 12, 8, 8
 VAR_MR, F_TW4, F_MID = 11, 0x04, 0x40
+IN_PAIRS, IN_SEPARATE = 1, 4  # fftz_in_kind
 
 
 class Stage(C.Structure):
@@ -185,6 +186,34 @@ def test_lines_per_cta_follow_the_batch_and_the_hint(ntf, tpc):
     assert p.tpc == 1 or ntf // p.tpc >= 296 or tpc
 
 
+def smooth13(n):
+    for q in (2, 3, 5, 7, 11, 13):
+        while n % q == 0:
+            n //= q
+    return n == 1
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_a_tile_holds_several_lines_where_two_fit(dtype):
+    """Column maps, real lines and lines-per-CTA hints of every length: a tile whose first choice of lines does not fit
+    takes the next smaller one, with a block of its own, not one line on a single warp."""
+    lib = aoclfftz_b200.load()
+    lib.fz_ragged_smem_cap.restype = I64
+    whole, share = 227 * 1024, lib.fz_ragged_smem_cap(dtype)
+    for n in filter(smooth13, range(2, 29000)):
+        line = (n + 32) * (8 << dtype) + 32
+        if 2 * line > whole or not lib.fz_mr_fits(dtype, I64(n), I64(whole)):
+            continue
+        for kw in (dict(col=True), dict(tpc=4), dict(tpc=8), dict(col=True, in_kind=IN_PAIRS),
+                   dict(col=True, in_kind=IN_SEPARATE)):
+            p = shape(n, dtype, ntf=4096, **kw)
+            assert p.tpc > 1 and p.threads >= 64, (n, kw)
+        if 2 * (line + 16 * (8 << dtype)) <= share:
+            for tw4 in (False, True):
+                for ntf in (9, 20, 4096):
+                    assert shape(n, dtype, col=True, tw4=tw4, ntf=ntf, threads=256, cap=share).tpc > 1, (n, tw4, ntf)
+
+
 @pytest.mark.parametrize("n,dtype,ntf,least", [(2, 0, 5000, 64), (144, 0, 40, 14), (5250, 0, 3, 1), (5600, 1, 2, 1), (1, 0, 9, 1)])
 def test_executor_tiles_keep_their_block_and_share(n, dtype, ntf, least):
     """The ragged executor's tiles: 256 threads, within its share of shared memory, small batches not cut up."""
@@ -194,9 +223,6 @@ def test_executor_tiles_keep_their_block_and_share(n, dtype, ntf, least):
     p = shape(n, dtype, ntf=ntf, threads=256, cap=cap)
     assert p.threads == 256 and lib.fftz_pass_smem_bytes(C.byref(p)) <= cap
     assert least <= p.tpc <= ntf
-
-
-IN_PAIRS, IN_SEPARATE = 1, 4  # fftz_in_kind
 
 
 def pair_items(p, s):
