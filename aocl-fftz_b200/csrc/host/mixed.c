@@ -310,11 +310,13 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     else if (colmap)
     {
         /* 8 neighbours (double lines above 440 points, whose 8 would leave fewer than
-         * four CTAs an SM: 4), doubled while a tile stays small. Measured on B200, lines a tile 4 / 6 / 8 / 12 / 16: 120000 x 64 double
-         * (375 and 320 points) 178 / 160 / 154 / 191 / 183 us, 60000 x 64 float (250 and
+         * four CTAs an SM: 4), doubled while a tile stays small. Measured on B200, lines
+         * a tile 4 / 6 / 8 / 12 / 16: 120000 x 64 double (375 and 320 points) 178 / 160 / 154 / 191 / 183 us, 60000 x 64 float (250 and
          * 240) 56 / 51 / 49 / 58 / 54, 1080-point float columns 66 / 56 / 51 / 56 / 51;
-         * 65521 x 32 double (512-point rows of its middle pass) 161 with 4, 182 with 8 */
-        const int64_t seg = k->dtype == 0 || k->n <= 440 ? 8 : 4, room = threads ? pts : pts / 2;
+         * 65521 x 32 double (512-point rows of its middle pass) 161 with 4, 182 with 8.
+         * Two sweeps of more than 1024 float points: 4 as well (convolutions of 2048 and
+         * 4096 points x 4096 columns: 85 / 146 us with 4, 101 / 268 with the most that fit) */
+        const int64_t seg = (k->dtype == 0 ? !two || k->n <= 1024 : k->n <= 440) ? 8 : 4, room = threads ? pts : pts / 2;
         lo = hi = seg < most ? seg : most;
         while (hi * 2 <= most && hi * 2 * k->n <= room && hi < 32) lo = hi = hi * 2;
         /* the executor's block is fixed: a few more columns where they fill it better */
@@ -330,6 +332,25 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
      * further apart */
     while (hi > 1 && mr_tile_bytes(k, colmap, hi) > cap) hi--;
     if (lo > hi) lo = hi;
+    if (colmap && !threads && want_tpc <= 0 && mr_tile_bytes(k, colmap, hi) > 114 * 1024)
+    {
+        /* Tiles that leave an SM one CTA. Columns that one round of CTAs can take: few a
+         * tile, since nothing but latency counts then, a power of two of them (whole
+         * sectors at the strided end). B200, columns a tile: float 5000 x 64 1 13.6, 5 30.7
+         * us; x 300 4 18.8, 5 28.6; 9000 x 64 1 25.7, 3 43.7; double 4840 x 17 1 15.2, 2 18.6;
+         * smaller tiles gain nothing (the passes of a 120000-point double line: 8 16.7, 4
+         * 18.6). From four rounds on a power of two as well: float 5000 x 4096 4 158, 5 248
+         * us; 7260 x 4096 2 303, 3 354; double 3630 x 4096 2 240, 3 262 */
+        int64_t c = 1;
+        while (c * 148 < k->ntf) c *= 2;
+        if (c < hi)
+            lo = hi = c;
+        else if (k->ntf >= 4 * 148 * hi)
+        {
+            while (hi & (hi - 1)) hi &= hi - 1;
+            lo = hi;
+        }
+    }
     double best = -1;
     int btpc = 1, bthr = 32;
     for (int64_t c = lo; c <= hi; c++)

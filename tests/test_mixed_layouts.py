@@ -214,6 +214,18 @@ def test_a_tile_holds_several_lines_where_two_fit(dtype):
                     assert shape(n, dtype, col=True, tw4=tw4, ntf=ntf, threads=256, cap=share).tpc > 1, (n, tw4, ntf)
 
 
+@pytest.mark.parametrize("two", [False, True])
+@pytest.mark.parametrize("n,dtype", [(4840, 0), (5000, 0), (9000, 0), (12000, 0), (2560, 1), (3630, 1), (4840, 1), (5000, 1)])
+def test_few_long_columns_spread_over_the_device(n, dtype, two):
+    """Columns whose tile would fill an SM: where one round of CTAs takes them all, no more a tile than that needs (a
+    power of two); many rounds of tiles hold a power of two of columns."""
+    for ntf in (1, 17, 64, 148):
+        assert shape(n, dtype, col=True, two=two, ntf=ntf).tpc == 1, ntf
+    assert shape(n, dtype, col=True, two=two, ntf=296).tpc <= 2
+    p = shape(n, dtype, col=True, two=two, ntf=50000)
+    assert p.tpc & (p.tpc - 1) == 0
+
+
 @pytest.mark.parametrize("n,dtype,ntf,least", [(2, 0, 5000, 64), (144, 0, 40, 14), (5250, 0, 3, 1), (5600, 1, 2, 1), (1, 0, 9, 1)])
 def test_executor_tiles_keep_their_block_and_share(n, dtype, ntf, least):
     """The ragged executor's tiles: 256 threads, within its share of shared memory, small batches not cut up."""
