@@ -138,8 +138,9 @@ void fz_log(const fz_plan *pl, const char *fmt, ...);
 /* ---- tables (tables.c) ---- */
 int64_t fz_blob_add(fz_blob *b, const void *data, size_t bytes);
 int64_t fz_blob_reserve(fz_blob *b, size_t bytes);
-/* stage twiddles for a radix list; returns blob offset, fills tw_off[] */
-int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off);
+/* stage twiddles for a radix list, the nontrivial ones times 1 + gain; returns
+ * blob offset, fills tw_off[] */
+int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off, double gain);
 /* four-step factor tables W_N^(hi*L), W_N^lo in the working dtype */
 int fz_tw4_tables(fz_blob *b, int dtype, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo);
 /* Bluestein tables for length n, 7-smooth convolution length m, direction */
@@ -160,6 +161,7 @@ int fz_mr_fits(int dtype, int64_t n, int64_t cap);
 int64_t fz_mr_blue_len(int dtype, int64_t n, int64_t cap);
 int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t *n2);
 int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap);
+double fz_mr_gain(int dtype, int R);
 int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k);
 
 /* ---- shared by api.c and ragged.c ---- */

@@ -368,7 +368,7 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
     }
     if (k->nstages > 0)
     {
-        p->off_tw = fz_stage_twiddles(&pl->blob, pl->dtype, (int)n, k->nstages, k->radix, k->tw_off);
+        p->off_tw = fz_stage_twiddles(&pl->blob, pl->dtype, (int)n, k->nstages, k->radix, k->tw_off, 0);
         if (p->off_tw < 0) return NULL;
     }
     snprintf(p->what, sizeof(p->what), "%s n=%lld x%lld",
@@ -836,7 +836,7 @@ static fz_pass *real_pass(fz_plan *pl, int64_t n0, int64_t ies, int64_t oes, con
     }
     if (k->nstages > 0)
     {
-        p->off_tw = fz_stage_twiddles(&pl->blob, pl->dtype, (int)n, k->nstages, k->radix, k->tw_off);
+        p->off_tw = fz_stage_twiddles(&pl->blob, pl->dtype, (int)n, k->nstages, k->radix, k->tw_off, 0);
         if (p->off_tw < 0) return NULL;
     }
     if (packed)

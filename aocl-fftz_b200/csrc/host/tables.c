@@ -18,7 +18,7 @@
 
 /* exp(-2 pi i r / N) for an exactly reduced 0 <= r < N. The angle is folded
  * into the first octant so that the long-double cosl/sinl see |x| <= pi/4. */
-static void w_n(int64_t r, int64_t N, double *re, double *im)
+static void w_nl(int64_t r, int64_t N, long double *re, long double *im)
 {
     r %= N;
     if (r < 0) r += N;
@@ -42,38 +42,55 @@ static void w_n(int64_t r, int64_t N, double *re, double *im)
     case 6: c = sa; s = -ca; break;
     default: { long double b = 2.0L * FZ_PI_L * (0.125L - f); c = cosl(b); s = -sinl(b); break; }
     }
+    *re = c;
+    *im = -s;
+}
+
+static void w_n(int64_t r, int64_t N, double *re, double *im)
+{
+    long double c, s;
+    w_nl(r, N, &c, &s);
     *re = (double)c;
-    *im = (double)(-s);
+    *im = (double)s;
 }
 
 /* All N roots exp(-2 pi i r / N), interleaved, by malloc (NULL on failure):
  * w_n on the part of the circle that the reflections at N / 2, N / 4 and N / 8
- * leave (each where it divides N), mirrored to the rest. */
-static double *roots(int64_t N)
-{
-    double *w = (double *)malloc(sizeof(double) * 2 * (size_t)N);
-    if (!w) return NULL;
-    const int64_t half = N / 2, quarter = N % 2 == 0 ? N / 4 : half, eighth = N % 4 == 0 ? N / 8 : quarter;
-    for (int64_t r = 0; r <= eighth; r++) w_n(r, N, &w[2 * r], &w[2 * r + 1]);
-    if (N % 4 == 0) /* W^{N/4 - r} = -i conj(W^r) */
-        for (int64_t r = eighth + 1; r <= N / 4; r++)
-        {
-            w[2 * r] = -w[2 * (N / 4 - r) + 1];
-            w[2 * r + 1] = -w[2 * (N / 4 - r)];
-        }
-    if (N % 2 == 0) /* W^{N/2 - r} = -conj(W^r) */
-        for (int64_t r = quarter + 1; r <= half; r++)
-        {
-            w[2 * r] = -w[2 * (half - r)];
-            w[2 * r + 1] = w[2 * (half - r) + 1];
-        }
-    for (int64_t r = half + 1; r < N; r++) /* W^{N - r} = conj(W^r) */
-    {
-        w[2 * r] = w[2 * (N - r)];
-        w[2 * r + 1] = -w[2 * (N - r) + 1];
+ * leave (each where it divides N), mirrored to the rest. Rounded to REAL. */
+#define FZ_ROOTS(NAME, REAL)                                                                                           \
+    static REAL *NAME(int64_t N)                                                                                       \
+    {                                                                                                                  \
+        REAL *w = (REAL *)malloc(sizeof(REAL) * 2 * (size_t)N);                                                        \
+        if (!w) return NULL;                                                                                           \
+        const int64_t half = N / 2, quarter = N % 2 == 0 ? N / 4 : half, eighth = N % 4 == 0 ? N / 8 : quarter;        \
+        for (int64_t r = 0; r <= eighth; r++)                                                                          \
+        {                                                                                                              \
+            long double re, im;                                                                                        \
+            w_nl(r, N, &re, &im);                                                                                      \
+            w[2 * r] = (REAL)re;                                                                                       \
+            w[2 * r + 1] = (REAL)im;                                                                                   \
+        }                                                                                                              \
+        if (N % 4 == 0) /* W^{N/4 - r} = -i conj(W^r) */                                                               \
+            for (int64_t r = eighth + 1; r <= N / 4; r++)                                                              \
+            {                                                                                                          \
+                w[2 * r] = -w[2 * (N / 4 - r) + 1];                                                                    \
+                w[2 * r + 1] = -w[2 * (N / 4 - r)];                                                                    \
+            }                                                                                                          \
+        if (N % 2 == 0) /* W^{N/2 - r} = -conj(W^r) */                                                                 \
+            for (int64_t r = quarter + 1; r <= half; r++)                                                              \
+            {                                                                                                          \
+                w[2 * r] = -w[2 * (half - r)];                                                                         \
+                w[2 * r + 1] = w[2 * (half - r) + 1];                                                                  \
+            }                                                                                                          \
+        for (int64_t r = half + 1; r < N; r++) /* W^{N - r} = conj(W^r) */                                             \
+        {                                                                                                              \
+            w[2 * r] = w[2 * (N - r)];                                                                                 \
+            w[2 * r + 1] = -w[2 * (N - r) + 1];                                                                        \
+        }                                                                                                              \
+        return w;                                                                                                      \
     }
-    return w;
-}
+FZ_ROOTS(roots, double)
+FZ_ROOTS(roots_l, long double)
 
 int64_t fz_blob_reserve(fz_blob *b, size_t bytes)
 {
@@ -116,9 +133,10 @@ static void put_c(fz_blob *b, int64_t off, int dtype, int64_t idx, double re, do
     }
 }
 
-int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off)
+int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off, double gain)
 {
-    /* stage s >= 1 uses W_{Ns*R}^{k*r}, k < Ns, r = 1..R-1, at [(r-1)*Ns + k] */
+    /* stage s >= 1 uses W_{Ns*R}^{k*r}, k < Ns, r = 1..R-1, at [(r-1)*Ns + k],
+     * times 1 + gain unless it is +-1 or +-i (scaled before the one rounding) */
     int64_t total = 1, ns = 1;
     for (int s = 0; s < nstages; s++)
     {
@@ -133,8 +151,15 @@ int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32
     put_c(b, off, dtype, 0, 1.0, 0.0);
     if (nstages < 2) return off;
     /* every W_{Ns*R}^{k*r} is a root of order n = the product of the radices */
-    double *w = roots(ns);
+    long double *w = roots_l(ns);
     if (!w) return -1;
+    if (gain != 0)
+        for (int64_t r = 0; r < ns; r++)
+            if (w[2 * r] != 0 && w[2 * r + 1] != 0)
+            {
+                w[2 * r] *= 1.0L + gain;
+                w[2 * r + 1] *= 1.0L + gain;
+            }
     const int64_t N = ns;
     ns = radix[0];
     for (int s = 1; s < nstages; s++)
@@ -142,7 +167,8 @@ int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32
         const int64_t R = radix[s], step = N / (ns * R);
         for (int64_t r = 1; r < R; r++)
             for (int64_t k = 0; k < ns; k++)
-                put_c(b, off, dtype, tw_off[s] + (r - 1) * ns + k, w[2 * (k * r * step)], w[2 * (k * r * step) + 1]);
+                put_c(b, off, dtype, tw_off[s] + (r - 1) * ns + k, (double)w[2 * (k * r * step)],
+                      (double)w[2 * (k * r * step) + 1]);
         ns *= R;
     }
     free(w);
