@@ -141,8 +141,10 @@ int64_t fz_blob_reserve(fz_blob *b, size_t bytes);
 /* stage twiddles for a radix list, the nontrivial ones times 1 + gain; returns
  * blob offset, fills tw_off[] */
 int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off, double gain);
-/* four-step factor tables W_N^(hi*L), W_N^lo in the working dtype */
-int fz_tw4_tables(fz_blob *b, int dtype, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo);
+/* four-step factor tables W_N^(hi*L), W_N^lo: floats, doubles, or each value as a
+ * sum of two doubles */
+enum { FZ_TW4_F32, FZ_TW4_F64, FZ_TW4_F64X2 };
+int fz_tw4_tables(fz_blob *b, int form, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo);
 /* Bluestein tables for length n, 7-smooth convolution length m, direction */
 int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int direction, int64_t *off_pre,
                         int64_t *off_post, int64_t *off_mid);

@@ -459,9 +459,23 @@ static int new_scratch(fz_plan *pl, int64_t elems)
 static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_dim *b, int nb, int src, int dst,
                     int flags);
 
+/* Four-step factors of length n for pass p (made at the first call for this n,
+ * *hi < 0 until then), more exact than the working precision for mixed-radix
+ * passes (kernels/fft_mr.cuh: MrTw4). */
+static int tw4_factors(fz_plan *pl, fz_pass *p, int64_t n, int64_t *hi, int64_t *lo, int64_t *L)
+{
+    const int form = (pl->dtype == 0 ? FZ_TW4_F32 : FZ_TW4_F64) + (p->k.variant == FFTZ_VAR_MR ? 1 : 0);
+    if (*hi < 0 && fz_tw4_tables(&pl->blob, form, n, L, hi, lo)) return -1;
+    p->k.tw4_n = n;
+    p->k.tw4_l = *L;
+    p->off_tw4hi = *hi;
+    p->off_tw4lo = *lo;
+    return 0;
+}
+
 static int fourstep_lines(fz_plan *pl, int64_t n, int64_t n1, int64_t n2, int64_t ies, int64_t oes, const fz_dim *b,
-                          int nb, int src, int dst, int flags, int64_t in_off, int64_t out_off, int64_t hi,
-                          int64_t lo, int64_t L, int S)
+                          int nb, int src, int dst, int flags, int64_t in_off, int64_t out_off, int64_t *hi,
+                          int64_t *lo, int64_t *L, int S)
 {
     fz_dim bb[FFTZ_MAX_BDIMS + 2];
     /* pass A: columns j2 of the n1 x n2 view; scratch layout [line][k1][j2] */
@@ -476,11 +490,7 @@ static int fourstep_lines(fz_plan *pl, int64_t n, int64_t n1, int64_t n2, int64_
         so *= b[i].n;
     }
     fz_pass *pa = line_pass(pl, n1, n2 * ies, n2, bb, nb + 1, 1, src, S, (flags & FFTZ_F_CONJ_IN) | FFTZ_F_TW4, 0);
-    if (!pa) return -1;
-    pa->k.tw4_n = n;
-    pa->k.tw4_l = L;
-    pa->off_tw4hi = hi;
-    pa->off_tw4lo = lo;
+    if (!pa || tw4_factors(pl, pa, n, hi, lo, L)) return -1;
     pa->in_off = in_off;
     /* pass B: rows k1 (contiguous j2) -> X[k1 + n1 k2] */
     bb[0].n = n1;
@@ -528,8 +538,7 @@ static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_d
 {
     int64_t n1, n2;
     if (choose_split(pl, n, &n1, &n2)) return -1;
-    int64_t L, hi, lo;
-    if (fz_tw4_tables(&pl->blob, pl->dtype, n, &L, &hi, &lo)) return -1;
+    int64_t L = 0, hi = -1, lo = -1;
     int64_t lines = lines_of(b, nb);
     int64_t chunk = pl->hints.batch_chunk;
     int nbig = 0;
@@ -548,14 +557,14 @@ static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_d
             fz_dim cb = one;
             cb.n = (lines - c0 < chunk) ? lines - c0 : chunk;
             if (fourstep_lines(pl, n, n1, n2, ies, oes, &cb, 1, src, dst, flags, c0 * one.is * esz,
-                               c0 * one.os * esz, hi, lo, L, S))
+                               c0 * one.os * esz, &hi, &lo, &L, S))
                 return -1;
         }
         return 0;
     }
     int S = new_scratch(pl, n * lines);
     if (S < 0) return -1;
-    return fourstep_lines(pl, n, n1, n2, ies, oes, b, nb, src, dst, flags, 0, 0, hi, lo, L, S);
+    return fourstep_lines(pl, n, n1, n2, ies, oes, b, nb, src, dst, flags, 0, 0, &hi, &lo, &L, S);
 }
 
 /* Bluestein (chirp-z) over a 7-smooth m >= 2n - 1 on mixed-radix tiles (the
@@ -602,8 +611,7 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
     int64_t lines = lines_of(b, nb);
     const int S0 = new_scratch(pl, m * lines), S1 = new_scratch(pl, m * lines);
     if (S0 < 0 || S1 < 0) return -1;
-    int64_t L, hi, lo;
-    if (fz_tw4_tables(&pl->blob, pl->dtype, m, &L, &hi, &lo)) return -1;
+    int64_t L = 0, hi = -1, lo = -1;
     fz_dim bb[FFTZ_MAX_BDIMS + 2];
     int64_t so;
     /* A: src -> S0, column FFTs of the padded chirped input */
@@ -619,14 +627,10 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
     }
     fz_pass *pa = line_pass(pl, n1, n2 * ies, n2, bb, nb + 1, 1, src, S0,
                             (bwd ? FFTZ_F_CONJ_IN : 0) | FFTZ_F_PRE_TAB | FFTZ_F_TW4, 1);
-    if (!pa) return -1;
+    if (!pa || tw4_factors(pl, pa, m, &hi, &lo, &L)) return -1;
     pa->k.pre_n = n;
     pa->k.pre_es = n2;
     pa->k.pre_cs = 1;
-    pa->k.tw4_n = m;
-    pa->k.tw4_l = L;
-    pa->off_tw4hi = hi;
-    pa->off_tw4lo = lo;
     pa->off_pre = pre;
     /* M: S0 -> S1, one pass per row k1 (contiguous j2): forward FFT over j2
      * (the second half of FFT_m of the chirped input, spectrum index
@@ -648,13 +652,9 @@ static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_
         so *= b[i].n;
     }
     fz_pass *pm = line_pass(pl, n2, 1, n1, bb, nb + 1, 1, S0, S1, FFTZ_F_MID_TAB | FFTZ_F_TW4, 1);
-    if (!pm) return -1;
+    if (!pm || tw4_factors(pl, pm, m, &hi, &lo, &L)) return -1;
     pm->k.mid_cs = n2;
     pm->off_mid = midT;
-    pm->k.tw4_n = m;
-    pm->k.tw4_l = L;
-    pm->off_tw4hi = hi;
-    pm->off_tw4lo = lo;
     snprintf(pm->what, sizeof(pm->what), "bluestein-mid n=%lld m=%lld x%lld", (long long)n, (long long)m,
              (long long)pm->k.ntf);
     /* D: S1 -> dst, rows k1' (contiguous k1): FFT over k1 -> k2', output

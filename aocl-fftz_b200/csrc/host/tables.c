@@ -175,34 +175,42 @@ int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32
     return off;
 }
 
-int fz_tw4_tables(fz_blob *b, int dtype, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo)
+int fz_tw4_tables(fz_blob *b, int form, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo)
 {
-    /* W_N^r = hi[r / L] * lo[r % L]: both factors formed in FP64 and stored in
-     * the working precision (the product is taken in the working precision) */
+    /* W_N^r = hi[r / L] * lo[r % L]: both factors formed in long double and stored
+     * in the precision that the product is taken in (form: FZ_TW4_*) */
     int64_t l = 1;
+    if (N > 0xFFFFFFFFLL)
+    {
+        fz_set_error("four-step length %lld above 2^32 - 1", (long long)N); /* the kernels' r has 32 bits */
+        return -1;
+    }
     while (l * l < N) l *= 2;
     /* lo holds at most 1024 factors while hi stays <= 2^20 entries: the
      * four-step epilogue's random lookups (r = column * k) then stay within
      * two 1024-entry tables that remain in L1 beside the stage twiddles */
     if (l > 1024 && (N + 1023) / 1024 <= ((int64_t)1 << 20)) l = 1024;
-    int64_t nhi = (N + l - 1) / l;
-    size_t esz = dtype == 0 ? 8 : 16;
+    const int64_t nhi = (N + l - 1) / l;
+    const size_t esz = form == FZ_TW4_F32 ? 8 : form == FZ_TW4_F64 ? 16 : 32;
     *L = l;
-    *off_hi = fz_blob_reserve(b, (size_t)nhi * esz);
-    if (*off_hi < 0) return -1;
-    for (int64_t j = 0; j < nhi; j++)
+    for (int side = 0; side < 2; side++)
     {
-        double re, im;
-        w_n(j * l, N, &re, &im);
-        put_c(b, *off_hi, dtype, j, re, im);
-    }
-    *off_lo = fz_blob_reserve(b, (size_t)l * esz);
-    if (*off_lo < 0) return -1;
-    for (int64_t j = 0; j < l; j++)
-    {
-        double re, im;
-        w_n(j, N, &re, &im);
-        put_c(b, *off_lo, dtype, j, re, im);
+        const int64_t n = side == 0 ? nhi : l, step = side == 0 ? l : 1;
+        const int64_t off = fz_blob_reserve(b, (size_t)n * esz);
+        if (off < 0) return -1;
+        *(side == 0 ? off_hi : off_lo) = off;
+        for (int64_t j = 0; j < n; j++)
+        {
+            long double re, im;
+            w_nl(j * step, N, &re, &im);
+            if (form == FZ_TW4_F64X2)
+            {
+                put_c(b, off, 1, 2 * j, (double)re, (double)im);
+                put_c(b, off, 1, 2 * j + 1, (double)(re - (double)re), (double)(im - (double)im));
+            }
+            else
+                put_c(b, off, form == FZ_TW4_F32 ? 0 : 1, j, (double)re, (double)im);
+        }
     }
     return 0;
 }

@@ -63,6 +63,14 @@ def test_one_pass_lines(kind, dtype, n, direction, former):
     check(kind, dtype, n, direction, former)
 
 
+@pytest.mark.parametrize("kind,dtype,n,direction,former", [
+    ("c2c", "f32", 117649, 1, 1.600e-7), ("c2c", "f32", 177147, 1, 1.765e-7), ("c2c", "f32", 500000, 1, 1.652e-7),
+    ("c2c", "f32", 531441, 1, 1.852e-7), ("c2c", "f64", 117649, 1, 2.879e-16), ("c2c", "f64", 161051, 1, 3.019e-16),
+    ("c2c", "f64", 390625, 1, 3.163e-16), ("c2c", "f64", 531441, 1, 4.000e-16), ("real", "f64", 16807, 1, 2.008e-16)])
+def test_four_step_lines(kind, dtype, n, direction, former):
+    check(kind, dtype, n, direction, former)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f64"])
 @pytest.mark.parametrize("n", [3, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16])
 def test_mean_gain_of_the_butterflies(n, dtype):

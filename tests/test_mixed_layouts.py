@@ -273,3 +273,40 @@ def test_mirrored_butterflies_cover_each_bin_once(n, col):
         x = np.random.default_rng(n).standard_normal((p.tpc, n)) + 0j
         if kind == IN_PAIRS:
             assert np.linalg.norm(simulate(p, x) - np.fft.fft(x, axis=1)) <= 1e-13 * np.linalg.norm(x) * np.sqrt(n)
+
+
+class Blob(C.Structure):
+    """fz_blob (csrc/host/fz_internal.h)."""
+    _fields_ = [("p", VP), ("len", C.c_size_t), ("cap", C.c_size_t)]
+
+
+@pytest.mark.parametrize("form,parts,eps", [(0, 1, 2.0 ** -24), (1, 1, 2.0 ** -53), (2, 2, 2.0 ** -63)])
+@pytest.mark.parametrize("N", [1, 6, 4096, 120000, 3 * 2 ** 20 + 1])
+def test_four_step_factor_tables(N, form, parts, eps):
+    """W_N^r = hi[r / L] lo[r % L] for every r, each entry rounded once: floats, doubles, or a sum of two doubles (whose
+    second is what the first left, down to the long double it was formed in)."""
+    lib = aoclfftz_b200.load()
+    b, L, hi, lo = Blob(), I64(), I64(), I64()
+    assert lib.fz_tw4_tables(C.byref(b), form, I64(N), C.byref(L), C.byref(hi), C.byref(lo)) == 0
+    raw = (C.c_ubyte * b.len).from_address(b.p)
+    real = np.float32 if form == 0 else np.float64
+
+    def entries(off, n):
+        v = np.frombuffer(raw, dtype=real, count=2 * parts * n, offset=off).astype(np.longdouble).reshape(n, parts, 2)
+        return v.sum(axis=1)
+
+    nhi = -(-N // L.value)
+    h, l = entries(hi.value, nhi), entries(lo.value, L.value)
+    for got, r in ((h, np.arange(nhi) * L.value), (l, np.arange(L.value))):
+        a = 2 * np.arctan2(np.longdouble(0), np.longdouble(-1)) * r.astype(np.longdouble) / N
+        # half a unit in the last place of a value below one, plus this angle's own error: up to 2 pi in long double, its
+        # pi, product and quotient each rounded by at most 2^-62, and the cosine
+        assert np.abs(got - np.stack([np.cos(a), -np.sin(a)], axis=1)).max() <= eps / 2 + 4 * 2.0 ** -62
+    assert b.len >= lo.value + L.value * parts * 2 * real().itemsize
+
+
+def test_four_step_factors_beyond_32_bits_are_refused():
+    lib = aoclfftz_b200.load()
+    b, L, hi, lo = Blob(), I64(), I64(), I64()
+    assert lib.fz_tw4_tables(C.byref(b), 1, I64(1 << 32), C.byref(L), C.byref(hi), C.byref(lo)) != 0
+    assert not b.p
