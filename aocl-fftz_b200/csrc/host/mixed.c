@@ -1,5 +1,6 @@
 /* Launch shape of mixed-radix lines (kernels/fft_mr.cuh): radix list, digit
  * strides with their bank padding, transforms and threads per CTA (C99). */
+#include <math.h>
 #include <string.h>
 
 #include "fz_internal.h"
@@ -118,48 +119,101 @@ static int64_t next_smooth7(int64_t n)
     }
 }
 
-/* Convolution length of a chirp-z transform of n points in one tile: the
- * 7-smooth m >= 2n - 1 with the fewest issue slots over both sweeps (a longer m
- * with fewer stages beats the nearest one); 0 when none fits cap bytes. */
+/* Rounding error of a chirp-z transform of n points over a convolution of m
+ * points: rel-L2^2 = 48 + (2 n / m) X, in 1e-16 (float; double in 2^-58 of that). The
+ * noise of both FFTs is white over the m points and the n wanted ones hold half
+ * of the signal, hence 2 n / m: padding lowers the error. X is the sum below over the
+ * stages of both FFTs, fitted on B200 to 1426 pairs of n (17 ... 400009) and m in float
+ * (residual 1.7% of rel-L2^2); double has the same, plus the error of a spectrum
+ * formed in double where it is (tables.c). */
+static double blue_noise(int nst, const int32_t *radix, int64_t m)
+{
+    static const double butterfly[17] = {0, 0, 0, 0.3, 0, 7.4, 4.7, 12.1, 8.0, 18.4, 13.3, 0, 11.0, 0, 17.6, 21.0, 17.1};
+    double x = 0;
+    for (int s = 0; s < nst; s++)
+    {
+        m /= radix[s];
+        x += 2 * butterfly[radix[s]];
+        if (s < nst - 1) x += 2 * 36.1 * (1 - 1.0 / radix[s]) * (1 - 1.0 / (double)m);
+    }
+    return x;
+}
+
+/* 1 if a convolution of m points with stage noise x is no less exact (to 1%) than
+ * one over the power of two, as it ran before lengths with odd factors were taken:
+ * X per bit measured by the bit length of that power of two (above 2^14 float and
+ * 2^13 double in three passes). A power of two itself always is. */
+static int blue_exact_enough(int dtype, int64_t n, int64_t m, double x)
+{
+    static const double former[2][21] = {
+        {0, 0, 0, 0, 0, 0, 19.5, 19.5, 23.2, 22.7, 23.2, 24.9, 27.0, 24.9, 26.2, 31.2, 31.2, 31.2, 31.2, 31.2, 31.2},
+        {0, 0, 0, 0, 0, 0, 21.0, 29.0, 33.0, 40.0, 40.5, 41.0, 41.0, 48.0, 48.6, 49.4, 47.9, 51.0, 54.0, 56.0, 54.0}};
+    int l = 6;
+    while (((int64_t)1 << l) < 2 * n - 1) l++;
+    const double p = (double)((int64_t)1 << l);
+    if ((double)m >= p) return 1;
+    /* the former kernels' gain error (fz_mr_gain) is not divided by the padding */
+    double limit = former[dtype == 0 ? 0 : 1][l < 20 ? l : 20] * l * (2.0 * (double)n < 0.56 * p ? 1.1 : 1.0);
+    if (dtype == 1) x += m <= FZ_EXACT_SPECTRUM ? 10 : 19.5 * log2((double)m);
+    return (22.6 + x) * p <= 1.03 * limit * (double)m;
+}
+
+/* Convolution length of a chirp-z transform of n points in one tile: of the
+ * 7-smooth m >= 2n - 1 that are exact enough, from the first on up to a quarter
+ * beyond it, the one with the fewest issue slots over both sweeps (a longer m with
+ * fewer stages beats the nearest one); 0 when none fits cap bytes. */
 int64_t fz_mr_blue_len(int dtype, int64_t n, int64_t cap)
 {
     int32_t r[FFTZ_MR_STAGES];
-    int64_t best = 0;
+    int64_t best = 0, last = INT64_MAX;
     double score = 0, c;
     const int64_t need = 2 * n - 1;
-    if (need * (dtype == 0 ? 8 : 16) > cap) return 0;
-    for (int64_t m = next_smooth7(need < 4 ? 4 : need); m <= need + need / 4 + 4; m = next_smooth7(m + 1))
-        if (fz_mr_fits(dtype, m, cap) && fz_mr_radices(m, 2, 0, r, &c) > 1 && (!best || (double)m * c < score))
-        {
-            best = m;
-            score = (double)m * c;
-        }
+    for (int64_t m = next_smooth7(need < 4 ? 4 : need); m <= last && fz_mr_fits(dtype, m, cap); m = next_smooth7(m + 1))
+    {
+        const int nst = fz_mr_radices(m, 2, 0, r, &c);
+        if (nst < 2 || (best && (double)m * c >= score) || !blue_exact_enough(dtype, n, m, blue_noise(nst, r, m))) continue;
+        if (!best) last = m + m / 4 + 4;
+        best = m;
+        score = (double)m * c;
+    }
     return best;
 }
 
 /* Convolution length m = n1 * n2 of a chirp-z transform in three passes: the
- * cheapest of the first 7-smooth lengths from 2n - 1 on, both factors one tile
- * and n2 of at least two stages, within a factor of four of each other. */
+ * cheapest of the first twelve 7-smooth lengths from 2n - 1 on that are exact enough
+ * and have both factors one tile, n2 of at least two stages, within a factor of
+ * four of each other (any such length when none is exact enough). */
 int64_t fz_mr_blue_split(int dtype, int64_t n, int64_t cap, int64_t *n1, int64_t *n2)
 {
-    int32_t r[FFTZ_MR_STAGES];
-    int64_t best = 0, m = 2 * n - 2;
+    int32_t ra[FFTZ_MR_STAGES], rb[FFTZ_MR_STAGES];
+    int64_t best = 0;
     double score = 0, ca, cb;
-    for (int tries = 0; tries < 64 && (tries < 12 || !best); tries++)
+    for (int strict = 1; strict >= 0 && !best; strict--)
     {
-        m = next_smooth7(m + 1);
-        for (int64_t a = 2; a * a <= 4 * m; a++)
+        int64_t m = 2 * n - 2;
+        for (int found = 0, tries = 0; found < 12 && tries < (strict ? 1000 : 64); tries++)
         {
-            const int64_t b = m / a;
-            if (m % a || a > 4 * b || b > 4 * a || !fz_mr_fits(dtype, a, cap) || !fz_mr_fits(dtype, b, cap)) continue;
-            if (fz_mr_radices(a, 1, 0, r, &ca) < 1 || fz_mr_radices(b, 2, 0, r, &cb) < 2) continue;
-            if (!best || (double)m * (ca + cb) < score)
+            m = next_smooth7(m + 1);
+            if (strict && m > 4 * n) break;
+            int any = 0;
+            for (int64_t a = 2; a * a <= 4 * m; a++)
             {
-                best = m;
-                score = (double)m * (ca + cb);
-                *n1 = a;
-                *n2 = b;
+                const int64_t b = m / a;
+                if (m % a || a > 4 * b || b > 4 * a || !fz_mr_fits(dtype, a, cap) || !fz_mr_fits(dtype, b, cap)) continue;
+                const int sa = fz_mr_radices(a, 1, 0, ra, &ca), sb = fz_mr_radices(b, 2, 0, rb, &cb);
+                if (sa < 1 || sb < 2) continue;
+                /* 90: the four-step factors between the passes */
+                if (strict && !blue_exact_enough(dtype, n, m, 90 + blue_noise(sa, ra, a) + blue_noise(sb, rb, b))) continue;
+                any = 1;
+                if (!best || (double)m * (ca + cb) < score)
+                {
+                    best = m;
+                    score = (double)m * (ca + cb);
+                    *n1 = a;
+                    *n2 = b;
+                }
             }
+            found += any;
         }
     }
     return best;

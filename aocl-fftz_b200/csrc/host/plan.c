@@ -568,13 +568,14 @@ static int fourstep(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_d
 }
 
 /* Bluestein (chirp-z) over a 7-smooth m >= 2n - 1 on mixed-radix tiles (the
- * reference pads to a 13-smooth m, core/common/bluestein_utils.c:39-67). A
- * convolution that fits a CTA (m up to 28672 float, 14400 double) is one kernel, which reads and writes
- * HBM once: measured on B200, n = 10007 float x 512, m = 32768 in three passes 452
- * us, m = 20736 in three passes 317 us, in one kernel 142 us; one line 52, 52
- * and 35 us. Only a few double lines near the limit are faster in three passes
- * (n = 7001: 45 us in one kernel against 37 us up to 32 lines, 46 against 66 us
- * for 64), both faster than three passes over a power of two (58 us). */
+ * reference pads to a 13-smooth m, core/common/bluestein_utils.c:39-67), of those no
+ * less exact than the next power of two (blue_exact_enough). A convolution that fits
+ * a CTA (fz_mr_fits: m up to 28812 float, 14406 double) is one kernel, which reads and
+ * writes HBM once. Measured on B200, one kernel / three passes over the best such m,
+ * us: n = 10007 float x 592 118 / 283, x 148 30 / 92, x 32 30 / 33, one line 30 / 24;
+ * 7001 double x 592 160 / 307, x 148 38 / 97, x 32 38 / 33, one line 37 / 21. Few lines
+ * near the limit are faster in three passes; over a power of two in three passes,
+ * as it had been, they took 52 and 56 us. */
 static int bluestein(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, const fz_dim *b, int nb, int src, int dst)
 {
     int64_t n1 = 0, n2 = 0, m = fz_mr_blue_len(pl->dtype, n, mixed_cap(pl));

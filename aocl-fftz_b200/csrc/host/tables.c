@@ -54,43 +54,17 @@ static void w_n(int64_t r, int64_t N, double *re, double *im)
     *im = (double)s;
 }
 
-/* All N roots exp(-2 pi i r / N), interleaved, by malloc (NULL on failure):
- * w_n on the part of the circle that the reflections at N / 2, N / 4 and N / 8
- * leave (each where it divides N), mirrored to the rest. Rounded to REAL. */
-#define FZ_ROOTS(NAME, REAL)                                                                                           \
-    static REAL *NAME(int64_t N)                                                                                       \
-    {                                                                                                                  \
-        REAL *w = (REAL *)malloc(sizeof(REAL) * 2 * (size_t)N);                                                        \
-        if (!w) return NULL;                                                                                           \
-        const int64_t half = N / 2, quarter = N % 2 == 0 ? N / 4 : half, eighth = N % 4 == 0 ? N / 8 : quarter;        \
-        for (int64_t r = 0; r <= eighth; r++)                                                                          \
-        {                                                                                                              \
-            long double re, im;                                                                                        \
-            w_nl(r, N, &re, &im);                                                                                      \
-            w[2 * r] = (REAL)re;                                                                                       \
-            w[2 * r + 1] = (REAL)im;                                                                                   \
-        }                                                                                                              \
-        if (N % 4 == 0) /* W^{N/4 - r} = -i conj(W^r) */                                                               \
-            for (int64_t r = eighth + 1; r <= N / 4; r++)                                                              \
-            {                                                                                                          \
-                w[2 * r] = -w[2 * (N / 4 - r) + 1];                                                                    \
-                w[2 * r + 1] = -w[2 * (N / 4 - r)];                                                                    \
-            }                                                                                                          \
-        if (N % 2 == 0) /* W^{N/2 - r} = -conj(W^r) */                                                                 \
-            for (int64_t r = quarter + 1; r <= half; r++)                                                              \
-            {                                                                                                          \
-                w[2 * r] = -w[2 * (half - r)];                                                                         \
-                w[2 * r + 1] = w[2 * (half - r) + 1];                                                                  \
-            }                                                                                                          \
-        for (int64_t r = half + 1; r < N; r++) /* W^{N - r} = conj(W^r) */                                             \
-        {                                                                                                              \
-            w[2 * r] = w[2 * (N - r)];                                                                                 \
-            w[2 * r + 1] = -w[2 * (N - r) + 1];                                                                        \
-        }                                                                                                              \
-        return w;                                                                                                      \
-    }
-FZ_ROOTS(roots, double)
-FZ_ROOTS(roots_l, long double)
+/* roots, host_fft, chirp_spectrum in double, and the same in long double (_l) */
+#define REAL double
+#define FORM(name) name
+#include "tables_fft.h"
+#undef REAL
+#undef FORM
+#define REAL long double
+#define FORM(name) name##_l
+#include "tables_fft.h"
+#undef REAL
+#undef FORM
 
 int64_t fz_blob_reserve(fz_blob *b, size_t bytes)
 {
@@ -215,119 +189,17 @@ int fz_tw4_tables(fz_blob *b, int form, int64_t N, int64_t *L, int64_t *off_hi, 
     return 0;
 }
 
-/* Forward FFT in double, m a product of 2, 3, 5 and 7: Stockham stages of 4 and
- * the prime factors between x and a second buffer. Returns 0, or -1 on allocation
- * failure. */
-static int host_fft(double *x, int64_t m)
-{
-    double *w = roots(m), *y = (double *)malloc(sizeof(double) * 2 * (size_t)m);
-    double *src = x, *dst = y;
-    if (!w || !y)
-    {
-        free(w);
-        free(y);
-        return -1;
-    }
-    int64_t n = m, st = 1; /* length still to transform, transforms side by side */
-    while (n > 1)
-    {
-        const int p = n % 4 == 0 ? 4 : n % 2 == 0 ? 2 : n % 3 == 0 ? 3 : n % 5 == 0 ? 5 : 7;
-        const int64_t h = n / p;
-        double e[7][2]; /* W_p^j */
-        for (int j = 0; j < p; j++)
-        {
-            e[j][0] = w[2 * (j * (m / p))];
-            e[j][1] = w[2 * (j * (m / p)) + 1];
-        }
-        for (int64_t k = 0; k < h; k++)
-            for (int64_t q = 0; q < st; q++)
-            {
-                double v[7][2], o[7][2];
-                for (int j = 0; j < p; j++)
-                {
-                    v[j][0] = src[2 * (q + st * (k + j * h))];
-                    v[j][1] = src[2 * (q + st * (k + j * h)) + 1];
-                }
-                if (p == 4)
-                {
-                    const double ar = v[0][0] + v[2][0], ai = v[0][1] + v[2][1], br = v[0][0] - v[2][0],
-                                 bi = v[0][1] - v[2][1], cr = v[1][0] + v[3][0], ci = v[1][1] + v[3][1],
-                                 dr = v[1][0] - v[3][0], di = v[1][1] - v[3][1];
-                    o[0][0] = ar + cr, o[0][1] = ai + ci, o[2][0] = ar - cr, o[2][1] = ai - ci;
-                    o[1][0] = br + di, o[1][1] = bi - dr, o[3][0] = br - di, o[3][1] = bi + dr;
-                }
-                else
-                    for (int r = 0; r < p; r++)
-                    {
-                        o[r][0] = v[0][0];
-                        o[r][1] = v[0][1];
-                        for (int j = 1, i = r; j < p; j++, i = i + r >= p ? i + r - p : i + r)
-                        {
-                            o[r][0] += v[j][0] * e[i][0] - v[j][1] * e[i][1];
-                            o[r][1] += v[j][0] * e[i][1] + v[j][1] * e[i][0];
-                        }
-                    }
-                for (int r = 0; r < p; r++) /* output r of the butterfly, times W_n^{k r} */
-                {
-                    const double *t = w + 2 * (k * r * st);
-                    double *d = dst + 2 * (q + st * (p * k + r));
-                    d[0] = o[r][0] * t[0] - o[r][1] * t[1];
-                    d[1] = o[r][0] * t[1] + o[r][1] * t[0];
-                }
-            }
-        double *sw = src;
-        src = dst;
-        dst = sw;
-        st *= p;
-        n = h;
-    }
-    if (src != x) memcpy(x, src, sizeof(double) * 2 * (size_t)m);
-    free(w);
-    free(y);
-    return 0;
-}
-
 int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int direction, int64_t *off_pre,
                         int64_t *off_post, int64_t *off_mid)
 {
-    /* forward chirp c_j = exp(-i pi (j^2 mod 2n) / n) = W_{2n}^{j^2 mod 2n}
-     * (core/common/bluestein_utils.c:88-159 keeps the square exact in integers) */
+    /* forward chirp c_j and the spectrum of its conjugate's periodic extension over m
+     * (there 1 / m costs no rounding of its own). In a double plan a spectrum formed in
+     * double has an error that counts (2.3e-16 of 3.8e-16 at m = 8192); long double takes
+     * it away where its time is short */
     size_t esz = dtype == 0 ? 8 : 16;
     double *c = (double *)malloc(sizeof(double) * 2 * (size_t)n);
-    double *bb = (double *)calloc(2 * (size_t)m, sizeof(double));
-    if (!c || !bb)
-    {
-        free(c);
-        free(bb);
-        return -1;
-    }
-    const int64_t n2 = 2 * n;
-    double *wc = roots(n2);
-    if (!wc)
-    {
-        free(c);
-        free(bb);
-        return -1;
-    }
-    for (int64_t j = 0; j < n; j++)
-    {
-        int64_t sq = (int64_t)(((unsigned __int128)j * (unsigned __int128)j) % (unsigned __int128)n2);
-        c[2 * j] = wc[2 * sq];
-        c[2 * j + 1] = wc[2 * sq + 1];
-    }
-    free(wc);
-    /* b_j = conj(c_j) at j and m - j, zero between */
-    for (int64_t j = 0; j < n; j++)
-    {
-        bb[2 * j] = c[2 * j];
-        bb[2 * j + 1] = -c[2 * j + 1];
-        if (j > 0)
-        {
-            bb[2 * (m - j)] = c[2 * j];
-            bb[2 * (m - j) + 1] = -c[2 * j + 1];
-        }
-    }
-    if (host_fft(bb, m))
+    double *bb = (double *)malloc(sizeof(double) * 2 * (size_t)m);
+    if (!c || !bb || (dtype == 1 && m <= FZ_EXACT_SPECTRUM ? chirp_spectrum_l(n, m, c, bb) : chirp_spectrum(n, m, c, bb)))
     {
         free(c);
         free(bb);
@@ -342,14 +214,10 @@ int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int directi
         free(bb);
         return -1;
     }
-    const double inv_m = 1.0 / (double)m;
     for (int64_t j = 0; j < n; j++)
     {
         put_c(b, *off_pre, dtype, j, c[2 * j], c[2 * j + 1]);
-        if (direction == 0)
-            put_c(b, *off_post, dtype, j, c[2 * j] * inv_m, c[2 * j + 1] * inv_m);
-        else
-            put_c(b, *off_post, dtype, j, c[2 * j] * inv_m, -c[2 * j + 1] * inv_m);
+        put_c(b, *off_post, dtype, j, c[2 * j], direction == 0 ? c[2 * j + 1] : -c[2 * j + 1]);
     }
     for (int64_t j = 0; j < m; j++) put_c(b, *off_mid, dtype, j, bb[2 * j], -bb[2 * j + 1]);
     free(c);

@@ -71,6 +71,20 @@ def test_four_step_lines(kind, dtype, n, direction, former):
     check(kind, dtype, n, direction, former)
 
 
+@pytest.mark.parametrize("dtype,n,former", [
+    ("f32", 17, 1.094e-7), ("f32", 101, 1.402e-7), ("f32", 521, 1.411e-7), ("f32", 1031, 1.528e-7),
+    ("f32", 2053, 1.501e-7), ("f32", 3001, 1.701e-7), ("f32", 4099, 1.586e-7), ("f32", 5003, 1.683e-7),
+    ("f32", 8209, 1.781e-7), ("f32", 10007, 1.860e-7), ("f32", 16411, 1.871e-7), ("f32", 20011, 1.951e-7),
+    ("f32", 32771, 1.900e-7), ("f32", 262147, 2.020e-7), ("f64", 17, 2.113e-16), ("f64", 101, 3.025e-16),
+    ("f64", 521, 3.243e-16), ("f64", 1031, 3.345e-16), ("f64", 2053, 3.772e-16), ("f64", 3001, 4.179e-16),
+    ("f64", 4099, 3.991e-16), ("f64", 5003, 4.192e-16), ("f64", 8209, 4.032e-16), ("f64", 10007, 4.251e-16),
+    ("f64", 16411, 4.057e-16), ("f64", 20011, 4.281e-16), ("f64", 32771, 4.438e-16), ("f64", 262147, 4.932e-16)])
+def test_chirp_lengths(dtype, n, former):
+    """Primes, most of them just above a power of two, whose convolution over the next power of two was the most exact
+    (its noise spreads over twice the points); formerly: that power of two."""
+    check("c2c", dtype, n, 1, former)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f64"])
 @pytest.mark.parametrize("n", [3, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16])
 def test_mean_gain_of_the_butterflies(n, dtype):
