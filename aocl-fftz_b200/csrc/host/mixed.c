@@ -413,10 +413,15 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
         if (smem - 1024 > cap) continue;
         int64_t by_smem = (228 * 1024) / smem;
         if (by_smem > 24) by_smem = 24;
+        /* a batch of one CTA an SM at most: the block that fills it alone. (Chosen as if
+         * others ran beside it, blocks were small: B200, double 2197 points x 1 11.8 us,
+         * 8.3 on the kernel before, float columns 2000 x 64 13.3.) */
+        const int alone = !threads && (k->ntf + c - 1) / c <= 148;
         for (int t = threads ? threads : 64; t <= (threads ? threads : tmax); t += 32)
         {
             int64_t ctas = tmax / t;
             if (ctas > by_smem) ctas = by_smem;
+            if (alone) ctas = 1;
             double used = 0, spent = 0;
             for (int s = 0; s < k->nstages; s++)
             {

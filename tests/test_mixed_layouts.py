@@ -226,6 +226,17 @@ def test_few_long_columns_spread_over_the_device(n, dtype, two):
     assert p.tpc & (p.tpc - 1) == 0
 
 
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("n", [1000, 2100, 2197, 4096, 12000])
+def test_a_lone_cta_is_not_a_small_one(n, dtype):
+    """One line: no other CTA shares its SM, so its block covers at least half of a stage's butterflies (or of the largest
+    block)."""
+    lib = aoclfftz_b200.load()
+    p = shape(n, dtype, ntf=1)
+    most = lib.fftz_mr_max_threads(dtype, p.mr.big)
+    assert 2 * p.threads >= min(most, max(st.nb for st in p.mr.st[: p.nstages]))
+
+
 @pytest.mark.parametrize("n,dtype,ntf,least", [(2, 0, 5000, 64), (144, 0, 40, 14), (5250, 0, 3, 1), (5600, 1, 2, 1), (1, 0, 9, 1)])
 def test_executor_tiles_keep_their_block_and_share(n, dtype, ntf, least):
     """The ragged executor's tiles: 256 threads, within its share of shared memory, small batches not cut up."""
