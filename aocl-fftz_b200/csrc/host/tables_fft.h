@@ -38,17 +38,13 @@ static REAL *FORM(roots)(int64_t N)
 }
 
 /* Forward FFT, m a product of 2, 3, 5 and 7: Stockham stages of 4 and the prime
- * factors between x and a second buffer. Returns 0, or -1 on allocation failure. */
-static int FORM(host_fft)(REAL *x, int64_t m)
+ * factors between x and a second buffer. w: roots of order m ws. Returns 0, or -1 on
+ * allocation failure. */
+static int FORM(host_fft)(REAL *x, int64_t m, const REAL *w, int64_t ws)
 {
-    REAL *w = FORM(roots)(m), *y = (REAL *)malloc(sizeof(REAL) * 2 * (size_t)m);
+    REAL *y = (REAL *)malloc(sizeof(REAL) * 2 * (size_t)m);
     REAL *src = x, *dst = y;
-    if (!w || !y)
-    {
-        free(w);
-        free(y);
-        return -1;
-    }
+    if (!y) return -1;
     int64_t n = m, st = 1; /* length still to transform, transforms side by side */
     while (n > 1)
     {
@@ -57,8 +53,8 @@ static int FORM(host_fft)(REAL *x, int64_t m)
         REAL e[7][2]; /* W_p^j */
         for (int j = 0; j < p; j++)
         {
-            e[j][0] = w[2 * (j * (m / p))];
-            e[j][1] = w[2 * (j * (m / p)) + 1];
+            e[j][0] = w[2 * (j * (m / p) * ws)];
+            e[j][1] = w[2 * (j * (m / p) * ws) + 1];
         }
         for (int64_t k = 0; k < h; k++)
             for (int64_t q = 0; q < st; q++)
@@ -90,7 +86,7 @@ static int FORM(host_fft)(REAL *x, int64_t m)
                     }
                 for (int r = 0; r < p; r++) /* output r of the butterfly, times W_n^{k r} */
                 {
-                    const REAL *t = w + 2 * (k * r * st);
+                    const REAL *t = w + 2 * (k * r * st * ws);
                     REAL *d = dst + 2 * (q + st * (p * k + r));
                     d[0] = o[r][0] * t[0] - o[r][1] * t[1];
                     d[1] = o[r][0] * t[1] + o[r][1] * t[0];
@@ -103,9 +99,40 @@ static int FORM(host_fft)(REAL *x, int64_t m)
         n = h;
     }
     if (src != x) memcpy(x, src, sizeof(REAL) * 2 * (size_t)m);
-    free(w);
     free(y);
     return 0;
+}
+
+/* The same of an even sequence, x_j = x_{m - j}, whose spectrum is even too: bins 2k
+ * are the half-length transform of x_j + x_{j + m/2}, again even, bins 4k + 1 one of
+ * a quarter of the length, and bin 4k + 3 is bin m - 4k - 3, one of those. Half the
+ * work of host_fft. */
+static int FORM(even_fft)(REAL *x, int64_t m, const REAL *w, int64_t ws)
+{
+    if (m % 4 != 0) return FORM(host_fft)(x, m, w, ws);
+    const int64_t h = m / 2, q = m / 4;
+    REAL *e = (REAL *)malloc(sizeof(REAL) * 2 * (size_t)(h + q)), *y = e + 2 * h;
+    if (!e) return -1;
+    for (int64_t j = 0; j < 2 * h; j++) e[j] = x[j] + x[j + 2 * h];
+    for (int64_t j = 0; j < q; j++)
+    {
+        const REAL ar = x[2 * j] - x[2 * (j + h)], ai = x[2 * j + 1] - x[2 * (j + h) + 1];
+        const REAL br = x[2 * (j + q)] - x[2 * (j + q + h)], bi = x[2 * (j + q) + 1] - x[2 * (j + q + h) + 1];
+        const REAL re = ar + bi, im = ai - br, *t = w + 2 * (j * ws); /* a - i b */
+        y[2 * j] = re * t[0] - im * t[1];
+        y[2 * j + 1] = re * t[1] + im * t[0];
+    }
+    const int rc = FORM(even_fft)(e, h, w, 2 * ws) || FORM(host_fft)(y, q, w, 4 * ws) ? -1 : 0;
+    for (int64_t k = 0; rc == 0 && k < q; k++)
+        for (int c = 0; c < 2; c++)
+        {
+            x[2 * (4 * k) + c] = e[2 * (2 * k) + c];
+            x[2 * (4 * k + 1) + c] = y[2 * k + c];
+            x[2 * (4 * k + 2) + c] = e[2 * (2 * k + 1) + c];
+            x[2 * (4 * k + 3) + c] = y[2 * (q - 1 - k) + c];
+        }
+    free(e);
+    return rc;
 }
 
 /* c: the chirp c_j = exp(-i pi (j^2 mod 2n) / n) = W_{2n}^{j^2 mod 2n}, j < n
@@ -130,7 +157,9 @@ static int FORM(chirp_spectrum)(int64_t n, int64_t m, double *c, double *bb)
         }
     }
     free(w);
-    if (rc == 0) rc = FORM(host_fft)(x, m);
+    w = rc == 0 ? FORM(roots)(m) : NULL;
+    rc = w ? FORM(even_fft)(x, m, w, 1) : -1;
+    free(w);
     for (int64_t j = 0; rc == 0 && j < 2 * m; j++) bb[j] = (double)(x[j] / (REAL)m);
     free(x);
     return rc;

@@ -321,3 +321,31 @@ def test_four_step_factors_beyond_32_bits_are_refused():
     b, L, hi, lo = Blob(), I64(), I64(), I64()
     assert lib.fz_tw4_tables(C.byref(b), 1, I64(1 << 32), C.byref(L), C.byref(hi), C.byref(lo)) != 0
     assert not b.p
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("n,m", [(3, 6), (17, 35), (17, 36), (101, 210), (101, 224), (521, 1125), (2053, 5145),
+                                 (2053, 4320), (5003, 10240), (16411, 53760)])
+def test_chirp_tables(n, m, dtype):
+    """The chirps and the convolution spectrum over m against long double: each part rounded once to the working
+    precision (rel. error of a complex value at most eps / 2), in double plans beyond 32768 points formed in double,
+    whose FFT adds at most eps a bit."""
+    import scipy.fft
+    lib = aoclfftz_b200.load()
+    eps = 2.0 ** (-23 if dtype == 0 else -52)
+    ct = np.complex64 if dtype == 0 else np.complex128
+    j = np.array([k * k % (2 * n) for k in range(n)]).astype(np.longdouble)
+    ang = j * 4 * np.arctan(np.longdouble(1)) / n
+    c = np.cos(ang) - 1j * np.sin(ang)
+    b = np.zeros(m, dtype=np.clongdouble)
+    b[:n] = np.conj(c)
+    b[m - np.arange(1, n)] = np.conj(c[1:])
+    for direction in (0, 1):
+        blob, offs = Blob(), [I64() for _ in range(3)]
+        assert lib.fz_bluestein_tables(C.byref(blob), dtype, I64(n), I64(m), direction, *[C.byref(o) for o in offs]) == 0
+        raw = (C.c_ubyte * blob.len).from_address(blob.p)
+        pre, post, mid = [np.frombuffer(raw, dtype=ct, count=k, offset=o.value) for k, o in zip((n, n, m), offs)]
+        for got, ref, bits in ((pre, c, 0), (post, c if direction == 0 else np.conj(c), 0),
+                               (mid, np.conj(scipy.fft.fft(b)) / m, np.log2(m) if dtype == 1 and m > 32768 else 0)):
+            err = np.linalg.norm((got - ref).astype(np.complex128)) / np.linalg.norm(ref.astype(np.complex128))
+            assert err <= (0.5 + bits) * eps
