@@ -54,18 +54,6 @@ static void w_n(int64_t r, int64_t N, double *re, double *im)
     *im = (double)s;
 }
 
-/* roots, host_fft, chirp_spectrum in double, and the same in long double (_l) */
-#define REAL double
-#define FORM(name) name
-#include "tables_fft.h"
-#undef REAL
-#undef FORM
-#define REAL long double
-#define FORM(name) name##_l
-#include "tables_fft.h"
-#undef REAL
-#undef FORM
-
 int64_t fz_blob_reserve(fz_blob *b, size_t bytes)
 {
     size_t off = (b->len + 255) & ~(size_t)255; /* 256-byte aligned tables */
@@ -107,6 +95,18 @@ static void put_c(fz_blob *b, int64_t off, int dtype, int64_t idx, double re, do
     }
 }
 
+/* roots, stage_entries, host_fft, chirp_spectrum in double and in long double (_l) */
+#define REAL double
+#define FORM(name) name
+#include "tables_fft.h"
+#undef REAL
+#undef FORM
+#define REAL long double
+#define FORM(name) name##_l
+#include "tables_fft.h"
+#undef REAL
+#undef FORM
+
 int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32_t *radix, int32_t *tw_off, double gain)
 {
     /* stage s >= 1 uses W_{Ns*R}^{k*r}, k < Ns, r = 1..R-1, at [(r-1)*Ns + k],
@@ -124,29 +124,10 @@ int64_t fz_stage_twiddles(fz_blob *b, int dtype, int n, int nstages, const int32
     if (off < 0) return -1;
     put_c(b, off, dtype, 0, 1.0, 0.0);
     if (nstages < 2) return off;
-    /* every W_{Ns*R}^{k*r} is a root of order n = the product of the radices */
-    long double *w = roots_l(ns);
-    if (!w) return -1;
-    if (gain != 0)
-        for (int64_t r = 0; r < ns; r++)
-            if (w[2 * r] != 0 && w[2 * r + 1] != 0)
-            {
-                w[2 * r] *= 1.0L + gain;
-                w[2 * r + 1] *= 1.0L + gain;
-            }
-    const int64_t N = ns;
-    ns = radix[0];
-    for (int s = 1; s < nstages; s++)
-    {
-        const int64_t R = radix[s], step = N / (ns * R);
-        for (int64_t r = 1; r < R; r++)
-            for (int64_t k = 0; k < ns; k++)
-                put_c(b, off, dtype, tw_off[s] + (r - 1) * ns + k, (double)w[2 * (k * r * step)],
-                      (double)w[2 * (k * r * step) + 1]);
-        ns *= R;
-    }
-    free(w);
-    return off;
+    /* a double plan's scaled roots have to be rounded after the scaling */
+    const int rc = dtype == 1 && gain != 0 ? stage_entries_l(b, off, dtype, nstages, radix, tw_off, ns, gain)
+                                           : stage_entries(b, off, dtype, nstages, radix, tw_off, ns, gain);
+    return rc ? -1 : off;
 }
 
 int fz_tw4_tables(fz_blob *b, int form, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo)

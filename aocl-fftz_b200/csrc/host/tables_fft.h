@@ -1,4 +1,4 @@
-/* Roots of unity, a forward FFT and the chirp spectrum on the host, for tables.c,
+/* Roots of unity, stage twiddles, a forward FFT and the chirp spectrum for tables.c,
  * which includes this once for each REAL it forms tables in; FORM(name) is the
  * function's name there. */
 
@@ -35,6 +35,33 @@ static REAL *FORM(roots)(int64_t N)
         w[2 * r + 1] = -w[2 * (N - r) + 1];
     }
     return w;
+}
+
+/* Entries of a stage-twiddle table at off: every W_{Ns*R}^{k*r} is a root of order N,
+ * the product of the radices; those but +-1 and +-i times 1 + gain. */
+static int FORM(stage_entries)(fz_blob *b, int64_t off, int dtype, int nstages, const int32_t *radix,
+                               const int32_t *tw_off, int64_t N, double gain)
+{
+    REAL *w = FORM(roots)(N);
+    if (!w) return -1;
+    for (int64_t r = 0; gain != 0 && r < N; r++)
+        if (w[2 * r] != 0 && w[2 * r + 1] != 0)
+        {
+            w[2 * r] *= 1 + (REAL)gain;
+            w[2 * r + 1] *= 1 + (REAL)gain;
+        }
+    int64_t ns = radix[0];
+    for (int s = 1; s < nstages; s++)
+    {
+        const int64_t R = radix[s], step = N / (ns * R);
+        for (int64_t r = 1; r < R; r++)
+            for (int64_t k = 0; k < ns; k++)
+                put_c(b, off, dtype, tw_off[s] + (r - 1) * ns + k, (double)w[2 * (k * r * step)],
+                      (double)w[2 * (k * r * step) + 1]);
+        ns *= R;
+    }
+    free(w);
+    return 0;
 }
 
 /* Forward FFT, m a product of 2, 3, 5 and 7: Stockham stages of 4 and the prime
