@@ -16,7 +16,6 @@ static int mr_cost(int R)
 
 typedef struct
 {
-    int64_t n; /* the whole line */
     int min_stages, pair;
     int cur[FFTZ_MR_STAGES], best[FFTZ_MR_STAGES];
     int nbest;
@@ -54,7 +53,6 @@ int fz_mr_radices(int64_t n, int min_stages, int pair, int32_t *radix, double *c
 {
     mr_search q;
     memset(&q, 0, sizeof(q));
-    q.n = n;
     q.min_stages = min_stages;
     q.pair = pair;
     int64_t m = n;
@@ -461,7 +459,6 @@ int fz_mr_shape(fftz_pass_t *k, int want_tpc, int threads, int64_t cap)
     mr_stride(k, colmap, bp);
     k->mr.mg_tpc = magic(k->tpc);
     if (ps >= 0) k->mr.mg_pair = magic((k->n / k->radix[ps] + 1) / 2);
-    k->fuse_load = k->fuse_store = 1;
     k->use_tma = 0;
     k->smem_tw = 0;
     return fftz_pass_smem_bytes(k) <= cap ? 0 : -1;
@@ -491,7 +488,7 @@ double fz_mr_gain(int dtype, int R)
  * allocation failure. */
 int64_t fz_mr_twiddles(fz_blob *b, fftz_pass_t *k)
 {
-    int32_t rev[FFTZ_MR_STAGES], off[FFTZ_MR_STAGES];
+    int32_t rev[FFTZ_MR_STAGES] = {0}, off[FFTZ_MR_STAGES];
     const int S = k->nstages;
     for (int s = 0; s < S; s++) rev[s] = k->radix[S - 1 - s];
     double gain = 0, share = 0;

@@ -83,13 +83,12 @@ static fz_pass *push_pass(fz_plan *pl)
     memset(p, 0, sizeof(*p));
     p->off_tw = p->off_tw4hi = p->off_tw4lo = p->off_pre = p->off_post = p->off_mid = p->off_rtw = -1;
     p->k.dtype = pl->dtype;
-    p->k.scale = 1.0;
     return p;
 }
 
 static int64_t absl(int64_t x) { return x < 0 ? -x : x; }
 
-/* every pass on the generic kernel (the persistent executor runs only that) */
+/* every pass on the runtime-radix kernels */
 static int generic_only(const fz_plan *pl) { return pl->hints.kernel_family == 3; }
 
 /* kernel_family 4: passes for the persistent ragged executor, every line a
@@ -293,8 +292,6 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
             goto generic;
         }
         if (is_pipe_variant(k->variant)) maxthr = fftz_pipe_max_threads((int)n);
-        k->fuse_load = 1;
-        k->fuse_store = 1;
     }
     else
     {
@@ -328,8 +325,6 @@ static fz_pass *line_pass(fz_plan *pl, int64_t n, int64_t ies, int64_t oes, cons
             fz_set_error("length %lld exceeds the generic kernel's thread budget", (long long)n);
             return NULL;
         }
-        k->fuse_load = 0;
-        k->fuse_store = 0;
     }
     int nslots = (int)n;
     if (k->nload > nslots) nslots = k->nload;

@@ -91,13 +91,6 @@ __device__ __forceinline__ void store_complex(const fftz_pass_t &P, typename Cpl
   const int f = P.flags;
   if (f & FFTZ_F_TW4) v = cmul(v, tw4<T>(P, col, kk));
   if (f & FFTZ_F_CONJ_OUT) v.y = -v.y;
-  const int64_t li = kk * P.post_es + col * P.post_cs;
-  if (P.post_n > 0 && li >= P.post_n) return;
-  if (f & FFTZ_F_POST_TAB) v = cmul(v, __ldg((const T2 *)P.post_tab + li));
-  if (f & FFTZ_F_SCALE) {
-    v.x = (T)(v.x * P.scale);
-    v.y = (T)(v.y * P.scale);
-  }
   ((T2 *)P.out)[obase + kk * P.oes] = v;
 }
 

@@ -245,21 +245,21 @@ __device__ __forceinline__ void fast_stage(const fftz_pass_t &P, typename Cplx<T
   if (!LAST) __syncthreads();
 }
 
-// Stage S of sweep SW out of NSW sweeps. GLOBALIN: the very first stage reads
-// HBM (fast kernel); the pipelined kernel has already staged the tile.
-template <typename T, int N, int S, int NST, int SW, int NSW, int FEAT, bool GLOBALIN, int STG = 0>
+// Stages S ... NST - 1. GLOBALIN: the first stage reads HBM (fast kernel); the
+// pipelined kernel has already staged the tile.
+template <typename T, int N, int S, int NST, int FEAT, bool GLOBALIN, int STG = 0>
 struct FastStages {
   static __device__ __forceinline__ void run(const fftz_pass_t &P, typename Cplx<T>::type *sdata,
                                              const int64_t *s_in, const int64_t *s_out, const int64_t *s_col,
                                              int stg_es = 1, const typename Cplx<T>::type *twb = nullptr) {
-    constexpr bool FIRSTG = (S == 0 && SW == 0);
-    fast_stage<T, N, S, FEAT, GLOBALIN && FIRSTG, (S == NST - 1 && SW == NSW - 1), GLOBALIN && FIRSTG,
+    constexpr bool FIRSTG = (S == 0);
+    fast_stage<T, N, S, FEAT, GLOBALIN && FIRSTG, S == NST - 1, GLOBALIN && FIRSTG,
                !GLOBALIN && FIRSTG, FIRSTG ? STG : 0>(P, sdata, s_in, s_out, s_col, stg_es, nullptr, nullptr, twb);
-    FastStages<T, N, S + 1, NST, SW, NSW, FEAT, GLOBALIN, STG>::run(P, sdata, s_in, s_out, s_col, stg_es, twb);
+    FastStages<T, N, S + 1, NST, FEAT, GLOBALIN, STG>::run(P, sdata, s_in, s_out, s_col, stg_es, twb);
   }
 };
-template <typename T, int N, int NST, int SW, int NSW, int FEAT, bool GLOBALIN, int STG>
-struct FastStages<T, N, NST, NST, SW, NSW, FEAT, GLOBALIN, STG> {
+template <typename T, int N, int NST, int FEAT, bool GLOBALIN, int STG>
+struct FastStages<T, N, NST, NST, FEAT, GLOBALIN, STG> {
   static __device__ __forceinline__ void run(const fftz_pass_t &, typename Cplx<T>::type *, const int64_t *,
                                              const int64_t *, const int64_t *, int = 1,
                                              const typename Cplx<T>::type * = nullptr) {}
@@ -289,7 +289,7 @@ __device__ __forceinline__ void fast_tile(const fftz_pass_t &P, int64_t tf0, uns
   }
   pdl_begin();
   __syncthreads();
-  FastStages<T, N, 0, ct_nstages(N), 0, 1, FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
+  FastStages<T, N, 0, ct_nstages(N), FEAT, true>::run(P, sdata, s_in, s_out, s_col, 1, twb);
 }
 
 template <typename T, int N, int FEAT>
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(ct_pipe_lb(N), 1) fft_pipe_kernel(const __grid
     cp_async_commit();
     cp_async_wait1();  // this thread's copies of the current tile have landed
     __syncthreads();   // ... and everyone else's
-    FastStages<T, N, 0, ct_nstages(N), 0, 1, FEAT, false>::run(P, cur, FZ_OFF(ob, 0), FZ_OFF(ob, 1), FZ_OFF(ob, 2));
+    FastStages<T, N, 0, ct_nstages(N), FEAT, false>::run(P, cur, FZ_OFF(ob, 0), FZ_OFF(ob, 1), FZ_OFF(ob, 2));
     if (!has_next) break;
     tile = next;
   }

@@ -8,11 +8,9 @@
 // register DFT and writes the R outputs at stride Ns into the auto-sorted
 // position, so the result lands in natural order without a bit-reversal pass.
 //
-// The first stage can read straight from HBM (fuse_load) and the last stage can
-// write straight to HBM (fuse_store): with lanes mapped along elements (mode 0)
-// or along neighbouring transforms (mode 1), both accesses are coalesced for
-// rows (unit element stride) and for columns (unit batch stride) respectively.
-// Other element kinds go through a load/store phase with a separate thread map.
+// Every element kind goes through a load and a store phase with a thread map of
+// its own: lanes along elements (mode 0) or along neighbouring transforms (mode 1),
+// coalesced for rows (unit element stride) and columns (unit batch stride).
 //
 // The backward transform is conj(FFT(conj(x))): conjugation is fused into the
 // load and the store, so only forward codelets and forward twiddles exist.
@@ -26,72 +24,32 @@
 
 namespace fftz {
 
-// One Stockham stage of radix R over the transform this thread is mapped to.
-// ROLE 0..3 fixes at compile time whether the stage reads HBM (bit 0) and
-// writes HBM (bit 1), so that the shared-memory-only middle stages compile
-// without the HBM load and epilogue code (measured on B200: float 5-15%
-// faster); ROLE 4 takes both from the runtime flags (measured faster for
-// double, whose per-role copies lose more to the call convention).
-template <typename T, int R, int ROLE>
-__device__ __noinline__ void run_stage(const fftz_pass_t &P, typename Cplx<T>::type *sdata, int s, int Ns,
-                                          bool from_g_rt, bool to_g_rt, int mode, const int64_t *s_in,
-                                          const int64_t *s_out, const int64_t *s_col) {
-  const bool from_g = ROLE == 4 ? from_g_rt : (ROLE & 1) != 0;
-  const bool to_g = ROLE == 4 ? to_g_rt : (ROLE & 2) != 0;
+// One Stockham stage of radix R, in shared memory, over the transform this thread
+// is mapped to.
+template <typename T, int R>
+__device__ __noinline__ void run_stage(const fftz_pass_t &P, typename Cplx<T>::type *sdata, int s, int Ns) {
   typedef typename Cplx<T>::type T2;
   constexpr int NB = kMaxE / R;
   constexpr int SH = Cplx<T>::PADSH;
   const int n = P.n;
   const int nb = n / R;
-  const int t = threadIdx.x;
-  // blocks wider than the tile (the persistent ragged executor) idle the rest
-  const bool active = t < P.tpc * P.tpt;
-  const int nbe = active ? nb : 0;
-  int p, j;
-  if (mode == 0) {
-    p = t / P.tpt;
-    j = t - p * P.tpt;
-  } else {
-    p = t % P.tpc;
-    j = t / P.tpc;
-  }
-  if (!active) p = 0;
+  const int p = threadIdx.x / P.tpt, j = threadIdx.x - p * P.tpt;
   T2 *sd = sdata + (size_t)p * P.sstride;
-  const int64_t col = s_col[p];
-  const bool valid = col >= 0;
   T2 v[NB][R];
-  if (from_g) {
-    const T2 *gin = (const T2 *)P.in + s_in[p];
-    const bool cj = (P.flags & FFTZ_F_CONJ_IN) != 0;
 #pragma unroll
-    for (int q = 0; q < NB; q++) {
-      const int b = j + q * P.tpt;
-      if (b < nbe) {
+  for (int q = 0; q < NB; q++) {
+    const int b = j + q * P.tpt;
+    if (b < nb) {
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-          T2 x = zero2<T2>();
-          if (valid) x = gin[(int64_t)(b + r * nb) * P.ies];
-          if (cj) x.y = -x.y;
-          v[q][r] = x;
-        }
-      }
+      for (int r = 0; r < R; r++) v[q][r] = sd[phys<SH>(b + r * nb)];
     }
-  } else {
-#pragma unroll
-    for (int q = 0; q < NB; q++) {
-      const int b = j + q * P.tpt;
-      if (b < nbe) {
-#pragma unroll
-        for (int r = 0; r < R; r++) v[q][r] = sd[phys<SH>(b + r * nb)];
-      }
-    }
-    __syncthreads();
   }
+  __syncthreads();
   const T2 *tw = (const T2 *)P.tw + P.tw_off[s];
 #pragma unroll
   for (int q = 0; q < NB; q++) {
     const int b = j + q * P.tpt;
-    if (b < nbe) {
+    if (b < nb) {
       const int k = (int)((unsigned)b % (unsigned)Ns);
       if (Ns > 1) {
 #pragma unroll
@@ -99,57 +57,29 @@ __device__ __noinline__ void run_stage(const fftz_pass_t &P, typename Cplx<T>::t
       }
       Dft<R>::template apply<T, T2>(v[q]);
       const int d0 = (b - k) * R + k;
-      if (to_g) {
-        if (valid) {
 #pragma unroll
-          for (int r = 0; r < R; r++) store_complex<T>(P, v[q][r], d0 + r * Ns, col, s_out[p]);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) sd[phys<SH>(d0 + r * Ns)] = v[q][r];
-      }
+      for (int r = 0; r < R; r++) sd[phys<SH>(d0 + r * Ns)] = v[q][r];
     }
   }
-  if (!to_g) __syncthreads();
-}
-
-template <typename T, int R>
-__device__ __forceinline__ void stage_radix(const fftz_pass_t &P, typename Cplx<T>::type *sdata, int s, int Ns,
-                                            bool from_g, bool to_g, int mode, const int64_t *s_in,
-                                            const int64_t *s_out, const int64_t *s_col) {
-  if constexpr (sizeof(T) != 4) {
-    run_stage<T, R, 4>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col);
-  } else if (from_g) {
-    if (to_g)
-      run_stage<T, R, 3>(P, sdata, s, Ns, true, true, mode, s_in, s_out, s_col);
-    else
-      run_stage<T, R, 1>(P, sdata, s, Ns, true, false, mode, s_in, s_out, s_col);
-  } else {
-    if (to_g)
-      run_stage<T, R, 2>(P, sdata, s, Ns, false, true, mode, s_in, s_out, s_col);
-    else
-      run_stage<T, R, 0>(P, sdata, s, Ns, false, false, mode, s_in, s_out, s_col);
-  }
+  __syncthreads();
 }
 
 template <typename T>
-__device__ __forceinline__ void stage_dispatch(const fftz_pass_t &P, typename Cplx<T>::type *sdata, int s,
-                                               int Ns, bool from_g, bool to_g, int mode, const int64_t *s_in,
-                                               const int64_t *s_out, const int64_t *s_col) {
+__device__ __forceinline__ void stage_dispatch(const fftz_pass_t &P, typename Cplx<T>::type *sdata, int s, int Ns) {
   switch (P.radix[s]) {
-    case 2: stage_radix<T, 2>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 3: stage_radix<T, 3>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 4: stage_radix<T, 4>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 5: stage_radix<T, 5>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 7: stage_radix<T, 7>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 8: stage_radix<T, 8>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 11: stage_radix<T, 11>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    case 13: stage_radix<T, 13>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
-    default: stage_radix<T, 16>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col); break;
+    case 2: run_stage<T, 2>(P, sdata, s, Ns); break;
+    case 3: run_stage<T, 3>(P, sdata, s, Ns); break;
+    case 4: run_stage<T, 4>(P, sdata, s, Ns); break;
+    case 5: run_stage<T, 5>(P, sdata, s, Ns); break;
+    case 7: run_stage<T, 7>(P, sdata, s, Ns); break;
+    case 8: run_stage<T, 8>(P, sdata, s, Ns); break;
+    case 11: run_stage<T, 11>(P, sdata, s, Ns); break;
+    case 13: run_stage<T, 13>(P, sdata, s, Ns); break;
+    default: run_stage<T, 16>(P, sdata, s, Ns); break;
   }
 }
 
-// Global -> shared load phase for every element kind (no stage fused).
+// Global -> shared load phase for every element kind.
 template <typename T>
 __device__ void load_phase(const fftz_pass_t &P, typename Cplx<T>::type *sdata, const int64_t *s_in,
                            const int64_t *s_col) {
@@ -171,12 +101,8 @@ __device__ void load_phase(const fftz_pass_t &P, typename Cplx<T>::type *sdata, 
     if (col >= 0) {
       switch (P.in_kind) {
         case FFTZ_IN_COMPLEX: {
-          const int64_t li = (int64_t)e * P.pre_es + col * P.pre_cs;
-          if (P.pre_n == 0 || li < P.pre_n) {
-            x = ((const T2 *)P.in)[s_in[p] + (int64_t)e * P.ies];
-            if (f & FFTZ_F_CONJ_IN) x.y = -x.y;
-            if (f & FFTZ_F_PRE_TAB) x = cmul(x, __ldg((const T2 *)P.pre_tab + li));
-          }
+          x = ((const T2 *)P.in)[s_in[p] + (int64_t)e * P.ies];
+          if (f & FFTZ_F_CONJ_IN) x.y = -x.y;
           break;
         }
         case FFTZ_IN_REAL_PAIRS: {
@@ -243,7 +169,7 @@ __device__ void load_phase(const fftz_pass_t &P, typename Cplx<T>::type *sdata, 
   }
 }
 
-// Shared -> global store phase for every element kind (no stage fused).
+// Shared -> global store phase for every element kind.
 template <typename T>
 __device__ void store_phase(const fftz_pass_t &P, typename Cplx<T>::type *sdata, const int64_t *s_out,
                             const int64_t *s_col) {
@@ -284,19 +210,14 @@ __device__ void store_phase(const fftz_pass_t &P, typename Cplx<T>::type *sdata,
       case FFTZ_OUT_REAL_PAIRS: {
         T2 v = sd[phys<SH>(k)];
         if (P.flags & FFTZ_F_CONJ_OUT) v.y = -v.y;
-        if (P.flags & FFTZ_F_SCALE) {
-          v.x = (T)(v.x * P.scale);
-          v.y = (T)(v.y * P.scale);
-        }
         T *g = (T *)P.out + s_out[p];
         g[(int64_t)(2 * k) * P.oes] = v.x;
         g[(int64_t)(2 * k + 1) * P.oes] = v.y;
         break;
       }
       default: {  // FFTZ_OUT_REAL
-        T2 v = sd[phys<SH>(k)];
         T *g = (T *)P.out + s_out[p];
-        g[(int64_t)k * P.oes] = (P.flags & FFTZ_F_SCALE) ? (T)(v.x * P.scale) : v.x;
+        g[(int64_t)k * P.oes] = sd[phys<SH>(k)].x;
         break;
       }
     }
@@ -307,7 +228,6 @@ __device__ void store_phase(const fftz_pass_t &P, typename Cplx<T>::type *sdata,
 template <typename T>
 __device__ __forceinline__ void generic_tile(const fftz_pass_t &P, int64_t blk, unsigned char *smem_raw) {
   typedef typename Cplx<T>::type T2;
-  constexpr int SH = Cplx<T>::PADSH;
   T2 *sdata = (T2 *)smem_raw;
   int64_t *s_in = (int64_t *)(sdata + (size_t)P.tpc * P.sstride);
   int64_t *s_out = s_in + P.tpc;
@@ -317,34 +237,13 @@ __device__ __forceinline__ void generic_tile(const fftz_pass_t &P, int64_t blk, 
   pdl_begin();
   __syncthreads();
 
-  const int nsweeps = (P.flags & FFTZ_F_MID_TAB) ? 2 : 1;
-  if (!P.fuse_load) load_phase<T>(P, sdata, s_in, s_col);
-  for (int sw = 0; sw < nsweeps; sw++) {
-    int Ns = 1;
-    for (int s = 0; s < P.nstages; s++) {
-      const bool from_g = P.fuse_load && sw == 0 && s == 0;
-      const bool to_g = P.fuse_store && sw == nsweeps - 1 && s == P.nstages - 1;
-      const int mode = from_g ? P.in_mode : (to_g ? P.out_mode : 0);
-      stage_dispatch<T>(P, sdata, s, Ns, from_g, to_g, mode, s_in, s_out, s_col);
-      Ns *= P.radix[s];
-    }
-    if (sw == 0 && nsweeps == 2) {
-      // between the sweeps: v = conj(v) * mid_tab[e] (spectrum product of Bluestein)
-      const T2 *mt = (const T2 *)P.mid_tab;
-      for (int i = threadIdx.x; i < P.tpc * P.n; i += blockDim.x) {
-        const int p = i / P.n;
-        const int e = i - p * P.n;
-        const int64_t c = s_col[p];
-        if (c < 0) continue;
-        T2 *a = sdata + (size_t)p * P.sstride + phys<SH>(e);
-        T2 v = *a;
-        v.y = -v.y;
-        *a = cmul(v, __ldg(mt + e + c * P.mid_cs));
-      }
-      __syncthreads();
-    }
+  load_phase<T>(P, sdata, s_in, s_col);
+  int Ns = 1;
+  for (int s = 0; s < P.nstages; s++) {
+    stage_dispatch<T>(P, sdata, s, Ns);
+    Ns *= P.radix[s];
   }
-  if (!P.fuse_store) store_phase<T>(P, sdata, s_out, s_col);
+  store_phase<T>(P, sdata, s_out, s_col);
 }
 
 // float: at most 80 registers (3 CTAs of 256 threads per SM) -- measured on

@@ -221,10 +221,7 @@ int line_pass(fftz_pass_t *k, int g, int64_t ies, int64_t oes, int64_t cols, int
   k->nload = n;
   k->nstore = n;
   k->dtype = 0;
-  k->scale = 1.0;
   k->variant = variant;
-  k->fuse_load = 1;
-  k->fuse_store = 1;
   k->nbdims = 1;
   k->bdim[0] = cols;
   k->ibs[0] = ics;

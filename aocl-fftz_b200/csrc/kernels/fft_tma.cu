@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(ct_lb<T>()) fft_tma_kernel(const __grid_consta
     for (int i = threadIdx.x; i < ct_tw_total(N); i += blockDim.x) twb[i] = __ldg(g + i);
     __syncthreads();
   }
-  FastStages<T, N, 0, ct_nstages(N), 0, 1, FEAT, true, 1>::run(P, sdata, s_in, s_out, s_col,
+  FastStages<T, N, 0, ct_nstages(N), FEAT, true, 1>::run(P, sdata, s_in, s_out, s_col,
                                                                    MODE == 1 ? tpc : 1, twb);
 }
 
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(ct_lb<T>(), 1) fft_tma_pipe_kernel(const __gri
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue(tile + gridDim.x);
     }
-    FastStages<T, N, 1, NST, 0, 1, FEAT, true, 0>::run(P, sdata, s_in, s_out, s_col);
+    FastStages<T, N, 1, NST, FEAT, true, 0>::run(P, sdata, s_in, s_out, s_col);
     __syncthreads();
   }
 }
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(ct_lb<T>()) fft_tma_stream_kernel(const __grid
       }
       return;
     }
-    FastStages<T, N, 0, NST, 0, 1, FEAT, true, 1>::run(P, (T2 *)(base + sl * slot_bytes), s_in, s_out, s_col, 1,
+    FastStages<T, N, 0, NST, FEAT, true, 1>::run(P, (T2 *)(base + sl * slot_bytes), s_in, s_out, s_col, 1,
                                                        nullptr);
     // every thread is done with the slot and the offsets: refill the slot
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

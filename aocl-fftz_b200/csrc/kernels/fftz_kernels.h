@@ -9,7 +9,7 @@
  * (tf_per_cta transforms per CTA), computed as a sequence of Stockham
  * radix stages in registers with shared-memory exchanges, with optional fused
  * prologue (conjugation, chirp / real-pair / Hermitian loads) and epilogue
- * (four-step twiddle, conjugation, table product, scale, Hermitian
+ * (four-step twiddle, conjugation, table product, Hermitian
  * recombination, real stores).
  */
 #ifndef FFTZ_KERNELS_H
@@ -58,7 +58,6 @@ enum fftz_out_kind {
 #define FFTZ_F_TW4        0x04 /* multiply output k of column c by W_{tw4_n}^{c*k}  */
 #define FFTZ_F_PRE_TAB    0x08 /* multiply loaded value e by pre_tab[e*pre_es + col*pre_cs] */
 #define FFTZ_F_POST_TAB   0x10 /* multiply stored value k by post_tab[k*post_es + col*post_cs] */
-#define FFTZ_F_SCALE      0x20 /* multiply stored value by scale                  */
 #define FFTZ_F_MID_TAB    0x40 /* two sweeps: between them v = conj(v) * mid_tab[e] */
 /* 4 x 4 blocked intermediate of a 4096 x 4096 four-step (split kernels only):
  * element k of column c at (k / 4) * 4 * ncols + 4 * c + k % 4 past the line */
@@ -102,7 +101,6 @@ typedef struct fftz_pass
     int32_t in_kind, out_kind;
     int32_t in_mode, out_mode;          /* 0: lanes along elements, 1: along transforms */
     int32_t flags;
-    int32_t fuse_load, fuse_store;      /* stage 0 reads global / last stage writes global */
     int32_t variant;                    /* FFTZ_VAR_*: which kernel family runs the pass */
     int32_t dtype;                      /* 0 float, 1 double */
     int32_t nbdims;
@@ -117,7 +115,6 @@ typedef struct fftz_pass
     int64_t pre_n, pre_es, pre_cs;      /* load bound (0: none) and table index map */
     int64_t post_n, post_es, post_cs;   /* store bound (0: none) and table index map */
     int64_t mid_cs;                     /* mid_tab index of element e of column col: e + col * mid_cs */
-    double scale;
     const void *in;
     void *out;
     const void *tw;                     /* stage twiddles, working dtype */

@@ -29,11 +29,11 @@ class Pass(C.Structure):
     """fftz_pass_t (csrc/kernels/fftz_kernels.h)."""
     _fields_ = [("n", I32), ("nstages", I32), ("radix", I32 * MAXS), ("tw_off", I32 * MAXS), ("tpt", I32), ("tpc", I32),
                 ("sstride", I32), ("nload", I32), ("nstore", I32), ("in_kind", I32), ("out_kind", I32), ("in_mode", I32),
-                ("out_mode", I32), ("flags", I32), ("fuse_load", I32), ("fuse_store", I32), ("variant", I32),
+                ("out_mode", I32), ("flags", I32), ("variant", I32),
                 ("dtype", I32), ("nbdims", I32), ("ies", I64), ("oes", I64), ("ntf", I64), ("bdim", I64 * MAXB),
                 ("ibs", I64 * MAXB), ("obs", I64 * MAXB), ("tw4_n", I64), ("tw4_l", I64), ("pre_n", I64),
                 ("pre_es", I64), ("pre_cs", I64), ("post_n", I64), ("post_es", I64), ("post_cs", I64), ("mid_cs", I64),
-                ("scale", C.c_double), ("in_", VP), ("out", VP), ("tw", VP), ("tw4_hi", VP), ("tw4_lo", VP),
+                ("in_", VP), ("out", VP), ("tw", VP), ("tw4_hi", VP), ("tw4_lo", VP),
                 ("pre_tab", VP), ("post_tab", VP), ("mid_tab", VP), ("rtw", VP), ("src_buf", I32), ("dst_buf", I32),
                 ("ind_dim", I32), ("use_tma", I32), ("smem_tw", I32), ("test_tx_short", I32), ("ind_in", VP),
                 ("ind_out", VP), ("mr", Mr), ("threads", I32), ("ntw", I32), ("pad2_", I32 * 2)]
