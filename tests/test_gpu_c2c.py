@@ -97,7 +97,7 @@ def test_fourstep(dtype, n):
 
 @pytest.mark.parametrize("dtype", ["f32", "f64"])
 def test_bluestein_multipass(dtype):
-    n = 65521  # largest prime below 2^16: m = 2^17 needs the four-pass form
+    n = 65521  # largest prime below 2^16: its convolution is longer than any one-kernel line
     check_c2c(dtype, [(n, 1, 1)], [(1, n, n)], 0)
     check_c2c(dtype, [(n, 1, 1)], [(1, n, n)], 1)
 
