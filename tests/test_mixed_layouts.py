@@ -113,8 +113,11 @@ def simulate(p, x, mid=None):
     y = np.full((p.tpc, n), np.nan + 0j)
     R, M = p.radix[0], n // p.radix[0]
     r = np.arange(R)[:, None]
-    if S == 1:
-        return np.fft.fft(x, axis=1)
+    if S == 1:  # a thread a line: inputs and outputs 0 + r
+        assert R == n and M == 1
+        line = np.arange(p.tpc)
+        y[line, r] = dft(x[line, r])
+        return y
     line, rest = items(p, 0, p.in_mode)
     v = dft(x[line, rest + r * M]) * twiddle(R, M, rest)
     first = line * p.sstride + rest + r * (M + p.mr.pad)
@@ -182,8 +185,10 @@ def test_two_sweeps_are_the_convolution(n):
 @pytest.mark.parametrize("ntf,tpc", [(1, 0), (3, 0), (5, 2), (700, 0), (100000, 3)])
 def test_lines_per_cta_follow_the_batch_and_the_hint(ntf, tpc):
     p = shape(360, ntf=ntf, tpc=tpc, tw4=True)
-    assert p.tpc <= ntf and (tpc == 0 or p.tpc == tpc)
-    assert p.tpc == 1 or ntf // p.tpc >= 296 or tpc
+    if tpc:
+        assert p.tpc == min(tpc, ntf)
+    else:
+        assert p.tpc == 1 or ntf // p.tpc >= 296
 
 
 def smooth13(n):
@@ -262,28 +267,62 @@ def pair_items(p, s):
     return line, q, np.where(q > 0, nb - q, 0 if nb & 1 else nb // 2)
 
 
+def half_spectrum_pairs(nb, R):
+    """mr_store_half / mr_load_half: (butterfly and value of bin k, of bin n - k, k) of every pair that an item q holds;
+    butterfly 0 is A (bins q + r nb), 1 is B (its mirror)."""
+    def pairs(q):
+        if q:
+            return [((0, r), (1, R - 1 - r), q + r * nb) for r in range(R)]
+        out = [((0, r), (0, (R - r) % R), r * nb) for r in range(R // 2 + 1)]
+        if nb % 2 == 0:
+            out += [((1, r), (1, R - 1 - r), nb // 2 + r * nb) for r in range((R - 1) // 2 + 1)]
+        return out
+    return pairs
+
+
 @pytest.mark.parametrize("col", [False, True])
-@pytest.mark.parametrize("n", [2, 16, 18, 25, 77, 121, 143, 240, 256, 1000, 1024, 2401, 22050, 28000])
+@pytest.mark.parametrize("n", [1, 2, 7, 13, 15, 16, 18, 25, 77, 121, 143, 240, 256, 1000, 1024, 2401, 22050])
 def test_mirrored_butterflies_cover_each_bin_once(n, col):
-    """r2c / c2r: the paired stage's items hold every butterfly of every line once, and bin k of one is bin n - k of the
-    other; the stage's radix is one its two-butterfly form exists for."""
+    """r2c / c2r: the paired stage's items hold every butterfly of every line once, and the pairs of bins k, n - k that they
+    recombine (separate) are every bin of the half spectrum (every value of the packed line) once, with numpy's result; the
+    stage's radix is one its two-butterfly form exists for."""
+    rng = np.random.default_rng(n)
     for kind in (IN_PAIRS, IN_SEPARATE):
         p = shape(n, col=col, in_kind=kind)
-        if p.nstages == 1:
-            assert n <= 16
-            continue
         s = p.nstages - 1 if kind == IN_PAIRS else 0
         R, nb = p.radix[s], n // p.radix[s]
-        assert R <= 8 or R in (11, 13)
-        line, a, b = pair_items(p, s)
+        assert p.nstages == 1 or R <= 8 or R in (11, 13)
+        if p.nstages == 1:
+            line, a, b = np.arange(p.tpc), np.zeros(p.tpc, int), np.zeros(p.tpc, int)
+        else:
+            line, a, b = pair_items(p, s)
         own = np.concatenate([line * nb + a, (line * nb + b)[a != b]])
         assert np.array_equal(np.sort(own), np.arange(p.tpc * nb))
-        r = np.arange(R)[:, None]
-        ordinary = a > 0
-        assert np.all((a + r * nb + b + (R - 1 - r) * nb)[:, ordinary] == n)
-        x = np.random.default_rng(n).standard_normal((p.tpc, n)) + 0j
+        x = rng.standard_normal(2 * n)
+        Z, X = np.fft.fft(x[0::2] + 1j * x[1::2]), np.fft.rfft(x)
+        w = np.exp(-1j * np.pi * np.arange(n + 1) / n)
+        bins, vals = np.full(n + 1, np.nan + 0j), np.full(n, np.nan + 0j)
+        pairs = half_spectrum_pairs(nb, R)
+        for q, m in {(int(q), int(m)) for q, m in zip(a, b)}:
+            at = {0: q, 1: m}
+            for (f, r), (g, t), k in pairs(q):
+                i, j = at[f] + r * nb, at[g] + t * nb
+                assert i == k and j == (n - k) % n
+                if kind == IN_PAIRS:
+                    E, O = (Z[i] + np.conj(Z[j])) / 2, -0.5j * (Z[i] - np.conj(Z[j]))
+                    assert np.isnan(bins[k]) and (k == n - k or np.isnan(bins[n - k]))
+                    bins[k], bins[n - k] = E + w[k] * O, np.conj(E - w[k] * O)
+                else:
+                    S, D = X[k] + np.conj(X[n - k]), np.conj(w[k]) * (X[k] - np.conj(X[n - k]))
+                    assert np.isnan(vals[i]) and (i == j or np.isnan(vals[j]))
+                    vals[j], vals[i] = np.conj(S) + 1j * np.conj(D), S + 1j * D
         if kind == IN_PAIRS:
-            assert np.linalg.norm(simulate(p, x) - np.fft.fft(x, axis=1)) <= 1e-13 * np.linalg.norm(x) * np.sqrt(n)
+            assert np.linalg.norm(bins - X) <= 1e-13 * np.linalg.norm(X)
+            if p.nstages > 1:
+                y = rng.standard_normal((p.tpc, n)) + 0j
+                assert np.linalg.norm(simulate(p, y) - np.fft.fft(y, axis=1)) <= 1e-13 * np.linalg.norm(y) * np.sqrt(n)
+        else:
+            assert np.linalg.norm(vals - 2 * Z) <= 1e-13 * np.linalg.norm(Z) * 2
 
 
 class Blob(C.Structure):
@@ -314,6 +353,28 @@ def test_four_step_factor_tables(N, form, parts, eps):
         # pi, product and quotient each rounded by at most 2^-62, and the cosine
         assert np.abs(got - np.stack([np.cos(a), -np.sin(a)], axis=1)).max() <= eps / 2 + 4 * 2.0 ** -62
     assert b.len >= lo.value + L.value * parts * 2 * real().itemsize
+
+
+@pytest.mark.parametrize("n1,n2,R", [(375, 320, 15), (16, 5000, 4), (1331, 121, 11)])
+def test_four_step_factors_of_a_butterfly(n1, n2, R):
+    """mr_store: output K + r nb of column c times W^{c K} W^{c nb r}, both factors found below N in the tables."""
+    lib = aoclfftz_b200.load()
+    N, nb = n1 * n2, n1 // R
+    b, L, hi, lo = Blob(), I64(), I64(), I64()
+    assert lib.fz_tw4_tables(C.byref(b), 1, I64(N), C.byref(L), C.byref(hi), C.byref(lo)) == 0
+    raw = (C.c_ubyte * b.len).from_address(b.p)
+    h = np.frombuffer(raw, dtype=np.complex128, count=-(-N // L.value), offset=hi.value)
+    l = np.frombuffer(raw, dtype=np.complex128, count=L.value, offset=lo.value)
+    assert L.value & (L.value - 1) == 0  # found by a shift and a mask
+    c, K, r = np.meshgrid(np.arange(0, n2, 7), np.arange(nb), np.arange(R), indexing="ij")
+
+    def factor(e):
+        assert e.max() < N
+        return h[e // L.value] * l[e % L.value]
+
+    exact = np.exp(-2j * np.pi * (c * (K + r * nb)) / N)
+    # three products of values of modulus 1, each part rounded once, and exp's own angle of up to 2 pi
+    assert np.abs(factor(c * K) * factor(c * nb * r) - exact).max() <= 16 * 2.0 ** -52
 
 
 def test_four_step_factors_beyond_32_bits_are_refused():
