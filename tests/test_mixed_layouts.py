@@ -36,7 +36,7 @@ class Pass(C.Structure):
                 ("in_", VP), ("out", VP), ("tw", VP), ("tw4_hi", VP), ("tw4_lo", VP),
                 ("pre_tab", VP), ("post_tab", VP), ("mid_tab", VP), ("rtw", VP), ("src_buf", I32), ("dst_buf", I32),
                 ("ind_dim", I32), ("use_tma", I32), ("smem_tw", I32), ("test_tx_short", I32), ("ind_in", VP),
-                ("ind_out", VP), ("mr", Mr), ("threads", I32), ("ntw", I32), ("pad2_", I32 * 2)]
+                ("ind_out", VP), ("mr", Mr), ("threads", I32), ("ntw", I32), ("pad2_", I32 * 6)]
 
 
 def shape(n, dtype=0, col=False, two=False, tw4=False, ntf=100000, tpc=0, threads=0, cap=0, in_kind=0):
