@@ -147,7 +147,7 @@ enum { FZ_TW4_F32, FZ_TW4_F64, FZ_TW4_F64X2 };
 int fz_tw4_tables(fz_blob *b, int form, int64_t N, int64_t *L, int64_t *off_hi, int64_t *off_lo);
 /* Bluestein tables for length n, 7-smooth convolution length m, direction; the
  * spectrum of a double plan is formed in long double up to this m */
-#define FZ_EXACT_SPECTRUM 32768
+#define FZ_EXACT_SPECTRUM 65536
 int fz_bluestein_tables(fz_blob *b, int dtype, int64_t n, int64_t m, int direction, int64_t *off_pre,
                         int64_t *off_post, int64_t *off_mid);
 /* appends the row-major copy T'[k1 * n2 + k2] = T[k1 + n1 * k2] of the table

@@ -211,9 +211,11 @@ _OPS_TW = {2: (0, 4, 6, 10, 0, 0), 3: (0, 12, 16, 16, 0, 0), 4: (0, 12, 22, 22, 
 
 
 def _radices(n):
-    """The stage radices the planner uses for a line of length n: 16s (then
-    8, 4 or 2) for powers of two, else the balanced power-of-two part and the
-    odd factors (csrc/host/plan.c generic_radices)."""
+    """A line of length n in radices that the reference has codelets for, as the
+    compile-time and in-place kernels split it (csrc/host/plan.c
+    generic_radices): 16s (then 8, 4 or 2) for powers of two, else the balanced
+    power-of-two part and the odd factors. Mixed-radix tiles take composites
+    (6, 9, 10, 12, 14, 15) that the reference has no counts for."""
     if n <= 1:
         return []
     if n & (n - 1) == 0:
@@ -233,7 +235,7 @@ def _radices(n):
         while m % q == 0:
             out.append(q)
             m //= q
-    if m != 1:  # Bluestein: count its power-of-two convolution length twice
+    if m != 1:  # Bluestein: opcount_cost counts a convolution length twice
         return None
     return out
 
@@ -251,8 +253,8 @@ def opcount_cost(passes):
     codelets in stage s, the plain codelet in stage 0 and the twiddled one
     after it, each weighted by its operation counts (codelet_cost); a pass of
     ntf lines costs ntf times that; a line without a radix split (Bluestein)
-    counts its power-of-two convolution length twice; elementwise passes 2 n
-    per line. It sees the arithmetic only -- not memory traffic, launch shape
+    counts the next power of two above 2 n twice, whatever convolution length
+    the plan takes; elementwise passes 2 n per line. It sees the arithmetic only -- not memory traffic, launch shape
     or kernel family."""
     cost = 0.0
     for kind, n, ntf, tpc in passes:
