@@ -386,10 +386,10 @@ def test_four_step_factors_beyond_32_bits_are_refused():
 
 @pytest.mark.parametrize("dtype", [0, 1])
 @pytest.mark.parametrize("n,m", [(3, 6), (17, 35), (17, 36), (101, 210), (101, 224), (521, 1125), (2053, 5145),
-                                 (2053, 4320), (5003, 10240), (16411, 53760)])
+                                 (2053, 4320), (5003, 10240), (16411, 53760), (40009, 81920)])
 def test_chirp_tables(n, m, dtype):
     """The chirps and the convolution spectrum over m against long double: each part rounded once to the working
-    precision (rel. error of a complex value at most eps / 2), in double plans beyond 32768 points formed in double,
+    precision (rel. error of a complex value at most eps / 2), in double plans beyond 65536 points formed in double,
     whose FFT adds at most eps a bit."""
     import scipy.fft
     lib = aoclfftz_b200.load()
@@ -407,6 +407,6 @@ def test_chirp_tables(n, m, dtype):
         raw = (C.c_ubyte * blob.len).from_address(blob.p)
         pre, post, mid = [np.frombuffer(raw, dtype=ct, count=k, offset=o.value) for k, o in zip((n, n, m), offs)]
         for got, ref, bits in ((pre, c, 0), (post, c if direction == 0 else np.conj(c), 0),
-                               (mid, np.conj(scipy.fft.fft(b)) / m, np.log2(m) if dtype == 1 and m > 32768 else 0)):
+                               (mid, np.conj(scipy.fft.fft(b)) / m, np.log2(m) if dtype == 1 and m > 65536 else 0)):
             err = np.linalg.norm((got - ref).astype(np.complex128)) / np.linalg.norm(ref.astype(np.complex128))
             assert err <= (0.5 + bits) * eps
