@@ -13,14 +13,13 @@ template <typename T, bool BIG> __host__ __device__ constexpr int mr_lb() {
 }
 
 // Measured on B200 against the ping-pong tiles this replaced (two buffers, one
-// prime radix a stage, 153 thread instructions a point at n = 1000; now 88):
-// n = 1000 x 32768 float 242 -> 125 us (2.16 -> 4.19 TB/s read + written),
+// prime radix a stage, 153 thread instructions a point at n = 1000; now 86):
+// n = 1000 x 32768 float 242 -> 130 us (2.16 -> 4.04 TB/s read + written),
 // four 1920 x 1080 images (rows, then columns) 181 -> 94 us, 120000 = 375 x 320 in
-// double x 64 (two passes) 307 -> 184 us, 77 x 100000 float 45 us. ncu at n = 1000
-// (94 instructions a point): issue 56%, shared-memory wavefronts 58%, DRAM 36% of
-// peak -- issue and the shared-memory pipe together, not HBM, bound it. Lines per
-// CTA at n = 1000, at 94 instructions: 2 166, 3 136, 4 146, 5 135 (fz_mr_shape's
-// choice), 6 142 us.
+// double x 64 (two passes) 307 -> 160 us, 77 x 100000 float 45 us. ncu at n = 1000:
+// issue 64%, shared-memory wavefronts 70%, DRAM 45% of peak -- issue and the
+// shared-memory pipe together, not HBM, bound it. Lines per CTA at n = 1000, at 94
+// instructions: 2 166, 3 136, 4 146, 5 135 (fz_mr_shape's choice), 6 142 us.
 // Real lines, against the kernels that loaded, transformed and recombined in
 // separate sweeps of shared memory (r2c / c2r us, before -> after): 2048 x 8192
 // float 56 / 54 -> 41 / 42, 512 x 262144 double 730 / 642 -> 521 / 460, 1024 x 65536
